@@ -34,19 +34,83 @@ inline long long base_off(int n, int inc) { return inc >= 0 ? 0 : (long long)(n 
 // ------------------------------------------------------------------- DGER
 constexpr int GER_ROWS = 512, GER_COLS = 32;
 
+// 512 rows x 32 columns per CTA, two rows per thread, eight columns' loads in
+// flight.  The bound is HBM (16 bytes per element and one DFMA: the FP64
+// pipe alone would take two thirds of that time), so nothing else per
+// element may use the FP64 pipe: alpha y_j is formed once per CTA and the
+// test for a zero y_j (netlib leaves that column alone) is a bit in an
+// integer mask.  With the product and the test per element the FP64 pipe was
+// the bound: 8192 x 8192 took 387 us, now 162 us (1.07 GB, 6.6 TB/s).
+// vec: A is 16-byte aligned and lda even, so that a thread's two adjacent
+// rows are one 128-bit access in every column.
 __global__ void __launch_bounds__(256)
 ger_kernel(int m, int n, double alpha, const double *__restrict__ x, int incx, const double *__restrict__ y,
-           int incy, double *__restrict__ A, long long lda)
+           int incy, double *__restrict__ A, long long lda, int vec)
 {
-    const int c0 = blockIdx.y * GER_COLS, c1 = min(n, c0 + GER_COLS);
-    for (int i = blockIdx.x * GER_ROWS + threadIdx.x; i < min(m, (blockIdx.x + 1) * GER_ROWS); i += blockDim.x) {
-        const double xi = __ldg(x + (long long)i * incx);
-        double *ap = A + (long long)c0 * lda + i;
-#pragma unroll 4
-        for (int j = c0; j < c1; j++, ap += lda) {
-            const double yj = __ldg(y + (long long)j * incy);
-            if (yj != 0.0) *ap = fma(xi, alpha * yj, *ap);
+    __shared__ double coef[GER_COLS];
+    __shared__ unsigned s_keep;
+    const int c0 = blockIdx.y * GER_COLS, cols = min(GER_COLS, n - c0);
+    const int tid = threadIdx.x;
+    if (tid < 32) {
+        const double yj = tid < cols ? __ldg(y + (long long)(c0 + tid) * incy) : 0.0;
+        coef[tid] = alpha * yj;
+        // y_j != 0 on the bit pattern (NaN counts as nonzero)
+        const unsigned keep = __ballot_sync(0xffffffffu, (__double_as_longlong(yj) << 1) != 0);
+        if (tid == 0) s_keep = keep;
+    }
+    __syncthreads();
+    const unsigned keep = s_keep;
+    // vec: rows r, r + 1 with r even; otherwise rows r and r + 256
+    const int r = blockIdx.x * GER_ROWS + (vec ? 2 * tid : tid);
+    const int r2 = vec ? r + 1 : r + 256;
+    if (r >= m) return;
+    double *ap = A + (long long)c0 * lda + r;
+    const double x0 = __ldg(x + (long long)r * incx);
+    const double x1 = r2 < m ? __ldg(x + (long long)r2 * incx) : 0.0;
+    if (keep == 0xffffffffu >> (GER_COLS - cols) && r2 < m) {   // no column is skipped
+        if (vec) {
+#pragma unroll 1
+            for (int j = 0; j < cols; j += 8) {
+                double2 v[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++)
+                    if (j + u < cols) v[u] = *(const double2 *)(ap + (j + u) * lda);
+#pragma unroll
+                for (int u = 0; u < 8; u++)
+                    if (j + u < cols) {
+                        const double c = coef[j + u];
+                        v[u].x = fma(x0, c, v[u].x);
+                        v[u].y = fma(x1, c, v[u].y);
+                        *(double2 *)(ap + (j + u) * lda) = v[u];
+                    }
+            }
+        } else {
+#pragma unroll 1
+            for (int j = 0; j < cols; j += 8) {
+                double v[8], w[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++)
+                    if (j + u < cols) {
+                        v[u] = ap[(j + u) * lda];
+                        w[u] = ap[(j + u) * lda + 256];
+                    }
+#pragma unroll
+                for (int u = 0; u < 8; u++)
+                    if (j + u < cols) {
+                        const double c = coef[j + u];
+                        ap[(j + u) * lda] = fma(x0, c, v[u]);
+                        ap[(j + u) * lda + 256] = fma(x1, c, w[u]);
+                    }
+            }
         }
+        return;
+    }
+    for (int j = 0; j < cols; j++) {
+        if (!((keep >> j) & 1)) continue;
+        double *q = ap + j * lda;
+        const double c = coef[j];
+        *q = fma(x0, c, *q);
+        if (r2 < m) q[r2 - r] = fma(x1, c, q[r2 - r]);
     }
 }
 
@@ -65,11 +129,14 @@ symv_tiles(int n, int nb, int lower, const double *__restrict__ A, long long lda
     __shared__ double sxI[SY_T], sxJ[SY_T];
     __shared__ double red[4][SY_T];
     // tile index -> (I, J) with I >= J (lower) in row-major triangle order
+    // (FP32 square root and integer correction: an FP64 one by every thread
+    // cost the FP64 pipe nearly half as much as the tile's products:
+    // n = 8192 took 198 us, now 136 us)
     const int t = blockIdx.x;
-    int I = (int)((sqrt(8.0 * (double)t + 1.0) - 1.0) * 0.5);
+    int I = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
     while ((long long)(I + 1) * (I + 2) / 2 <= t) I++;
     while ((long long)I * (I + 1) / 2 > t) I--;
-    int J = t - I * (I + 1) / 2;
+    int J = (int)(t - (long long)I * (I + 1) / 2);
     if (!lower) { const int tmp = I; I = J; J = tmp; }   // upper: I <= J
     const int r0 = I * SY_T, c0 = J * SY_T;
     const int tid = threadIdx.x;
@@ -112,19 +179,28 @@ symv_tiles(int n, int nb, int lower, const double *__restrict__ A, long long lda
     if (tid < SY_T) colp[tid] = (red[0][tid] + red[1][tid]) + (red[2][tid] + red[3][tid]);
 }
 
-// y_i = alpha * sum_q part[b][q][i] + beta y_i  (beta == 0 sets y)
-__global__ void __launch_bounds__(256)
+// y_i = alpha * sum_q part[b][q][i] + beta y_i  (beta == 0 sets y).  One CTA
+// per output block, four threads per row, each summing a quarter of the
+// partials in order with eight loads in flight (one thread per row walking
+// all 128 partials of n = 8192 took 19.6 us, now 6.8 us).
+__global__ void __launch_bounds__(4 * SY_T)
 symv_finish(int n, int nb, const double *__restrict__ part, double alpha, double beta, double *__restrict__ y,
             int incy)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int b = i / SY_T, l = i % SY_T;
-        const double *p = part + (size_t)b * nb * SY_T + l;
-        double s = 0.0;
-        for (int q = 0; q < nb; q++) s += p[(size_t)q * SY_T];
-        double *yp = y + (long long)i * incy;
-        *yp = (beta == 0.0) ? alpha * s : fma(alpha, s, beta * *yp);
-    }
+    __shared__ double red[4][SY_T];
+    const int b = blockIdx.x, l = threadIdx.x & (SY_T - 1), g = threadIdx.x / SY_T;
+    const int q0 = (int)((long long)nb * g / 4), q1 = (int)((long long)nb * (g + 1) / 4);
+    const double *p = part + (size_t)b * nb * SY_T + l;
+    double s = 0.0;
+#pragma unroll 8
+    for (int q = q0; q < q1; q++) s += p[(size_t)q * SY_T];
+    red[g][l] = s;
+    __syncthreads();
+    const int i = b * SY_T + l;
+    if (g || i >= n) return;
+    s = (red[0][l] + red[1][l]) + (red[2][l] + red[3][l]);
+    double *yp = y + (long long)i * incy;
+    *yp = (beta == 0.0) ? alpha * s : fma(alpha, s, beta * *yp);
 }
 
 // ------------------------------------------------------------------ DTRSV
@@ -233,8 +309,9 @@ extern "C" gbx_status gbx_dger(gbx_ctx *ctx, int m, int n, double alpha, const d
     dim3 g((m + GER_ROWS - 1) / GER_ROWS, (n + GER_COLS - 1) / GER_COLS);
     if (g.y > 65535) return gbx_fail(ctx, GBX_ERR_UNSUPPORTED, "DGER: n too large");
     gbx_timer_begin(ctx, GBX_TIMER_GEMV);
+    const int vec = (((uintptr_t)A) & 15) == 0 && lda % 2 == 0;
     ger_kernel<<<g, 256, 0, S(ctx)>>>(m, n, alpha, x + base_off(m, incx), incx, y + base_off(n, incy), incy, A,
-                                      lda);
+                                      lda, vec);
     gbx_timer_end(ctx);
     gbx_count_launch(ctx, 1);
     return gbx_check_launch(ctx, "dger");
@@ -263,8 +340,7 @@ extern "C" gbx_status gbx_dsymv(gbx_ctx *ctx, char uplo, int n, double alpha, co
     } else {
         cudaMemsetAsync(part, 0, sizeof(double) * (size_t)nb * nb * SY_T, S(ctx));
     }
-    const int sms = gbx_ctx_sms(ctx);
-    symv_finish<<<std::min(sms * 4, (n + 255) / 256), 256, 0, S(ctx)>>>(n, nb, part, alpha, beta, yb, incy);
+    symv_finish<<<nb, 4 * SY_T, 0, S(ctx)>>>(n, nb, part, alpha, beta, yb, incy);
     gbx_count_launch(ctx, 1);
     return gbx_check_launch(ctx, "dsymv");
 }
