@@ -13,12 +13,9 @@
 //     FMAs per 8 bytes: on GB300's FP64 pipe (2 lanes per clock per SM) that
 //     is the bound, not HBM.  Per-tile partial vectors are summed in a fixed
 //     order by a second kernel (deterministic).
-//   * DTRSV: blocked substitution in 64-row steps.  The 64x64 diagonal blocks
-//     of op(A) are inverted once (trinv_blocks of trsm.cu); step J is one
-//     launch whose every CTA forms x_J = inv(A_JJ) b_J from the running
-//     right-hand side and subtracts op(A)_IJ x_J from its rows I beyond J.
-//     The running right-hand side lives in workspace, so no CTA reads what
-//     another writes in the same launch.
+//   * DTRSV: one cooperative launch in which every CTA owns a 64-row block
+//     and passes its part of the solution to the later blocks through global
+//     memory as soon as it is known (see trsv_solve).
 #include "gbx_internal.h"
 #include "gemm_host.h"
 
@@ -204,63 +201,251 @@ symv_finish(int n, int nb, const double *__restrict__ part, double alpha, double
 }
 
 // ------------------------------------------------------------------ DTRSV
-constexpr int TV_NB = 64;
+constexpr int TV_NB = 64, TV_LD = TV_NB + 1, TV_THREADS = 256, TV_STAGES = 3;
+constexpr int TV_TILE = TV_NB * TV_LD;
+constexpr size_t TV_SMEM = sizeof(double) * ((TV_STAGES + 1) * TV_TILE + 4 * TV_NB + TV_NB + 8 * 16);
+constexpr int TV_FOLD = 24;
+constexpr unsigned long long TV_TIMEOUT_NS = 2000000000ull;
+constexpr int TV_TIMEOUT_CODE = 9;
 
-__global__ void gather_vec(int n, const double *__restrict__ x, int incx, double *__restrict__ w, int npad)
+struct TrsvArgs {
+    int n, nblk, fwd, tr, unit, incx;
+    const double *A;
+    long long lda;
+    double *x;          // element 0 of the vector
+    double *xw;         // solution in solve order, nblk * 64 values, all bits set until known
+    int *status, *status_host;
+};
+
+__device__ __forceinline__ unsigned long long tv_now()
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npad; i += gridDim.x * blockDim.x)
-        w[i] = i < n ? x[(long long)i * incx] : 0.0;
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
 }
 
-// Step J (solve order position): every CTA computes x_J = inv_J b_J (64 x 64
-// from the inverted diagonal blocks), CTA 0 stores it to x, and each CTA
-// subtracts op(A)(rows, cols J) x_J from its 256 rows of the running
-// right-hand side w (rows of the not yet solved blocks only).
-//   fwd: op(A) lower, blocks solved in increasing order, updated rows below;
-//   otherwise upper, decreasing order, updated rows above.
-//   tr:  op(A) = A^T (A read transposed: a warp per row, lanes along k).
-__global__ void __launch_bounds__(256)
-trsv_step(int n, int J, int fwd, int tr, const double *__restrict__ A, long long lda, const double *__restrict__ inv,
-          double *__restrict__ w, double *__restrict__ x, int incx)
+// 8-byte asynchronous copy; ok == 0 writes zero and reads nothing.
+__device__ __forceinline__ void tv_copy8(double *dst, const double *src, int ok)
 {
-    __shared__ double sx[TV_NB];
-    __shared__ double sb[TV_NB];
-    const int tid = threadIdx.x;
-    const int c0 = J * TV_NB;
-    if (tid < TV_NB) sb[tid] = w[c0 + tid];
-    __syncthreads();
-    const double *iv = inv + (size_t)J * TV_NB * TV_NB;
-    if (tid < TV_NB) {
-        double s = 0.0;
-        for (int k = 0; k < TV_NB; k++) s = fma(iv[(size_t)k * TV_NB + tid], sb[k], s);
-        sx[tid] = s;
-        if (blockIdx.x == 0 && c0 + tid < n) x[(long long)(c0 + tid) * incx] = s;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;"
+                 :: "r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(ok ? 8 : 0) : "memory");
+}
+
+// op(A) in solve order: T(p, c) = op(A)(g(p), g(c)) with g(p) = p for a lower
+// op(A) and n - 1 - p for an upper one, so that T is always lower triangular
+// and solved forwards.  Address of T(p, c); p, c < n.
+__device__ __forceinline__ const double *tv_at(const TrsvArgs &a, int p, int c)
+{
+    const long long r = a.fwd ? p : a.n - 1 - p, q = a.fwd ? c : a.n - 1 - c;
+    return a.tr ? a.A + r * a.lda + q : a.A + q * a.lda + r;
+}
+
+// Starts the copy of the 64 x 64 block (s, K), K < s, to dst[k * 65 + i]:
+// neighbouring threads take neighbouring addresses in memory.
+__device__ __forceinline__ void tv_fetch(const TrsvArgs &a, double *dst, int s, int K)
+{
+    const int t = threadIdx.x & 63, g = threadIdx.x >> 6;
+    const int i0 = a.tr ? g : t, k0 = a.tr ? t : g;
+    const int p0 = s * TV_NB + i0, c0 = K * TV_NB + k0;
+    const long long sgn = a.fwd ? 1 : -1;
+    const double *src = tv_at(a, min(p0, a.n - 1), c0);
+    const long long step = 4 * sgn * a.lda;
+    double *d = dst + k0 * TV_LD + i0;
+#pragma unroll
+    for (int u = 0; u < 16; u++) {
+        const int ok = p0 + (a.tr ? 4 * u : 0) < a.n;
+        tv_copy8(d, ok ? src + u * step : a.A, ok);
+        d += a.tr ? 4 : 4 * TV_LD;
+    }
+}
+
+// X = inverse of the lower triangular 64 x 64 block D (D[k * 65 + i] is row i,
+// column k; the same layout for X; W: 32 x 33 scratch), by the whole CTA:
+// the two 32 x 32 diagonal blocks by substitution, lane j owning column j
+// and four warps sharing a block's rows, then X21 = -X22 (D21 X11).  FP64
+// instructions hold the SM's 2-lane pipe 16 cycles each whatever their
+// predicate, so the loops skip the zero parts by warp.
+__device__ __forceinline__ void tv_invert(const double *D, double *X, double *W)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int b = warp >> 2, part = warp & 3, o = 32 * b;   // diagonal block, rows r = 4 u + part
+    const double rd = 1.0 / D[(o + lane) * TV_LD + o + lane];   // lane i: 1 / D_ii of this warp's block
+    double s[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) s[u] = (4 * u + part == lane) ? 1.0 : 0.0;
+#pragma unroll
+    for (int i = 0; i < 32; i++) {
+        const double ri = __shfl_sync(0xffffffffu, rd, i);
+        if ((i & 3) == part) X[(o + lane) * TV_LD + o + i] = s[i >> 2] * ri;
+        asm volatile("bar.sync %0, 128;" :: "r"(1 + b) : "memory");
+        const double w = X[(o + lane) * TV_LD + o + i];
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            if (4 * u + 3 > i && 4 * u + part > i) s[u] = fma(-D[(o + i) * TV_LD + o + 4 * u + part], w, s[u]);
     }
     __syncthreads();
-    const int cols = min(TV_NB, n - c0);
-    // rows this CTA updates: the 256-row slab blockIdx.x of the unsolved range
-    const int lo = fwd ? c0 + TV_NB : 0, hi = fwd ? n : c0;
-    const int rbeg = lo + blockIdx.x * 256;
-    if (rbeg >= hi) return;
-    if (!tr) {
-        const int i = rbeg + tid;
-        if (i >= hi) return;
-        const double *ap = A + (long long)c0 * lda + i;
-        double s = 0.0;
-#pragma unroll 8
-        for (int k = 0; k < cols; k++) s = fma(ap[(long long)k * lda], sx[k], s);
-        w[i] -= s;
-    } else {
-        const int warp = tid >> 5, lane = tid & 31;
-        for (int i = rbeg + warp; i < min(hi, rbeg + 256); i += 8) {
-            const double *ap = A + (long long)i * lda + c0;   // op(A)(i, c0 + k) = A(c0 + k, i)
-            double s = 0.0;
-            if (lane < cols) s = ap[lane] * sx[lane];
-            if (lane + 32 < cols) s = fma(ap[lane + 32], sx[lane + 32], s);
+    // W = D21 X11, lane = row, this warp's columns j = warp + 8 u
 #pragma unroll
-            for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (lane == 0) w[i] -= s;
+    for (int u = 0; u < 4; u++) {
+        const int j = warp + 8 * u;
+        double v = 0.0;
+#pragma unroll 4
+        for (int k = j; k < 32; k++) v = fma(D[k * TV_LD + 32 + lane], X[j * TV_LD + k], v);
+        W[j * 33 + lane] = v;
+    }
+    __syncthreads();
+    // X21 = -X22 W, lane = column, this warp's rows i = warp + 8 u; X12 = 0
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const int i = warp + 8 * u;
+        double v = 0.0;
+#pragma unroll 4
+        for (int k = 0; k <= i; k++) v = fma(-X[(32 + k) * TV_LD + 32 + i], W[lane * 33 + k], v);
+        X[lane * TV_LD + 32 + i] = v;
+        X[(32 + lane) * TV_LD + i] = 0.0;
+    }
+    __syncthreads();
+}
+
+// This warp's 16 values of solution block K (columns 16 q .. of it): lanes
+// 0-15 hold them in v once known.  The values themselves are the flags: a
+// block's owner stores them over the "all bits set" pattern.  A wait that
+// lasts 2 s gives up: the status word is set and the values become NaN, so
+// that every later block still finishes.
+__device__ __forceinline__ double tv_load(const double *p, int lane)
+{
+    return lane < 16 ? *(const volatile double *)(p + lane) : 0.0;
+}
+__device__ __forceinline__ double tv_wait(const TrsvArgs &a, const double *p, double v, int lane)
+{
+    if (__all_sync(0xffffffffu, __double_as_longlong(v) != -1ll)) return v;
+    const unsigned long long t0 = tv_now();
+    while (true) {
+        if (__double_as_longlong(v) == -1ll) v = tv_load(p, lane);
+        if (__all_sync(0xffffffffu, __double_as_longlong(v) != -1ll)) return v;
+        if (__any_sync(0xffffffffu, tv_now() - t0 > TV_TIMEOUT_NS)) {
+            if (lane == 0) {
+                atomicCAS(a.status, 0, TV_TIMEOUT_CODE);
+                *(volatile int *)a.status_host = TV_TIMEOUT_CODE;
+                __threadfence_system();
+            }
+            return __longlong_as_double(0x7ff8000000000000ll);
         }
+    }
+}
+
+// x := T^-1 x, blocks of 64 rows in solve order; CTA b owns blocks b,
+// b + gridDim.x, ...  All CTAs are resident (cooperative launch), and a block
+// waits only for earlier ones.  For its block s a CTA
+//   * inverts the diagonal block (while it waits anyway, except the first);
+//   * subtracts T(s, K) x_K for every earlier block K as x_K appears, the
+//     64 x 64 blocks of T prefetched three deep into shared memory (they do
+//     not depend on x), 16 of the products per thread and block;
+//   * x_s = inv (b - sum) goes to the later blocks through xw and to x.
+// What bounds it: the chain over the blocks, each link one hand-over through
+// L2 (about 1 us) and the products between x_(s-1) and x_s, 1 us per 64 x 64
+// on the SM's two FP64 lanes.  From the 24th block on there is time to form
+// M = inv T(s, s-1) beforehand, so that x_s = inv (b - sum over K < s-1) -
+// M x_(s-1) needs one product after x_(s-1) instead of two (M costs 47 us,
+// by which the chain has come to that block).  64 rows per block: half of it
+// would double the hand-overs, double of it the products per link.
+// n = 8192: 300 us for N or T; one launch per 64 rows, each forming
+// x_s in every CTA, took 4.1 ms.
+__global__ void __launch_bounds__(TV_THREADS)
+trsv_solve(TrsvArgs a)
+{
+    extern __shared__ __align__(16) double tv_sm[];
+    double *stage = tv_sm;                          // TV_STAGES blocks
+    double *X = stage + TV_STAGES * TV_TILE;        // inverse of the diagonal block
+    double *red = X + TV_TILE;                      // [4][64]
+    double *st = red + 4 * TV_NB;                   // [64]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int i = tid & 63, q = tid >> 6;           // row, quarter of the columns
+    double *xs = st + TV_NB + 16 * warp;            // this warp's 16 solution values
+
+    for (int s = blockIdx.x; s < a.nblk; s += gridDim.x) {
+        const int p = s * TV_NB + i;
+        // diagonal block into stage 0 (identity beyond n)
+        for (int t = tid; t < TV_NB * TV_NB; t += TV_THREADS) {
+            const int u = t & 63, v = t >> 6;
+            const int r = a.tr ? v : u, k = a.tr ? u : v;
+            const int pr = s * TV_NB + r, pk = s * TV_NB + k;
+            double d = r == k ? 1.0 : 0.0;
+            if (k <= r && pr < a.n && !(a.unit && r == k)) d = *tv_at(a, pr, pk);
+            stage[k * TV_LD + r] = d;
+        }
+        const bool fold = s >= TV_FOLD;
+        if (fold) tv_fetch(a, stage + TV_TILE, s, s - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const double b = p < a.n ? a.x[(long long)(a.fwd ? p : a.n - 1 - p) * a.incx] : 0.0;
+        __syncthreads();
+        tv_invert(stage, X, stage + 2 * TV_TILE);
+        double M[16];
+        if (fold) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();
+            // M(i, 16 q ..): row i of the inverse reaches column i at most
+            const double *T1 = stage + TV_TILE + 16 * q * TV_LD;
+#pragma unroll
+            for (int k = 0; k < 16; k++) M[k] = 0.0;
+            const int jend = (warp & 1) ? 64 : 32;
+            for (int j = 0; j < jend; j++) {
+                const double v = X[j * TV_LD + i];
+#pragma unroll
+                for (int k = 0; k < 16; k++) M[k] = fma(v, T1[k * TV_LD + j], M[k]);
+            }
+            __syncthreads();
+        }
+        const int nk = fold ? s - 1 : s;   // blocks subtracted one by one
+#pragma unroll
+        for (int f = 0; f < TV_STAGES - 1; f++) {
+            if (f < nk) tv_fetch(a, stage + f * TV_TILE, s, f);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
+        double acc = 0.0, xv = 0.0;
+        if (s > 0) xv = tv_load(a.xw + 16 * q, lane);
+        for (int K = 0; K < nk; K++) {
+            asm volatile("cp.async.wait_group %0;" :: "n"(TV_STAGES - 2) : "memory");
+            __syncthreads();   // block K is in, block K - 1 consumed
+            if (K + TV_STAGES - 1 < nk)
+                tv_fetch(a, stage + ((K + TV_STAGES - 1) % TV_STAGES) * TV_TILE, s, K + TV_STAGES - 1);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            xv = tv_wait(a, a.xw + (long long)K * TV_NB + 16 * q, xv, lane);
+            __syncwarp();
+            if (lane < 16) xs[lane] = xv;
+            __syncwarp();
+            if (K + 1 < s) xv = tv_load(a.xw + (long long)(K + 1) * TV_NB + 16 * q, lane);
+            const double *T = stage + (K % TV_STAGES) * TV_TILE + 16 * q * TV_LD + i;
+#pragma unroll
+            for (int k = 0; k < 16; k++) acc = fma(T[k * TV_LD], xs[k], acc);
+        }
+        red[q * TV_NB + i] = acc;
+        __syncthreads();
+        if (tid < TV_NB) st[i] = b - ((red[i] + red[TV_NB + i]) + (red[2 * TV_NB + i] + red[3 * TV_NB + i]));
+        __syncthreads();
+        double v = 0.0;
+        if ((warp & 1) || q < 2) {   // rows < 32 end at column 31
+#pragma unroll
+            for (int k = 0; k < 16; k++) v = fma(X[(16 * q + k) * TV_LD + i], st[16 * q + k], v);
+        }
+        if (fold) {
+            xv = tv_wait(a, a.xw + (long long)(s - 1) * TV_NB + 16 * q, xv, lane);
+            __syncwarp();
+            if (lane < 16) xs[lane] = xv;
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < 16; k++) v = fma(-M[k], xs[k], v);
+        }
+        red[q * TV_NB + i] = v;
+        __syncthreads();
+        if (tid < TV_NB) {
+            const double r = (red[i] + red[TV_NB + i]) + (red[2 * TV_NB + i] + red[3 * TV_NB + i]);
+            // the "not yet known" pattern is a NaN: publish another NaN in its place
+            const double o = __double_as_longlong(r) == -1ll ? __longlong_as_double(0x7ff8000000000000ll) : r;
+            *(volatile double *)(a.xw + p) = o;
+            if (p < a.n) a.x[(long long)(a.fwd ? p : a.n - 1 - p) * a.incx] = r;
+        }
+        __syncthreads();   // shared memory is reused by the next block
     }
 }
 
@@ -345,12 +530,6 @@ extern "C" gbx_status gbx_dsymv(gbx_ctx *ctx, char uplo, int n, double alpha, co
     return gbx_check_launch(ctx, "dsymv");
 }
 
-namespace gbx_gemm {
-// inverted 64x64 diagonal blocks of op(A) (trsm.cu)
-gbx_status trinv_diag_blocks(gbx_ctx *ctx, int na, const double *A, long long lda, int tr, int lower, int unit,
-                             double *inv);
-}
-
 extern "C" gbx_status gbx_dtrsv(gbx_ctx *ctx, char uplo, char trans, char diag, int n, const double *A, int lda,
                                 double *x, int incx)
 {
@@ -359,29 +538,37 @@ extern "C" gbx_status gbx_dtrsv(gbx_ctx *ctx, char uplo, char trans, char diag, 
     if (info) return gbx_fail(ctx, GBX_ERR_ARG, "DTRSV parameter %d", info);
     if (n == 0) return GBX_OK;
     const int tri = gbx_op_tri(uplo, trans, diag);
-    const int fwd = (tri & gbx_gemm::TRI_LOWER) != 0;
-    const int tr = !gbx_lsame(trans, 'N');
-    const int nblk = (n + TV_NB - 1) / TV_NB, npad = nblk * TV_NB;
-    double *inv, *w;
+    const int nblk = (n + TV_NB - 1) / TV_NB;
+    double *xw;
+    TrsvArgs p{};
     gbx_status st;
-    if ((st = gbx_ws(ctx, GBX_WS_TMP1, sizeof(double) * (size_t)nblk * TV_NB * TV_NB, (void **)&inv)) != GBX_OK)
-        return st;
-    if ((st = gbx_ws(ctx, GBX_WS_TMP2, sizeof(double) * (size_t)npad, (void **)&w)) != GBX_OK) return st;
-    if ((st = gbx_gemm::trinv_diag_blocks(ctx, n, A, lda, tr, fwd, (tri & gbx_gemm::TRI_UNIT) != 0, inv)) !=
-        GBX_OK)
-        return st;
-    double *xb = x + base_off(n, incx);
-    const int sms = gbx_ctx_sms(ctx);
-    gather_vec<<<std::min(sms * 4, (npad + 255) / 256), 256, 0, S(ctx)>>>(n, xb, incx, w, npad);
-    gbx_count_launch(ctx, 1);
+    if ((st = gbx_ws(ctx, GBX_WS_TMP2, sizeof(double) * (size_t)nblk * TV_NB, (void **)&xw)) != GBX_OK) return st;
+    if ((st = gbx_ctx_status(ctx, &p.status, &p.status_host)) != GBX_OK) return st;
+    p.n = n;
+    p.nblk = nblk;
+    p.fwd = (tri & gbx_gemm::TRI_LOWER) != 0;
+    p.tr = !gbx_lsame(trans, 'N');
+    p.unit = (tri & gbx_gemm::TRI_UNIT) != 0;
+    p.A = A;
+    p.lda = lda;
+    p.x = x + base_off(n, incx);
+    p.incx = incx;
+    p.xw = xw;
+    // every value "not yet known" (all bits set)
+    cudaError_t e = cudaMemsetAsync(xw, 0xFF, sizeof(double) * (size_t)nblk * TV_NB, S(ctx));
+    // a per-device function attribute; setting it is a cheap host call
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(trsv_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TV_SMEM);
+    if (e != cudaSuccess) return gbx_fail(ctx, GBX_ERR_CUDA, "dtrsv: %s", cudaGetErrorString(e));
+    const int grid = std::min(nblk, gbx_ctx_sms(ctx));   // one CTA per SM is always resident
+    void *args[] = {&p};
     gbx_timer_begin(ctx, GBX_TIMER_GEMV);
-    for (int s = 0; s < nblk; s++) {
-        const int J = fwd ? s : nblk - 1 - s;
-        const int rows = fwd ? std::max(0, n - (J + 1) * TV_NB) : J * TV_NB;
-        const int grid = std::max(1, (rows + 255) / 256);
-        trsv_step<<<grid, 256, 0, S(ctx)>>>(n, J, fwd, tr, A, lda, inv, w, xb, incx);
-    }
+    e = cudaLaunchCooperativeKernel((const void *)trsv_solve, dim3(grid), dim3(TV_THREADS), args, TV_SMEM, S(ctx));
     gbx_timer_end(ctx);
-    gbx_count_launch(ctx, (uint64_t)nblk);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return gbx_fail(ctx, GBX_ERR_CUDA, "dtrsv: %s", cudaGetErrorString(e));
+    }
+    gbx_count_launch(ctx, 1);
     return gbx_check_launch(ctx, "dtrsv");
 }
