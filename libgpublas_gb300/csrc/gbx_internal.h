@@ -35,10 +35,15 @@ gbx_status gbx_fail(gbx_ctx *ctx, gbx_status st, const char *fmt, ...);
 #define GBX_WS_BATCH    10  /* grouped/batched descriptors                  */
 #define GBX_WS_STAGE_D  11
 #define GBX_WS_TRSM_X   12  /* dtrsm_ozaki: inverse of the triangle          */
-#define GBX_WS_SPARE13  13  /* unused                                      */
+#define GBX_WS_SGEMM    13  /* SGEMM: bf16 planes of both operands          */
 #define GBX_WS_GEMV     14  /* gemv partial sums                            */
 #define GBX_WS_RED      15  /* reduction partials                           */
 gbx_status gbx_ws(gbx_ctx *ctx, int slot, size_t bytes, void **ptr);
+/* Whether gbx_ws would return without allocating. */
+int gbx_ws_ready(const gbx_ctx *ctx, int slot, size_t bytes);
+/* A number that differs from call to call on a context (a kernel's mark in
+ * device memory is recognised by it, so the mark need not be reset). */
+int gbx_ctx_epoch(gbx_ctx *ctx);
 /* Pinned host scratch owned by the context (for small results). */
 gbx_status gbx_pinned(gbx_ctx *ctx, size_t bytes, void **ptr);
 void gbx_count_launch(gbx_ctx *ctx, int n);
@@ -50,8 +55,8 @@ void gbx_timer_end(gbx_ctx *ctx);
  * mapped host mirror, which such kernels set to the status when it is
  * nonzero as they finish.  gbx_ctx_sync reports a nonzero mirror (5: a
  * non-finite Ozaki operand, GBX_ERR_ARG; else GBX_ERR_TIMEOUT) and clears
- * both.  Word 0 is the status; word 12 is the DPOTRF step's last-CTA
- * counter, which its kernel resets. */
+ * both.  Word 0 is the status, word 4 that of the SGEMM tensor kernel; word
+ * 12 is the DPOTRF step's last-CTA counter, which its kernel resets. */
 gbx_status gbx_ctx_status(gbx_ctx *ctx, int **dev_status, int **host_mirror);
 /* Check cudaGetLastError after a launch, record and map it. */
 gbx_status gbx_check_launch(gbx_ctx *ctx, const char *what);
@@ -162,6 +167,8 @@ int gbx_check_gemm_args(char ta, char tb, int m, int n, int k, int lda, int ldb,
 // FP64 GEMM core block tile (64, 32 or 16) for an m x n output (a triangle
 // when triangular) on `sms` SMs
 int gbx_dgemm_tile_choice(int m, int n, int triangular, int sms);
+// whether an m x n x k SGEMM runs on the tensor cores
+int gbx_sgemm_tensor_choice(int m, int n, int k, int sms);
 int gbx_check_syrk_args(char uplo, char trans, int n, int k, int lda, int ldc);
 int gbx_check_trxm_args(char side, char uplo, char ta, char diag, int m, int n, int lda, int ldb);
 int gbx_check_rank_k_args(char uplo, char trans, int allowed, int n, int k, int lda, int ldc);

@@ -42,6 +42,7 @@ struct gbx_ctx {
     void  *pinned;
     size_t pinned_bytes;
     uint64_t launches;
+    int epoch;
     int *status_dev;     // device status words of kernels with bounded waits ([0]; [12] a counter)
     int *status_host;    // mapped pinned mirror of status_dev[0], written by the kernels on failure
     int *status_mirror;  // the mirror's device address
@@ -338,6 +339,17 @@ extern "C" gbx_status gbx_ws(gbx_ctx *c, int slot, size_t bytes, void **ptr)
     }
     *ptr = c->ws[slot];
     return GBX_OK;
+}
+
+extern "C" int gbx_ws_ready(const gbx_ctx *c, int slot, size_t bytes)
+{
+    return c && slot >= 0 && slot < GBX_WS_SLOTS && c->ws_bytes[slot] >= bytes;
+}
+
+extern "C" int gbx_ctx_epoch(gbx_ctx *c)
+{
+    c->epoch = (int)((unsigned)c->epoch + 1u);
+    return c->epoch;
 }
 
 extern "C" gbx_status gbx_ctx_reserve(gbx_ctx *c, size_t bytes)

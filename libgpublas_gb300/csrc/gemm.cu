@@ -56,8 +56,17 @@ template gbx_status scale_matrix<double>(gbx_ctx *, int, int, double, double *, 
 template gbx_status scale_matrix<fcplx>(gbx_ctx *, int, int, fcplx, fcplx *, long long, int, int);
 template gbx_status scale_matrix<dcplx>(gbx_ctx *, int, int, dcplx, dcplx *, long long, int, int);
 
+// The same kernel behind a device-side condition.
+template <typename T, int TM, int TN, int BK>
+__global__ void __launch_bounds__(GEMM_THREADS)
+gemm_simt_if(GemmArgs<T> p, const int *flag, int epoch)
+{
+    if (*flag != epoch) return;
+    gemm_simt_tile<T, TM, TN, BK>(p, blockIdx.x);
+}
+
 template <typename T, int TM>
-gbx_status launch_gemm_tile(gbx_ctx *ctx, GemmArgs<T> p, const char *what)
+gbx_status launch_gemm_tile(gbx_ctx *ctx, GemmArgs<T> p, const char *what, const int *flag = nullptr, int epoch = 0)
 {
     constexpr int TN = TM, BK = TM == 1 ? 16 : 8;
     constexpr int BM = 16 * TM, BN = 16 * TN;
@@ -70,6 +79,13 @@ gbx_status launch_gemm_tile(gbx_ctx *ctx, GemmArgs<T> p, const char *what)
         blocks = (long long)p.tiles_m * (p.tiles_m + 1) / 2;
     }
     if (blocks > 0x7fffffffLL) return gbx_fail(ctx, GBX_ERR_UNSUPPORTED, "%s: grid too large", what);
+    if constexpr (std::is_same<T, float>::value) {
+        if (flag) {
+            gemm_simt_if<T, TM, TN, BK><<<(unsigned)blocks, GEMM_THREADS, 0, S(ctx)>>>(p, flag, epoch);
+            gbx_count_launch(ctx, 1);
+            return gbx_check_launch(ctx, what);
+        }
+    }
     gbx_timer_begin(ctx, GBX_TIMER_GEMM_FP64);
     gemm_simt_kernel<T, TM, TN, BK><<<(unsigned)blocks, GEMM_THREADS, 0, S(ctx)>>>(p);
     gbx_timer_end(ctx);
@@ -94,7 +110,7 @@ gbx_status launch_gemm_tile(gbx_ctx *ctx, GemmArgs<T> p, const char *what)
 // operand reuse), 64x64 and 32x32 for complex double (its 8x8 register tile
 // would not fit), then smaller for the skinny and small products.
 template <typename T>
-gbx_status launch_gemm(gbx_ctx *ctx, GemmArgs<T> p, const char *what)
+static gbx_status choose_and_launch(gbx_ctx *ctx, GemmArgs<T> p, const char *what, const int *flag, int epoch)
 {
     if (p.m <= 0 || p.n <= 0) return GBX_OK;
     const long long want = 2LL * gbx_ctx_sms(ctx);
@@ -108,14 +124,23 @@ gbx_status launch_gemm(gbx_ctx *ctx, GemmArgs<T> p, const char *what)
         if (bm == 32) return launch_gemm_tile<T, 2>(ctx, p, what);
         return launch_gemm_tile<T, 1>(ctx, p, what);
     } else if constexpr (sizeof(T) <= 8) {
-        if (tiles(128) >= want) return launch_gemm_tile<T, 8>(ctx, p, what);
-        if (tiles(64) >= want) return launch_gemm_tile<T, 4>(ctx, p, what);
-        if (tiles(32) >= want) return launch_gemm_tile<T, 2>(ctx, p, what);
-        return launch_gemm_tile<T, 1>(ctx, p, what);
+        if (tiles(128) >= want) return launch_gemm_tile<T, 8>(ctx, p, what, flag, epoch);
+        if (tiles(64) >= want) return launch_gemm_tile<T, 4>(ctx, p, what, flag, epoch);
+        if (tiles(32) >= want) return launch_gemm_tile<T, 2>(ctx, p, what, flag, epoch);
+        return launch_gemm_tile<T, 1>(ctx, p, what, flag, epoch);
     } else {
         if (tiles(64) >= want) return launch_gemm_tile<T, 4>(ctx, p, what);
         return launch_gemm_tile<T, 2>(ctx, p, what);
     }
+}
+template <typename T>
+gbx_status launch_gemm(gbx_ctx *ctx, GemmArgs<T> p, const char *what)
+{
+    return choose_and_launch<T>(ctx, p, what, nullptr, 0);
+}
+gbx_status launch_gemm_if(gbx_ctx *ctx, GemmArgs<float> p, const char *what, const int *flag, int epoch)
+{
+    return choose_and_launch<float>(ctx, p, what, flag, epoch);
 }
 template gbx_status launch_gemm<float>(gbx_ctx *, GemmArgs<float>, const char *);
 template gbx_status launch_gemm<double>(gbx_ctx *, GemmArgs<double>, const char *);

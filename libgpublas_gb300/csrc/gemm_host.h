@@ -8,6 +8,10 @@
 namespace gbx_gemm {
 template <typename T>
 gbx_status launch_gemm(gbx_ctx *ctx, GemmArgs<T> p, const char *what);
+// The SIMT SGEMM of a full C, which does nothing unless *flag == epoch when it runs.
+gbx_status launch_gemm_if(gbx_ctx *ctx, GemmArgs<float> p, const char *what, const int *flag, int epoch);
+// SGEMM on the tensor cores (sgemm_tc.cu); *done: the call was taken.
+gbx_status sgemm_tensor(gbx_ctx *ctx, const GemmArgs<float> &p, const char *what, bool *done);
 // C = beta * C on the whole matrix or one triangle (beta == 0 sets zero);
 // herm: the diagonal's imaginary part is set to zero (Hermitian C).
 template <typename T>

@@ -18,6 +18,7 @@
 #include "gemm_host.h"
 
 #include <cuda_runtime.h>
+#include <type_traits>
 
 using namespace gbx_gemm;
 
@@ -73,6 +74,11 @@ gbx_status gemm_t(gbx_ctx *ctx, const char *nm, char ta, char tb, int m, int n, 
     p.B = B; p.ldb = ldb; p.tb = !gbx_lsame(tb, 'N'); p.conjb = gbx_lsame(tb, 'C');
     p.alpha = alpha; p.beta = beta;
     p.C = C; p.ldc = ldc;
+    if constexpr (std::is_same<T, float>::value) {
+        bool done;
+        const gbx_status st = sgemm_tensor(ctx, p, nm, &done);
+        if (done || st != GBX_OK) return st;
+    }
     return launch_gemm<T>(ctx, p, nm);
 }
 
