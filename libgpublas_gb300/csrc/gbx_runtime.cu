@@ -250,7 +250,10 @@ extern "C" gbx_status gbx_ctx_status(gbx_ctx *c, int **dev_status, int **host_mi
     if (!c->status_dev) {
         if (cudaMalloc((void **)&c->status_dev, 64) != cudaSuccess)
             return gbx_fail(c, GBX_ERR_ALLOC, "status word");
-        if (cudaMemset(c->status_dev, 0, 64) != cudaSuccess ||
+        // cleared before anything on the context's streams, which do not
+        // order with the legacy stream of a plain cudaMemset
+        if (cudaMemsetAsync(c->status_dev, 0, 64, c->stream) != cudaSuccess ||
+            cudaStreamSynchronize(c->stream) != cudaSuccess ||
             cudaHostAlloc((void **)&c->status_host, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
             cudaHostGetDevicePointer((void **)&c->status_mirror, c->status_host, 0) != cudaSuccess) {
             cudaGetLastError();
