@@ -1,6 +1,8 @@
 // l1_kernels.cuh — device code of the Level-1 routines (included by l1.cu).
 #pragma once
 
+#include "launch.cuh"
+
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -30,10 +32,56 @@ __device__ __forceinline__ double block_sum(double v)
     double r = 0.0;
     if (w == 0) {
         r = l < L1_THREADS / 32 ? s_warp[l] : 0.0;
-        r = warp_sum(r);
+#pragma unroll
+        for (int o = L1_THREADS / 64; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
     }
     __syncthreads();
     return r;
+}
+
+// The sums of a, b and c over the block, in thread 0.
+__device__ __forceinline__ void block_sum3(double &a, double &b, double &c)
+{
+    __shared__ double s_warp[3][L1_THREADS / 32];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {   // three chains: their latencies overlap
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+        c += __shfl_xor_sync(0xffffffffu, c, o);
+    }
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    if (l == 0) { s_warp[0][w] = a; s_warp[1][w] = b; s_warp[2][w] = c; }
+    __syncthreads();
+    if (w == 0) {
+        a = l < L1_THREADS / 32 ? s_warp[0][l] : 0.0;
+        b = l < L1_THREADS / 32 ? s_warp[1][l] : 0.0;
+        c = l < L1_THREADS / 32 ? s_warp[2][l] : 0.0;
+#pragma unroll
+        for (int o = L1_THREADS / 64; o > 0; o >>= 1) {
+            a += __shfl_xor_sync(0xffffffffu, a, o);
+            b += __shfl_xor_sync(0xffffffffu, b, o);
+            c += __shfl_xor_sync(0xffffffffu, c, o);
+        }
+    }
+    __syncthreads();
+}
+
+// Second half of a reduction in the same launch: true in every thread of the
+// block that finishes last, once the partials that the blocks' threads 0 wrote
+// before the call can be read (with __ldcg).  The counter is zero before the
+// launch and again after it.  A second launch cost 2 to 4 us a call, as much as
+// a short vector's whole first pass.
+__device__ __forceinline__ bool last_block(unsigned *counter)
+{
+    __shared__ unsigned s_last;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(counter, 1u) == gridDim.x - 1;
+        if (s_last) *counter = 0u;
+        __threadfence();
+    }
+    __syncthreads();
+    return s_last != 0u;
 }
 
 __device__ __forceinline__ double2 ldg2(const double2 *p) { return __ldg(p); }
@@ -48,6 +96,7 @@ static __global__ void zero_index(int *res) { *res = 0; }
 static __global__ void __launch_bounds__(L1_THREADS)
 axpy_unit(int n, double a, const double *__restrict__ x, double *__restrict__ y)
 {
+    gbx_launch::pdl_enter();
     const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long stride = (long long)gridDim.x * blockDim.x;
     const unsigned px = (unsigned)((uintptr_t)x & 15), py = (unsigned)((uintptr_t)y & 15);
@@ -80,6 +129,7 @@ axpy_unit(int n, double a, const double *__restrict__ x, double *__restrict__ y)
 static __global__ void __launch_bounds__(L1_THREADS)
 axpy_strided(int n, double a, const double *__restrict__ x, int incx, double *__restrict__ y, int incy)
 {
+    gbx_launch::pdl_enter();
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         double *yp = y + i * incy;
@@ -90,6 +140,7 @@ axpy_strided(int n, double a, const double *__restrict__ x, int incx, double *__
 static __global__ void __launch_bounds__(L1_THREADS)
 scal_kernel(int n, double a, double *__restrict__ x, int incx)
 {
+    gbx_launch::pdl_enter();
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
         x[i * incx] = (a == 0.0) ? 0.0 : a * x[i * incx];
@@ -97,9 +148,10 @@ scal_kernel(int n, double a, double *__restrict__ x, int incx)
 
 // ----------------------------------------------------------------- ddot ---
 static __global__ void __launch_bounds__(L1_THREADS)
-dot_partial(int n, const double *__restrict__ x, int incx, const double *__restrict__ y, int incy,
-            double *__restrict__ part)
+dot_kernel(int n, const double *__restrict__ x, int incx, const double *__restrict__ y, int incy,
+           double *__restrict__ part, unsigned *counter, double *__restrict__ res)
 {
+    gbx_launch::pdl_enter();
     const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long stride = (long long)gridDim.x * blockDim.x;
     double s0 = 0.0, s1 = 0.0;
@@ -110,11 +162,19 @@ dot_partial(int n, const double *__restrict__ x, int incx, const double *__restr
         const long long n2 = (long long)(n - peel) >> 1;
         const double2 *x2 = (const double2 *)(x + peel), *y2 = (const double2 *)(y + peel);
         long long i = tid;
-        for (; i + stride < n2; i += 2 * stride) {
-            double2 xa = ldg2(x2 + i), xb = ldg2(x2 + i + stride);
-            double2 ya = ldg2(y2 + i), yb = ldg2(y2 + i + stride);
-            s0 = fma(xa.x, ya.x, s0); s1 = fma(xa.y, ya.y, s1);
-            s0 = fma(xb.x, yb.x, s0); s1 = fma(xb.y, yb.y, s1);
+        // eight 128-bit loads in flight per thread
+        for (; i + 3 * stride < n2; i += 4 * stride) {
+            double2 xv[4], yv[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                xv[u] = ldg2(x2 + i + u * stride);
+                yv[u] = ldg2(y2 + i + u * stride);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                s0 = fma(xv[u].x, yv[u].x, s0);
+                s1 = fma(xv[u].y, yv[u].y, s1);
+            }
         }
         for (; i < n2; i += stride) {
             double2 xa = ldg2(x2 + i), ya = ldg2(y2 + i);
@@ -125,15 +185,15 @@ dot_partial(int n, const double *__restrict__ x, int incx, const double *__restr
         for (long long i = tid; i < n; i += stride) s0 = fma(x[i * incx], y[i * incy], s0);
     }
     double b = block_sum(s0 + s1);
+    if (gridDim.x == 1) {
+        if (threadIdx.x == 0) *res = b;
+        return;
+    }
     if (threadIdx.x == 0) part[blockIdx.x] = b;
-}
-
-static __global__ void __launch_bounds__(L1_THREADS)
-sum_partials(const double *__restrict__ part, int g, double *__restrict__ res)
-{
+    if (!last_block(counter)) return;
     double s = 0.0;
-    for (int i = threadIdx.x; i < g; i += blockDim.x) s += part[i];
-    double b = block_sum(s);
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += L1_THREADS) s += __ldcg(part + i);
+    b = block_sum(s);
     if (threadIdx.x == 0) *res = b;
 }
 
@@ -255,9 +315,36 @@ __device__ __forceinline__ bool all_medium4(double a, double b, double c, double
     return !__any_sync(__activemask(), out);
 }
 
-static __global__ void __launch_bounds__(L1_THREADS)
-nrm2_partial(int n, const double *__restrict__ x, int incx, double *__restrict__ part)
+__device__ __forceinline__ double blue_finish(double asml, double amed, double abig)
 {
+    double scl, sumsq;
+    if (abig > 0.0) {
+        if (amed > 0.0 || isnan(amed)) abig = fma(amed * Blue::sbig, Blue::sbig, abig);
+        scl = 1.0 / Blue::sbig;
+        sumsq = abig;
+    } else if (asml > 0.0) {
+        if (amed > 0.0 || isnan(amed)) {
+            const double am = sqrt(amed), as = sqrt(asml) / Blue::ssml;
+            const double ymin = as > am ? am : as, ymax = as > am ? as : am;
+            scl = 1.0;
+            const double r = ymin / ymax;
+            sumsq = ymax * ymax * (1.0 + r * r);
+        } else {
+            scl = 1.0 / Blue::ssml;
+            sumsq = asml;
+        }
+    } else {
+        scl = 1.0;
+        sumsq = amed;
+    }
+    return scl * sqrt(sumsq);
+}
+
+static __global__ void __launch_bounds__(L1_THREADS)
+nrm2_kernel(int n, const double *__restrict__ x, int incx, double *__restrict__ part, unsigned *counter,
+            double *__restrict__ res)
+{
+    gbx_launch::pdl_enter();
     const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long stride = (long long)gridDim.x * blockDim.x;
     double asml = 0.0, amed = 0.0, abig = 0.0;
@@ -294,52 +381,27 @@ nrm2_partial(int n, const double *__restrict__ x, int incx, double *__restrict__
     } else {
         for (long long i = tid; i < n; i += stride) blue_acc(x[i * incx], asml, amed, abig);
     }
-    double s = block_sum(asml);
-    double m = block_sum(amed);
-    double b = block_sum(abig);
-    if (threadIdx.x == 0) {
-        part[3 * blockIdx.x + 0] = s;
-        part[3 * blockIdx.x + 1] = m;
-        part[3 * blockIdx.x + 2] = b;
-    }
-}
-
-__device__ __forceinline__ double blue_finish(double asml, double amed, double abig)
-{
-    double scl, sumsq;
-    if (abig > 0.0) {
-        if (amed > 0.0 || isnan(amed)) abig = fma(amed * Blue::sbig, Blue::sbig, abig);
-        scl = 1.0 / Blue::sbig;
-        sumsq = abig;
-    } else if (asml > 0.0) {
-        if (amed > 0.0 || isnan(amed)) {
-            const double am = sqrt(amed), as = sqrt(asml) / Blue::ssml;
-            const double ymin = as > am ? am : as, ymax = as > am ? as : am;
-            scl = 1.0;
-            const double r = ymin / ymax;
-            sumsq = ymax * ymax * (1.0 + r * r);
-        } else {
-            scl = 1.0 / Blue::ssml;
-            sumsq = asml;
+    // most vectors have no element outside the medium range: one sum instead of three
+    const int outside = __syncthreads_or(asml != 0.0 || abig != 0.0);
+    if (outside) block_sum3(asml, amed, abig);
+    else amed = block_sum(amed);
+    if (gridDim.x > 1) {
+        if (threadIdx.x == 0) {
+            part[3 * blockIdx.x + 0] = asml;
+            part[3 * blockIdx.x + 1] = amed;
+            part[3 * blockIdx.x + 2] = abig;
         }
-    } else {
-        scl = 1.0;
-        sumsq = amed;
+        if (!last_block(counter)) return;
+        asml = amed = abig = 0.0;
+        for (int i = threadIdx.x; i < (int)gridDim.x; i += L1_THREADS) {
+            asml += __ldcg(part + 3 * i);
+            amed += __ldcg(part + 3 * i + 1);
+            abig += __ldcg(part + 3 * i + 2);
+        }
+        if (__syncthreads_or(asml != 0.0 || abig != 0.0)) block_sum3(asml, amed, abig);
+        else amed = block_sum(amed);
     }
-    return scl * sqrt(sumsq);
-}
-
-static __global__ void __launch_bounds__(L1_THREADS)
-nrm2_finish(const double *__restrict__ part, int g, double *__restrict__ res)
-{
-    double s = 0.0, m = 0.0, b = 0.0;
-    for (int i = threadIdx.x; i < g; i += blockDim.x) {
-        s += part[3 * i]; m += part[3 * i + 1]; b += part[3 * i + 2];
-    }
-    s = block_sum(s);
-    m = block_sum(m);
-    b = block_sum(b);
-    if (threadIdx.x == 0) *res = blue_finish(s, m, b);
+    if (threadIdx.x == 0) *res = blue_finish(asml, amed, abig);
 }
 
 // ------------------------------------------------------- idamax / idamin ---
@@ -347,8 +409,8 @@ nrm2_finish(const double *__restrict__ part, int g, double *__restrict__ res)
 // an element is the bit pattern of |x_i| (monotone in |x_i| for non-NaN
 // values); for the arg-min the key is its complement.  NaN gets key 0 and
 // never beats a number, which is netlib's rule (a NaN never compares greater
-// or smaller) except when x_1 itself is NaN: netlib then returns 1, handled in
-// the finishing kernel.
+// or smaller) except when x_1 itself is NaN: netlib then returns 1, handled by
+// the block that writes the result.
 template <bool IS_MIN>
 __device__ __forceinline__ unsigned long long amax_key(double v)
 {
@@ -391,9 +453,10 @@ __device__ __forceinline__ void block_best(unsigned long long &k, long long &i)
 
 template <bool IS_MIN>
 static __global__ void __launch_bounds__(L1_THREADS)
-iamax_partial(int n, const double *__restrict__ x, int incx, unsigned long long *__restrict__ keys,
-              long long *__restrict__ idx)
+iamax_kernel(int n, const double *__restrict__ x, int incx, unsigned long long *__restrict__ keys,
+             long long *__restrict__ idx, unsigned *counter, int *__restrict__ res)
 {
+    gbx_launch::pdl_enter();
     const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long stride = (long long)gridDim.x * blockDim.x;
     unsigned long long bk = 0ull;
@@ -444,20 +507,20 @@ iamax_partial(int n, const double *__restrict__ x, int incx, unsigned long long 
         }
     }
     block_best(bk, bi);
-    if (threadIdx.x == 0) { keys[blockIdx.x] = bk; idx[blockIdx.x] = bi; }
-}
-
-template <bool IS_MIN>
-static __global__ void __launch_bounds__(L1_THREADS)
-iamax_finish(const double *__restrict__ x, const unsigned long long *__restrict__ keys,
-             const long long *__restrict__ idx, int g, int *__restrict__ res)
-{
-    unsigned long long bk = 0ull;
-    long long bi = 0x7fffffffffffffffll;
-    for (int i = threadIdx.x; i < g; i += blockDim.x)
-        if (better(keys[i], idx[i], bk, bi)) { bk = keys[i]; bi = idx[i]; }
-    block_best(bk, bi);
-    if (threadIdx.x == 0) *res = isnan(x[0]) ? 1 : (int)(bi + 1);
+    if (gridDim.x > 1) {
+        if (threadIdx.x == 0) { keys[blockIdx.x] = bk; idx[blockIdx.x] = bi; }
+        if (!last_block(counter)) return;
+        bk = 0ull;
+        bi = 0x7fffffffffffffffll;
+        for (int i = threadIdx.x; i < (int)gridDim.x; i += L1_THREADS) {
+            const unsigned long long k = __ldcg(keys + i);
+            const long long e = __ldcg(idx + i);
+            if (better(k, e, bk, bi)) { bk = k; bi = e; }
+        }
+        block_best(bk, bi);
+    }
+    // x_1 NaN: netlib returns 1
+    if (threadIdx.x == 0) *res = abs_bits(x[0]) > 0x7FF0000000000000ull ? 1 : (int)(bi + 1);
 }
 
 }  // namespace gbx_l1

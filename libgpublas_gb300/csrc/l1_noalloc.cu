@@ -82,6 +82,17 @@ dot_chunk_partial(int n, const double *__restrict__ x, int incx, const double *_
     if (threadIdx.x == 0) part[blockIdx.x] = b;
 }
 
+// The partials' sum by one block, as a launch of its own: the array is shared
+// by every call on the device, so no counter could tell the last block.
+__global__ void __launch_bounds__(L1_THREADS)
+sum_partials(const double *__restrict__ part, int g, double *__restrict__ res)
+{
+    double s = 0.0;
+    for (int i = threadIdx.x; i < g; i += blockDim.x) s += part[i];
+    double b = block_sum(s);
+    if (threadIdx.x == 0) *res = b;
+}
+
 }  // namespace
 
 extern "C" gbx_status gbx_ddot_noalloc(void *stream, int n, const double *x, int incx, const double *y,

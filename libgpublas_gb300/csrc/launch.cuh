@@ -1,0 +1,39 @@
+// launch.cuh — kernel launches that overlap the previous kernel's end
+// (programmatic stream serialisation).  A kernel launched with launch_pdl may
+// have its CTAs placed on the SMs before the kernel ahead of it in the stream
+// has finished; every thread of it calls pdl_enter() before it touches memory,
+// which waits until that kernel is complete and its writes are visible.
+// Without it each of a program's short calls pays its launch, about 2 us, after
+// the call before has drained.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <utility>
+
+namespace gbx_launch {
+
+// First statement of a kernel launched with launch_pdl: the next kernel may be
+// placed from here on, this one's work starts when the previous is complete.
+__device__ __forceinline__ void pdl_enter()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+cudaError_t launch_pdl(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A &&...args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(std::forward<A>(args))...);
+}
+
+}  // namespace gbx_launch
