@@ -20,6 +20,19 @@ __device__ __forceinline__ void pdl_enter()
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// Hand-over between the warps of a CTA on named barrier id (1-15) of `threads`
+// threads: the producing warp arrives without waiting, the others wait.
+__device__ __forceinline__ void bar_arrive(int id, int threads)
+{
+    __threadfence_block();
+    __syncwarp();
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void bar_wait(int id, int threads)
+{
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
 template <typename... P, typename... A>
 cudaError_t launch_pdl(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A &&...args)
 {

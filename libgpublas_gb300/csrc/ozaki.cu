@@ -33,6 +33,7 @@
 // at most half the SMs run as half-width tiles.
 #include "gbx_internal.h"
 #include "gemm_host.h"
+#include "launch.cuh"
 #include "tc_ptx.cuh"
 
 #include <cuda.h>
@@ -2652,78 +2653,142 @@ extern "C" gbx_status gbx_dsyrk_ozaki(gbx_ctx *ctx, char uplo, char trans, int n
 // well-conditioned diagonal blocks of a Cholesky factorization the extra
 // error of applying the inverse is a factor cond(op(A)) on the rounding of X.
 namespace {
-// Inverse of a triangular matrix of order n <= 256 in FP64, one warp per
-// column of the inverse.  An upper triangle U is handled as the lower
-// triangle L' = P U P (P the order-reversing permutation; U^-1 = P L'^-1 P).
-// Column j of W = L'^-1 solves L' w = e_j by forward substitution, lane l
-// holding rows l, l + 32, ...: at step i the owner lane scales w_i by the
-// inverse diagonal entry, broadcasts it, and every lane subtracts
-// w_i L'(r, i) from its rows r > i.  The columns of L' stream through shared
-// memory 16 at a time.  Each step costs one FP64 warp instruction per
-// 32-row slot still below the pivot, and an FP64 warp instruction occupies
-// the SM's 2-lane FP64 pipe for 16 cycles whatever its predicate: CTAs of 2
-// warps spread the columns over as many SMs as possible, and slots above
-// the pivot are skipped.  The FP64 DTRSM of the identity this replaces ran
-// its small GEMM updates on one or two SMs (~270 µs for n = 128).
-// X = W, or W^T for op = 'T'/'C'.
-constexpr int OZ_TI_WARPS = 2, OZ_TI_PANEL = 16, OZ_TI_NMAX = 256;
+// Inverse of a triangular matrix of order n <= 256 in FP64.  An upper triangle
+// U is handled as the lower triangle L' = P U P (P the order-reversing
+// permutation; U^-1 = P L'^-1 P); X = W = L'^-1, or W^T for op = 'T'/'C'.
+// Two launches:
+//   * oz_trinv_diag: the 32 x 32 diagonal blocks, one CTA of four warps each;
+//   * oz_trinv_kernel: forward substitution by blocks of 32 rows, two columns
+//     of the inverse per CTA (j and n - 1 - j: together they have about n rows
+//     to solve whatever j is), one thread per row.  Block I of both columns is
+//     the inverse diagonal block times the running right-hand side; then every
+//     row below subtracts its 32 products, from columns of L' that were loaded
+//     during the block before.
+// The bound is the FP64 pipe (2 lanes per clock per SM, n^2 / 2 FMAs per CTA: 16
+// us at n = 256) and eight block steps.  n = 256: TRINV_US us in all; one warp
+// per column stepping through its 256 rows one by one took 235 us.
+constexpr int OZ_TI_NMAX = 256, OZ_TI_BLK = 32;
 
-__global__ void __launch_bounds__(OZ_TI_WARPS * 32)
-oz_trinv_kernel(int n, const double *__restrict__ T, long long ldt, int lower, int unit, int trans,
-                double *__restrict__ X, long long ldx)
-{
-    __shared__ double sT[OZ_TI_PANEL][OZ_TI_NMAX];
-    __shared__ double sR[OZ_TI_NMAX];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // L'(r, c) for r >= c
-    auto tget = [&](int r, int c) -> double {
+struct OzTriView {
+    const double *T;
+    long long ld;
+    int n, lower;
+    // L'(r, c), r >= c
+    __device__ __forceinline__ double operator()(int r, int c) const
+    {
         const int rr = lower ? r : n - 1 - r, cc = lower ? c : n - 1 - c;
-        return T[(long long)cc * ldt + rr];
+        return T[(long long)cc * ld + rr];
+    }
+};
+
+// D: per block 32 x 32, column-major.  Lane j substitutes for column j, warp w
+// holding rows 4u + w; the warp of row i + 1 finishes and publishes it before
+// its other rows and does not wait for the other warps (an FP64 warp
+// instruction takes 64 cycles on its sub-partition, so a single warp took 24 us).
+__global__ void __launch_bounds__(128)
+oz_trinv_diag(OzTriView L, int unit, double *__restrict__ D)
+{
+    using namespace gbx_launch;
+    pdl_enter();
+    __shared__ double sL[OZ_TI_BLK][OZ_TI_BLK + 1];   // [column][row]
+    __shared__ double sw[OZ_TI_BLK][OZ_TI_BLK + 1];   // row i of the inverse
+    __shared__ double ri[OZ_TI_BLK];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r0 = blockIdx.x * OZ_TI_BLK;
+    const int m = min(OZ_TI_BLK, L.n - r0);
+#pragma unroll
+    for (int q = 0; q < 8; q++) {   // identity beyond n
+        const int c = 4 * q + warp;
+        double v = lane == c ? 1.0 : 0.0;
+        if (c <= lane && lane < m && !(unit && lane == c)) v = L(r0 + lane, r0 + c);
+        sL[c][lane] = v;
+        if (lane == c) ri[c] = 1.0 / v;
+    }
+    __syncthreads();
+    double s[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) s[u] = 4 * u + warp == lane ? 1.0 : 0.0;
+    auto publish = [&](int i) {
+        sw[i][lane] = s[i >> 2] * ri[i];
+        bar_arrive(1 + (i & 7), 128);
     };
-    for (int i = threadIdx.x; i < n; i += blockDim.x) sR[i] = unit ? 1.0 : 1.0 / tget(i, i);
-    const int jfirst = blockIdx.x * OZ_TI_WARPS;
-    const int j = jfirst + warp;   // this warp's column of L'^-1
-    double w[OZ_TI_NMAX / 32];
+    if (warp == 0) publish(0);
 #pragma unroll
-    for (int s = 0; s < OZ_TI_NMAX / 32; s++) w[s] = (s * 32 + lane == j) ? 1.0 : 0.0;
-    for (int p0 = jfirst / OZ_TI_PANEL * OZ_TI_PANEL; p0 < n; p0 += OZ_TI_PANEL) {
-        __syncthreads();   // the previous panel is consumed (and sR written)
-        const int rows = n - p0;
-        for (int t = threadIdx.x; t < OZ_TI_PANEL * rows; t += blockDim.x) {
-            const int c = t / rows, r = p0 + t % rows;
-            sT[c][r] = (p0 + c < n && r >= p0 + c) ? tget(r, p0 + c) : 0.0;
+    for (int i = 0; i < OZ_TI_BLK - 1; i++) {
+        if (warp != (i & 3)) bar_wait(1 + (i & 7), 128);
+        const double w = sw[i][lane];
+        if (warp == ((i + 1) & 3)) {
+            s[(i + 1) >> 2] = fma(-sL[i][i + 1], w, s[(i + 1) >> 2]);
+            publish(i + 1);
         }
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            if (4 * u + 3 > i && 4 * u + warp > i + (warp == ((i + 1) & 3) ? 1 : 0))
+                s[u] = fma(-sL[i][4 * u + warp], w, s[u]);
+    }
+    if (warp != ((OZ_TI_BLK - 1) & 3)) bar_wait(1 + ((OZ_TI_BLK - 1) & 7), 128);
+    __syncthreads();
+    double *d = D + (size_t)blockIdx.x * OZ_TI_BLK * OZ_TI_BLK;
+    for (int t = threadIdx.x; t < OZ_TI_BLK * OZ_TI_BLK; t += 128) d[t] = sw[t & 31][t >> 5];
+}
+
+__global__ void __launch_bounds__(OZ_TI_NMAX)
+oz_trinv_kernel(OzTriView L, int trans, const double *__restrict__ D, double *__restrict__ X, long long ldx)
+{
+    gbx_launch::pdl_enter();
+    __shared__ double st[2][OZ_TI_BLK], sx[2][OZ_TI_BLK];
+    const int n = L.n, r = threadIdx.x, warp = r >> 5, lane = r & 31;
+    const int c0 = blockIdx.x, c1 = n - 1 - c0;   // c0 <= c1; equal: one column
+    const int nb = (n + OZ_TI_BLK - 1) / OZ_TI_BLK, first = c0 / OZ_TI_BLK;
+    // block step: thread (column, row, quarter of the products)
+    const int pc = r >> 7, pi = (r >> 2) & 31, pq = r & 3;
+    double t0 = r == c0 ? 1.0 : 0.0, t1 = r == c1 ? 1.0 : 0.0;
+    double x0 = 0.0, x1 = 0.0;   // this row's results
+    double l[OZ_TI_BLK], d[8];
+    auto load = [&](int I) {
+        if (I >= nb) return;
+#pragma unroll
+        for (int k = 0; k < OZ_TI_BLK; k++)
+            l[k] = (warp > I && r < n) ? L(r, I * OZ_TI_BLK + k) : 0.0;
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            d[k] = D[(size_t)I * OZ_TI_BLK * OZ_TI_BLK + (8 * pq + k) * OZ_TI_BLK + pi];
+    };
+    load(first);
+    for (int I = first; I < nb; I++) {
+        const bool two = c1 < (I + 1) * OZ_TI_BLK;   // the second column has begun (uniform)
+        if (warp == I) { st[0][lane] = t0; st[1][lane] = t1; }
         __syncthreads();
-        if (j >= n) continue;
-        for (int c = 0; c < OZ_TI_PANEL; c++) {
-            const int i = p0 + c;
-            if (i >= n) break;
-            if (i < j) continue;   // uniform over the warp
-            const int slot = i >> 5;
-            double wo = 0.0;
+        double x = 0.0;
+        if (pc == 0 || two) {
 #pragma unroll
-            for (int s = 0; s < OZ_TI_NMAX / 32; s++)
-                if (s == slot) wo = w[s];
-            const double wi = __shfl_sync(0xffffffffu, wo * sR[i], i & 31);
+            for (int k = 0; k < 8; k++) x = fma(d[k], st[pc][8 * pq + k], x);
+            x += __shfl_xor_sync(0xffffffffu, x, 1);
+            x += __shfl_xor_sync(0xffffffffu, x, 2);
+        }
+        if (pq == 0) sx[pc][pi] = x;
+        __syncthreads();
+        if (warp == I) { x0 = sx[0][lane]; x1 = sx[1][lane]; }
+        if (warp > I) {
+            if (two) {
 #pragma unroll
-            for (int s = 0; s < OZ_TI_NMAX / 32; s++) {
-                if (s < slot || s * 32 >= n) continue;   // warp-uniform: no FP64 issue
-                const int r = s * 32 + lane;
-                if (r > i && r < n) w[s] = fma(-sT[c][r], wi, w[s]);
-                else if (r == i) w[s] = wi;
+                for (int k = 0; k < OZ_TI_BLK; k++) {
+                    t0 = fma(-l[k], sx[0][k], t0);
+                    t1 = fma(-l[k], sx[1][k], t1);
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < OZ_TI_BLK; k++) t0 = fma(-l[k], sx[0][k], t0);
             }
         }
+        load(I + 1);
     }
-    if (j >= n) return;
-#pragma unroll
-    for (int s = 0; s < OZ_TI_NMAX / 32; s++) {
-        const int r = s * 32 + lane;
-        if (r >= n) continue;
-        const double v = r >= j ? w[s] : 0.0;
-        const int R = lower ? r : n - 1 - r, J = lower ? j : n - 1 - j;   // entry (R, J) of T^-1
-        if (trans) X[(long long)R * ldx + J] = v;
-        else X[(long long)J * ldx + R] = v;
-    }
+    if (r >= n) return;
+    // entry (R, J) of T^-1
+    const int R = L.lower ? r : n - 1 - r, J0 = L.lower ? c0 : n - 1 - c0, J1 = L.lower ? c1 : n - 1 - c1;
+    if (r < c0) x0 = 0.0;
+    if (r < c1) x1 = 0.0;
+    X[trans ? (long long)R * ldx + J0 : (long long)J0 * ldx + R] = x0;
+    X[trans ? (long long)R * ldx + J1 : (long long)J1 * ldx + R] = x1;
 }
 
 __global__ void oz_set_identity(int n, double *X, long long ldx)
@@ -2752,14 +2817,19 @@ extern "C" gbx_status gbx_dtrsm_ozaki(gbx_ctx *ctx, char side, char uplo, char t
     if (alpha == 0.0 || na > 1024) return gbx_dtrsm(ctx, side, uplo, ta, diag, m, n, alpha, A, lda, B, ldb);
     gbx_status st;
     void *px;
-    if ((st = gbx_ws(ctx, GBX_WS_TRSM_X, sizeof(double) * (size_t)na * na, &px)) != GBX_OK) return st;
+    // the inverse, then (n <= 256) its inverted diagonal blocks
+    const int nblk = (na + OZ_TI_BLK - 1) / OZ_TI_BLK;
+    const size_t dsz = na <= OZ_TI_NMAX ? (size_t)nblk * OZ_TI_BLK * OZ_TI_BLK : 0;
+    if ((st = gbx_ws(ctx, GBX_WS_TRSM_X, sizeof(double) * ((size_t)na * na + dsz), &px)) != GBX_OK) return st;
     double *X = (double *)px;
     cudaStream_t s = S_(ctx);
     if (na <= OZ_TI_NMAX) {
-        // X = op(A)^-1 by the warp-per-column substitution kernel
-        oz_trinv_kernel<<<(na + OZ_TI_WARPS - 1) / OZ_TI_WARPS, OZ_TI_WARPS * 32, 0, s>>>(
-            na, A, lda, gbx_lsame(uplo, 'L') ? 1 : 0, gbx_lsame(diag, 'U') ? 1 : 0, gbx_lsame(ta, 'N') ? 0 : 1, X, na);
-        gbx_count_launch(ctx, 1);
+        // X = op(A)^-1 by blocked substitution
+        const OzTriView L{A, lda, na, gbx_lsame(uplo, 'L') ? 1 : 0};
+        double *D = X + (size_t)na * na;
+        gbx_launch::launch_pdl(oz_trinv_diag, nblk, 128, 0, s, L, gbx_lsame(diag, 'U') ? 1 : 0, D);
+        gbx_launch::launch_pdl(oz_trinv_kernel, (na + 1) / 2, OZ_TI_NMAX, 0, s, L, gbx_lsame(ta, 'N') ? 0 : 1, D, X, na);
+        gbx_count_launch(ctx, 2);
         if ((st = gbx_check_launch(ctx, "dtrsm_ozaki inverse")) != GBX_OK) return st;
     } else {
         // X = op(A)^-1 I by the FP64 DTRSM

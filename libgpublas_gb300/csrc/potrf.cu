@@ -6,137 +6,155 @@
 // Blocked in 32-column steps.  On GB300 one SM does about 4 GFLOP/s of FP64,
 // so a factorisation of a 256 x 256 block confined to one CTA costs over a
 // millisecond; here only the 32 x 32 diagonal factorisations are serial:
-//   * potrf_step(j0): every CTA factors the 32 x 32 diagonal block at j0 in
-//     shared memory (redundantly: 5.5k FMAs), the last CTA to finish writes
-//     it back, and each CTA solves 8 rows of the panel below against it
-//     (x L^T = a, one warp per row);
+//   * potrf_step(j0): every CTA (one warp per SM sub-partition) factors the
+//     32 x 32 diagonal block at j0 (redundantly) together with 8 rows of the
+//     panel below it, which take the same column operations; the last CTA to
+//     finish writes the diagonal block back;
 //   * potrf_syrk(j0): the trailing update A22 -= A21 A21^T, one 16 x 16
 //     lower tile per CTA (8k FMAs each).  The GEMM core would put this
 //     product on one or two 128 x 128 tiles, i.e. one or two SMs: 63 µs for
-//     a 64 x 64 x 64 update, most of the old 64-column version's 250 µs per
-//     128 x 128 block.
+//     a 64 x 64 x 64 update.
 // A non-positive pivot sets *info to its 1-based column (LAPACK convention,
 // first failure wins); the rest of the block is then unspecified.
 #include "gbx_internal.h"
+#include "launch.cuh"
 
 #include <cuda_runtime.h>
 
 namespace {
 
-constexpr int PB = 32;          // panel width
-constexpr int PT_THREADS = 256;
-constexpr int PR = 8;           // panel rows per CTA (one warp per row)
-static_assert(PB == 32 && PR * 32 == PT_THREADS, "the panel solve maps lane j to column j, one warp per row");
+using namespace gbx_launch;
 
-// One step j0: the diagonal block factor and the panel rows of this CTA.
-// FP64 arithmetic retires two lanes per clock per SM on this part, so the
-// step is spread thin: the 32 x 32 factor (about 5.5k FMAs) is repeated by
-// every CTA and the panel below is split 8 rows per CTA; divisions and
-// square roots, long dependent FP64 sequences, are replaced by one rsqrt per
-// column (L_kk = d * rsqrt(d), the column and the panel scaled by rsqrt(d)).
-// An FP64 warp instruction holds the SM's 2-lane FP64 pipe for 16 cycles
-// whatever its predicate, so the trailing update of each column walks only
-// the live triangle (a table of (row, column) pairs).
+constexpr int PB = 32;          // panel width: one lane per row of the diagonal block
+constexpr int PR = 8;           // panel rows per CTA
+constexpr int PT_THREADS = 128;
+
+// 1 / d to within an ulp or two for a positive d: an approximate reciprocal y
+// and one step of Halley's third-order iteration, y (1 + e + e^2) with
+// e = 1 - d y (e < 2^-18 leaves e^3 < 2^-54), three dependent FP64 operations
+// where a division takes a dozen (64 cycles each on this part).  NaN for a d
+// whose reciprocal is near the ends of the range: its column is divided by d.
+__device__ __forceinline__ double potrf_recip(double d)
+{
+    const unsigned ex = ((unsigned)(__double_as_longlong(d) >> 52)) & 0x7ffu;
+    if (ex - 23u > 2000u) return __longlong_as_double(0x7ff8000000000000ll);
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    const double e = fma(-d, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
+
+// The division of the rare columns, out of line (the steps are unrolled).
+__device__ __noinline__ double potrf_ratio(double a, double d) { return a / d; }
+
+// One step j0.  Warp w holds columns 4q + w of the diagonal block (lane = row,
+// a[q]) and of this CTA's 8 panel rows (lane = row + 8 (q mod 4), p[q / 4]).
+// The factorisation is A = L' D L'^T with L' = L diag(L)^-1: at step k every warp
+// scales the published column k by -1/d_k and subtracts its multiples from its
+// own later columns; the warp of column k + 1 updates that one first, publishes
+// it with its reciprocal and arrives on a named barrier that only the others
+// wait on, so the chain from pivot to pivot is one multiplication, two FMAs (the
+// panel's column too) and a reciprocal.  The square roots come at the end, one
+// per column in parallel.  The FP64 rate of an SM is half a lane per clock in
+// each of its four sub-partitions: an FP64 warp instruction takes 64 cycles on
+// its own, so one warp alone runs at a quarter of the rate (a one-warp version
+// took 64 us); the chain's seven operations and hand-over set 500 to 900 cycles
+// per column.
+// Measured: 18 us per step; with a barrier of 256 threads and a reciprocal
+// square root per column it was 30 us.
 __global__ void __launch_bounds__(PT_THREADS)
 potrf_step(int n, int j0, double *__restrict__ A, long long lda, int *__restrict__ info, unsigned *done)
 {
-    extern __shared__ double sm[];
-    double(*L)[PB + 1] = (double(*)[PB + 1])sm;                   // diagonal block
-    double(*X)[PB + 1] = (double(*)[PB + 1])(sm + PB * (PB + 1));  // this CTA's panel rows
-    __shared__ double rinv[PB];
-    __shared__ unsigned short tri[PB * (PB - 1) / 2];   // (r << 8 | c), c <= r < PB - 1, by r(r+1)/2 + c
-    __shared__ int s_bad, s_last;
-    const int tid = threadIdx.x;
+    pdl_enter();
+    __shared__ double colA[PB][PB];   // column k, unscaled, once final
+    __shared__ double colP[PB][PR];
+    __shared__ double rec[PB];        // reciprocal (then reciprocal square root) of pivot k
+    __shared__ int s_last;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int b = min(PB, n - j0);
-    for (int t = tid; t < PB * (PB - 1) / 2; t += PT_THREADS) {
-        int r = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
-        while ((r + 1) * (r + 2) / 2 <= t) r++;
-        while (r * (r + 1) / 2 > t) r--;
-        tri[t] = (unsigned short)((r << 8) | (t - r * (r + 1) / 2));
+    const int r0 = j0 + b + blockIdx.x * PR;   // first panel row (b = PB whenever there is a panel)
+    const int pr = lane & (PR - 1), pg = lane >> 3;
+    double *D = A + (long long)j0 * lda + j0;
+    double a[8], p[2];
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        const int j = 4 * q + warp;
+        a[q] = (lane < b && j <= lane) ? D[(long long)j * lda + lane] : (j == lane ? 1.0 : 0.0);
     }
-    for (int t = tid; t < PB * PB; t += PT_THREADS) {
-        const int i = t % PB, k = t / PB;
-        L[i][k] = (i < b && k < b && i >= k) ? A[(long long)(j0 + k) * lda + j0 + i] : (i == k ? 1.0 : 0.0);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int j = 4 * (pg + 4 * h) + warp;
+        p[h] = (r0 + pr < n && j < b) ? A[(long long)(j0 + j) * lda + r0 + pr] : 0.0;
     }
-    // the panel rows are loaded now too (they do not depend on the factor)
-    const int r0 = j0 + b + blockIdx.x * PR;
-    for (int t = tid; t < PR * PB; t += PT_THREADS) {
-        const int rr = t % PR, k = t / PR;
-        X[rr][k] = (r0 + rr < n && k < b) ? A[(long long)(j0 + k) * lda + r0 + rr] : 0.0;
-    }
-    if (tid == 0) s_bad = 0;
-    __syncthreads();
-    // Right-looking factorisation of the diagonal block in shared memory,
-    // one barrier per column.  The pivot of column k + 1 is formed by the
-    // thread that finishes its last update (the first pair of column k's
-    // update is (k+1, k+1)), the update of column k uses the unscaled column
-    // times y^2, and column k is scaled during the next column's update
-    // (which reads only column k + 1).
-    auto pivot = [&](int k, double d) {
-        if (!(d > 0.0)) {
-            s_bad = k + 1;
-        } else {
-            const double y = rsqrt(d);
-            L[k][k] = d * y;
-            rinv[k] = y;
-        }
+    // publishes column k (this warp's): values, reciprocal of the pivot, panel
+    auto publish = [&](int k, double ak, double pk) {
+        colA[k][lane] = ak;
+        if (pg == ((k >> 2) & 3)) colP[k][pr] = pk;
+        const double r = potrf_recip(__shfl_sync(0xffffffffu, ak, k));
+        if (lane == 0) rec[k] = r;
+        bar_arrive(1 + (k & 7), PT_THREADS);
     };
-    if (tid == 0) pivot(0, L[0][0]);
-    __syncthreads();
-    for (int k = 0; k < b; k++) {
-        if (s_bad) break;   // uniform: read after a barrier
-        if (k > 0) {
-            const double yp = rinv[k - 1];
-            for (int i = k + tid; i < b; i += PT_THREADS) L[i][k - 1] *= yp;
+    if (warp == 0) publish(0, a[0], p[0]);
+#pragma unroll
+    for (int k = 0; k < PB - 1; k++) {
+        if (warp != (k & 3)) bar_wait(1 + (k & 7), PT_THREADS);
+        const double r = rec[k];
+        double m = -(colA[k][lane] * r);
+        if ((__double_as_longlong(r) & 0x7ff0000000000000ll) == 0x7ff0000000000000ll)   // uniform
+            m = -potrf_ratio(colA[k][lane], colA[k][k]);
+        const double pk = colP[k][pr];
+        constexpr unsigned ALL = 0xffffffffu;
+        if (warp == ((k + 1) & 3)) {
+            a[(k + 1) >> 2] = fma(m, colA[k][k + 1], a[(k + 1) >> 2]);
+            const double mk = __shfl_sync(ALL, m, k + 1);
+            publish(k + 1, a[(k + 1) >> 2], fma(pk, mk, p[(k + 1) >> 4]));
         }
-        const double y = rinv[k], y2 = y * y;
-        const int m = b - k - 1;
-        for (int t = tid; t < m * (m + 1) / 2; t += PT_THREADS) {
-            const int rc = tri[t];
-            const int i = k + 1 + (rc >> 8), j = k + 1 + (rc & 255);
-            const double v = fma(-L[i][k] * y2, L[j][k], L[i][j]);
-            L[i][j] = v;
-            if (t == 0) pivot(k + 1, v);
+#pragma unroll
+        for (int q = 0; q < 8; q++)
+            if (4 * q + 3 > k && 4 * q + warp > k + (warp == ((k + 1) & 3) ? 1 : 0)) {
+                a[q] = fma(m, colA[k][4 * q + warp], a[q]);
+            }
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            if (16 * h + 15 <= k) continue;
+            // a lane's columns up to k + 1 are published already: its value no longer matters
+            const double mj = __shfl_sync(ALL, m, (4 * (pg + 4 * h) + warp) & 31);
+            p[h] = fma(pk, mj, p[h]);
         }
-        __syncthreads();
     }
+    if (warp != ((PB - 1) & 3)) bar_wait(1 + ((PB - 1) & 7), PT_THREADS);
     __syncthreads();
-    if (!s_bad) {   // uniform over the CTA
-        // panel: x L11^T = a for this CTA's rows, right-looking; one warp per
-        // row, lane j owning column j (PB = 32)
-        const int rr = tid >> 5, c = tid & 31;
-        for (int k = 0; k < b; k++) {
-            const double xk = X[rr][k] * rinv[k];
-            if (c > k && c < b) X[rr][c] = fma(-xk, L[c][k], X[rr][c]);
-            __syncwarp();
-            if (c == k) X[rr][k] = xk;
-            __syncwarp();
-        }
-        __syncthreads();
+    // 1-based column of the first non-positive pivot (zero, negative or NaN, by
+    // the bit pattern), or 0; every warp gets the same answer
+    const double d = colA[lane][lane];
+    const unsigned neg =
+        __ballot_sync(0xffffffffu, (unsigned long long)__double_as_longlong(d) - 1ull >= 0x7ff0000000000000ull);
+    const int bad = __ffs((int)neg);
+    const double y = rsqrt(d);   // L_ik = a_ik / sqrt(d_k)
+    if (warp == 0) rec[lane] = y;
+    __syncthreads();
+    if (!bad) {
         for (int t = tid; t < PR * PB; t += PT_THREADS) {
             const int q = t % PR, k = t / PR;
-            if (r0 + q < n && k < b) A[(long long)(j0 + k) * lda + r0 + q] = X[q][k];
+            if (r0 + q < n && k < b) A[(long long)(j0 + k) * lda + r0 + q] = colP[k][q] * rec[k];
         }
     }
-    // The factored diagonal block goes back to A only when every CTA has
-    // read the original (the last CTA to finish writes it; all CTAs hold the
-    // same factor), so no CTA can read a half-written block.
+    // The factored diagonal block goes back to A only when every CTA has read
+    // the original (the last CTA to finish writes it; all CTAs hold the same
+    // factor), so no CTA can read a half-written block.
     __syncthreads();
     if (tid == 0) {
         __threadfence();
         s_last = atomicAdd(done, 1u) == gridDim.x - 1;
+        if (s_last) {
+            *done = 0u;
+            if (bad) atomicCAS(info, 0, j0 + bad);
+        }
     }
     __syncthreads();
-    if (!s_last) return;
-    if (tid == 0) *done = 0u;
-    if (s_bad) {
-        if (tid == 0) atomicCAS(info, 0, j0 + s_bad);
-        return;
-    }
-    for (int t = tid; t < b * b; t += PT_THREADS) {
-        const int i = t % b, k = t / b;
-        if (i >= k) A[(long long)(j0 + k) * lda + j0 + i] = L[i][k];
-    }
+    if (!s_last || bad) return;
+    for (int k = warp; k < b; k += 4)
+        if (lane < b && k <= lane) D[(long long)k * lda + lane] = colA[k][lane] * rec[k];
 }
 
 // A22 (m x m, lower) -= A21 A21^T with A21 m x PB: one 16 x 16 tile of the
@@ -145,6 +163,7 @@ potrf_step(int n, int j0, double *__restrict__ A, long long lda, int *__restrict
 __global__ void __launch_bounds__(256)
 potrf_syrk(int m, const double *__restrict__ A21, double *__restrict__ A22, long long lda)
 {
+    pdl_enter();
     __shared__ double Li[16][PB + 1], Lj[16][PB + 1];
     const int b = blockIdx.x;
     int ti = (int)((sqrtf(8.0f * (float)b + 1.0f) - 1.0f) * 0.5f);
@@ -181,20 +200,18 @@ extern "C" gbx_status gbx_dpotrf_small(gbx_ctx *ctx, char uplo, int n, double *A
     if (st != GBX_OK) return st;
     unsigned *done = (unsigned *)(words + 12);
     cudaMemsetAsync(info, 0, sizeof(int), s);
-    constexpr size_t SMEM = 2 * sizeof(double) * PB * (PB + 1);
-    cudaFuncSetAttribute(potrf_step, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
     for (int j0 = 0; j0 < n; j0 += PB) {
         const int b = n - j0 < PB ? n - j0 : PB;
         const int rows = n - j0 - b;
         const int grid = rows > 0 ? (rows + PR - 1) / PR : 1;
-        potrf_step<<<grid, PT_THREADS, SMEM, s>>>(n, j0, A, lda, info, done);
+        launch_pdl(potrf_step, grid, PT_THREADS, 0, s, n, j0, A, lda, info, done);
         gbx_count_launch(ctx, 1);
         if ((st = gbx_check_launch(ctx, "dpotrf_small")) != GBX_OK) return st;
         if (rows > 0) {
             const double *A21 = A + (long long)j0 * lda + j0 + b;
             double *A22 = A + (long long)(j0 + b) * lda + j0 + b;
             const int nt = (rows + 15) / 16;
-            potrf_syrk<<<nt * (nt + 1) / 2, 256, 0, s>>>(rows, A21, A22, lda);
+            launch_pdl(potrf_syrk, nt * (nt + 1) / 2, 256, 0, s, rows, A21, A22, lda);
             gbx_count_launch(ctx, 1);
             if ((st = gbx_check_launch(ctx, "dpotrf_small update")) != GBX_OK) return st;
         }
