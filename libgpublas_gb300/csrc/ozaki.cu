@@ -191,7 +191,7 @@ struct OzPrepOp {
     int *scale2;             // optional second copy over Rp2 rows (symmetric rank-k)
     int Rp2;
     uint8_t *X8;             // S digit planes [s][Rp][Kp]
-    float *gpart;            // one-launch path: (emax, num, den) per 16-row block
+    float *gpart;            // one-launch path: (emax, num, den) per row block
 };
 
 __device__ __forceinline__ void oz_stats_rowk_block(const SrcView &v, int rows, int K, int blk, int *expo,
@@ -374,140 +374,128 @@ oz_prep_finish(OzPrepOp a, OzPrepOp b, int b_stats, double tol, int forced, unsi
     }
 }
 
-// E4M3 byte of an integer digit |d| <= 16 (exact).
-__device__ __forceinline__ uint32_t e4m3_of_digit(int d)
+// Digit planes of PER consecutive k of one row with exponent e (|x| < 2^e), x
+// given as binary64 bit patterns: bytes dst .. dst + PER - 1 of plane 0, the
+// planes `plane` bytes apart.  Integer and FP32 pipes only.
+//   N = round(|x| * 2^(4 - e + 5(S-1))) as a 128-bit integer (N <= 16 *
+// 32^(S-1) <= 2^69).  Balanced base-32 digits d_s in [-16, 16] with N = sum_s
+// d_s 32^(S-1-s): adding C = 16 * sum_{s<S} 32^s once turns every 5-bit chunk c of
+// N + C into the digit c - 16 (the carries are resolved by the one addition); the
+// top chunk is taken unmasked (N <= 16 * 32^(S-1) bounds it by 32).
+//   A chunk becomes its E4M3 byte through FP32: 2^23 + c is the chunk under a
+// constant exponent field, one FMA subtracts 2^23 + 16 and applies the sign (both
+// exact), and one conversion makes two bytes.  Four and a half instructions a
+// digit; looking the byte up in a table in shared memory took eleven more, and
+// the preparation is bound by instruction issue.
+// SEL: with selects instead of branches, so that a thread's elements are not
+// separated by control flow and their integer chains overlap (more
+// instructions: for launches that do not fill the SMs).
+template <int PER, bool SEL>
+__device__ __forceinline__ void oz_digits(const unsigned long long (&x)[PER], int e, int S, uint8_t *dst, size_t plane)
 {
-    const int a = d < 0 ? -d : d;
-    if (a == 0) return 0u;
-    const int E = 31 - __clz(a);
-    const int mant = ((a << 3) >> E) - 8;
-    return ((d < 0) ? 0x80u : 0u) | (uint32_t)((E + 7) << 3) | (uint32_t)mant;
-}
-
-// Slices one 16-row x 128-k tile of an operand: S digit planes X8[s][r][k]
-// (K-major, rows padded to Rp, k to Kp), OZ_SPLIT_PER consecutive k per
-// thread; padding gets digit 0.  The tile is staged through shared memory so
-// col_k sources are read coalesced.
-constexpr int OZ_SPLIT_ROWS = 16, OZ_SPLIT_PER = 8;
-// the one-launch preparation: 256 threads per 16-row block (16 per row for
-// the statistics, 8 k per thread for the digits), or 512 (4 k per thread for
-// the digits) when the blocks fit on the SMs at once: the digit split is then
-// the block's longest step, and more warps per block shorten it (with more
-// blocks than SMs, 512-thread blocks measured slower)
-constexpr int OZ_SMALL_THREADS = 256;
-
-// PER consecutive k per thread (blockDim = 16 * 128 / PER); pre: the same
-// tile already staged by the caller (one-launch path, K <= 128); expo_s: the
-// 16 rows' exponents in the caller's shared memory (one-launch path), else
-// they are read from expo
-template <int PER, bool SEL = false>
-__device__ __forceinline__ void oz_split_tile(const SrcView &v, int rows, int K, int Rp, int Kp, const int *expo,
-                                              int S, uint8_t *X8, int blk, const double (*pre)[129] = nullptr,
-                                              const int *expo_s = nullptr)
-{
-    static_assert(PER == 4 || PER == 8, "split width");
-    __shared__ double tile[OZ_SPLIT_ROWS][129];
-    // E4M3 byte of the digit c - 16 at [c] and of 16 - c at [40 + c], c in
-    // [0, 32]: a negative element reads the second table (no per-digit sign)
-    __shared__ uint32_t e4m3_tbl[80];
-    const int kblocks = Kp / 128;
-    const int r0 = (blk / kblocks) * OZ_SPLIT_ROWS, k0 = (blk % kblocks) * 128;
-    __syncthreads();   // a previous call's readers of tile are done
-    if (threadIdx.x < 33) {
-        e4m3_tbl[threadIdx.x] = e4m3_of_digit((int)threadIdx.x - 16);
-        e4m3_tbl[40 + threadIdx.x] = e4m3_of_digit(16 - (int)threadIdx.x);
-    }
-    // load: col_k -> threads along rows; row_k -> threads along k
-    if (!pre)
-        for (int t = threadIdx.x; t < OZ_SPLIT_ROWS * 128; t += blockDim.x) {
-            int rr, kk;
-            if (v.row_k) { kk = t & 127; rr = t >> 7; }
-            else         { rr = t % OZ_SPLIT_ROWS; kk = t / OZ_SPLIT_ROWS; }
-            const int r = r0 + rr, k = k0 + kk;
-            tile[rr][kk] = (r < rows && k < K) ? src_get(v, r, k) : 0.0;
-        }
-    const double (*T)[129] = pre ? pre : tile;
-    __syncthreads();
-    constexpr int TPR = 128 / PER;   // threads per row
-    const int rr = threadIdx.x / TPR, kq = (threadIdx.x % TPR) * PER;
-    const int r = r0 + rr;
-    if (r >= Rp) return;
-    const int e = r < rows ? (expo_s ? expo_s[rr] : expo[r]) : 0;
-    // N_j = round(|x_j| * 2^(4 - e + 5(S-1))) as a 128-bit integer hi:lo.
-    // |x| < 2^e bounds N_j by 16 * 32^(S-1) <= 2^69.  Integer pipe only.
+    static_assert(PER == 4 || PER == 8, "one 32- or 64-bit store per plane");
     const int top = 4 - e + 5 * (S - 1);
-    unsigned long long lo[PER], hi[PER];
-    unsigned neg = 0u;
-    // (SEL: with selects instead of branches, so that the elements of a
-    // thread are not separated by control flow and their integer chains
-    // overlap; more instructions, so only where few blocks run)
-#pragma unroll
-    for (int j = 0; j < PER; j++) {
-        const unsigned long long b = (unsigned long long)__double_as_longlong(T[rr][kq + j]);
-        neg |= (unsigned)(b >> 63) << j;
-        const int E = (int)((b >> 52) & 0x7FF);
-        const unsigned long long M = (b & 0xFFFFFFFFFFFFFull) | (E ? (1ull << 52) : 0ull);
-        const int sh = (E ? E : 1) - 1075 + top;
-        if constexpr (!SEL) {
-            if (M == 0ull || sh <= -54) { lo[j] = 0ull; hi[j] = 0ull; }
-            else if (sh < 0) { lo[j] = (M + (1ull << (-sh - 1))) >> (-sh); hi[j] = 0ull; }
-            else if (sh == 0) { lo[j] = M; hi[j] = 0ull; }
-            else if (sh < 64) { lo[j] = M << sh; hi[j] = M >> (64 - sh); }
-            else { lo[j] = 0ull; hi[j] = M << (sh - 64); }
-            continue;
-        }
-        // sh < 0: M * 2^sh rounded half up (0 for sh <= -54; M = 0 gives 0);
-        // sh >= 0: M << sh in 128 bits (sh <= 69)
-        const int rs = max(1, min(-sh, 63));
-        const unsigned long long mr = sh < 0 ? (sh <= -54 ? 0ull : (M + (1ull << (rs - 1))) >> rs) : M;
-        const int ls = max(sh, 0);
-        lo[j] = ls < 64 ? mr << (ls & 63) : 0ull;
-        hi[j] = ls == 0 ? 0ull : (ls < 64 ? mr >> ((64 - ls) & 63) : mr << ((ls - 64) & 63));
-    }
-    // Balanced base-32 digits d_s in [-16, 16] with N = sum_s d_s 32^(S-1-s):
-    // adding C = 16 * sum_{s<S} 32^s once turns every 5-bit chunk c of N + C
-    // into the digit c - 16 (the carries are resolved by the one addition);
-    // the top chunk is taken unmasked (N <= 16 * 32^(S-1) bounds it by 32).
     unsigned long long clo = 0ull, chi = 0ull;
     for (int s = 0; s < S; s++) {
         const int b = 5 * s + 4;
         if (b < 64) clo |= 1ull << b;
         else chi |= 1ull << (b - 64);
     }
-    // N + C as three 32-bit words (N + C < 2^71)
+    // N + C as three 32-bit words (N + C < 2^71), and the sign with its offset
     uint32_t w0[PER], w1[PER], w2[PER];
+    float sg[PER], of[PER];
 #pragma unroll
     for (int j = 0; j < PER; j++) {
-        const unsigned long long nl = lo[j] + clo;
-        const unsigned long long nh = hi[j] + chi + (nl < clo ? 1ull : 0ull);
+        const unsigned long long b = x[j];
+        const int E = (int)((b >> 52) & 0x7FF);
+        const unsigned long long M = (b & 0xFFFFFFFFFFFFFull) | (E ? (1ull << 52) : 0ull);
+        const int sh = (E ? E : 1) - 1075 + top;
+        unsigned long long lo, hi;
+        if constexpr (!SEL) {
+            if (M == 0ull || sh <= -54) { lo = 0ull; hi = 0ull; }
+            else if (sh < 0) { lo = (M + (1ull << (-sh - 1))) >> (-sh); hi = 0ull; }
+            else if (sh == 0) { lo = M; hi = 0ull; }
+            else if (sh < 64) { lo = M << sh; hi = M >> (64 - sh); }
+            else { lo = 0ull; hi = M << (sh - 64); }
+        } else {
+            // sh < 0: M * 2^sh rounded half up (0 for sh <= -54; M = 0 gives 0);
+            // sh >= 0: M << sh in 128 bits (sh <= 69)
+            const int rs = max(1, min(-sh, 63));
+            const unsigned long long mr = sh < 0 ? (sh <= -54 ? 0ull : (M + (1ull << (rs - 1))) >> rs) : M;
+            const int ls = max(sh, 0);
+            lo = ls < 64 ? mr << (ls & 63) : 0ull;
+            hi = ls == 0 ? 0ull : (ls < 64 ? mr >> ((64 - ls) & 63) : mr << ((ls - 64) & 63));
+        }
+        const unsigned long long nl = lo + clo;
+        const unsigned long long nh = hi + chi + (nl < clo ? 1ull : 0ull);
         w0[j] = (uint32_t)nl;
         w1[j] = (uint32_t)(nl >> 32);
         w2[j] = (uint32_t)nh;
+        const uint32_t neg = (uint32_t)(b >> 32) & 0x80000000u;
+        sg[j] = __uint_as_float(0x3F800000u | neg);
+        of[j] = __uint_as_float(__float_as_uint(-8388624.0f) ^ neg);   // -(2^23 + 16), signed
     }
-    const uint32_t *tb[PER];   // each element's table (by its sign)
-#pragma unroll
-    for (int j = 0; j < PER; j++) tb[j] = e4m3_tbl + (((neg >> j) & 1u) ? 40 : 0);
     // chunk t (bit 5t, from the low end) is the digit of plane S - 1 - t;
     // unrolled over t so that its word and bit offset are constants (one
     // funnel shift per chunk)
+    uint8_t *d = dst + (size_t)(S - 1) * plane;
 #pragma unroll
     for (int t = 0; t < OZ_SMAX; t++) {
         if (t >= S) break;
         const int sh = 5 * t, wk = sh >> 5, off = sh & 31;
         const uint32_t mask = t == S - 1 ? 63u : 31u;
-        uint32_t w[PER / 4] = {};
+        uint32_t w[PER / 4];
 #pragma unroll
-        for (int j = 0; j < PER; j++) {
-            uint32_t c = wk == 0 ? __funnelshift_r(w0[j], w1[j], off)
-                                 : (wk == 1 ? __funnelshift_r(w1[j], w2[j], off) : w2[j] >> off);
-            c &= mask;
-            // the digit of x = sign(x) * (c - 16) as an E4M3 byte
-            w[j >> 2] |= tb[j][c] << (8 * (j & 3));
+        for (int q = 0; q < PER / 4; q++) {
+            float v[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int j = 4 * q + i;
+                const uint32_t c = wk == 0 ? __funnelshift_r(w0[j], w1[j], off)
+                                           : (wk == 1 ? __funnelshift_r(w1[j], w2[j], off) : w2[j] >> off);
+                v[i] = fmaf(__uint_as_float((c & mask) | 0x4B000000u), sg[j], of[j]);
+            }
+            asm("{\n\t.reg .b16 lo, hi;\n\t"
+                "cvt.rn.satfinite.e4m3x2.f32 lo, %2, %1;\n\t"
+                "cvt.rn.satfinite.e4m3x2.f32 hi, %4, %3;\n\t"
+                "mov.b32 %0, {lo, hi};\n\t}"
+                : "=r"(w[q]) : "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]));
         }
-        uint8_t *dst = X8 + ((size_t)(S - 1 - t) * Rp + r) * Kp + k0 + kq;
-        if constexpr (PER == 8) *(uint2 *)dst = make_uint2(w[0], w[PER / 4 - 1]);
-        else *(uint32_t *)dst = w[0];
+        if constexpr (PER == 8) *(uint2 *)d = make_uint2(w[0], w[PER / 4 - 1]);
+        else *(uint32_t *)d = w[0];
+        d -= plane;
     }
+}
+
+// Slices one 16-row x 128-k tile of an operand: S digit planes X8[s][r][k]
+// (K-major, rows padded to Rp, k to Kp), eight consecutive k per thread; padding
+// gets digit 0.  The tile is staged through shared memory so col_k sources are
+// read coalesced.
+constexpr int OZ_SPLIT_ROWS = 16, OZ_SPLIT_PER = 8;
+
+__device__ __forceinline__ void oz_split_tile(const SrcView &v, int rows, int K, int Rp, int Kp, const int *expo,
+                                              int S, uint8_t *X8, int blk)
+{
+    __shared__ double tile[OZ_SPLIT_ROWS][129];
+    const int kblocks = Kp / 128;
+    const int r0 = (blk / kblocks) * OZ_SPLIT_ROWS, k0 = (blk % kblocks) * 128;
+    // load: col_k -> threads along rows; row_k -> threads along k
+    for (int t = threadIdx.x; t < OZ_SPLIT_ROWS * 128; t += blockDim.x) {
+        int rr, kk;
+        if (v.row_k) { kk = t & 127; rr = t >> 7; }
+        else         { rr = t % OZ_SPLIT_ROWS; kk = t / OZ_SPLIT_ROWS; }
+        const int r = r0 + rr, k = k0 + kk;
+        tile[rr][kk] = (r < rows && k < K) ? src_get(v, r, k) : 0.0;
+    }
+    __syncthreads();
+    constexpr int TPR = 128 / OZ_SPLIT_PER;   // threads per row
+    const int rr = threadIdx.x / TPR, kq = (threadIdx.x % TPR) * OZ_SPLIT_PER;
+    const int r = r0 + rr;
+    if (r >= Rp) return;
+    unsigned long long x[OZ_SPLIT_PER];
+#pragma unroll
+    for (int j = 0; j < OZ_SPLIT_PER; j++) x[j] = (unsigned long long)__double_as_longlong(tile[rr][kq + j]);
+    oz_digits<OZ_SPLIT_PER, false>(x, r < rows ? expo[r] : 0, S, X8 + (size_t)r * Kp + k0 + kq, (size_t)Rp * Kp);
 }
 
 __global__ void __launch_bounds__(256)
@@ -515,152 +503,137 @@ oz_prep_split(OzPrepOp a, OzPrepOp b, const int *__restrict__ S_dev)
 {
     const int S = *S_dev;
     if ((int)blockIdx.x < a.split_blocks)
-        oz_split_tile<OZ_SPLIT_PER>(a.v, a.rows, a.K, a.Rp, a.Kp, a.expo, S, a.X8, blockIdx.x);
+        oz_split_tile(a.v, a.rows, a.K, a.Rp, a.Kp, a.expo, S, a.X8, blockIdx.x);
     else
-        oz_split_tile<OZ_SPLIT_PER>(b.v, b.rows, b.K, b.Rp, b.Kp, b.expo, S, b.X8, blockIdx.x - a.split_blocks);
+        oz_split_tile(b.v, b.rows, b.K, b.Rp, b.Kp, b.expo, S, b.X8, blockIdx.x - a.split_blocks);
 }
 
 // ---- small K: the whole preparation in one launch ---------------------------
-// Each CTA owns 16 complete rows of one operand: a first pass over their K
-// extent gives the row statistics (maximum and sum of squares), a second
-// writes P digit planes, P the largest slice count the tolerance can call
-// for (the slice count itself is not known yet; the leading S planes of the
-// P-digit balanced expansion represent the row to within 16.5 * 2^(-5S) of
-// its maximum, the same bound as rounding at S digits); every CTA leaves a partial of the slice-count statistic,
-// from which the product kernel chooses S.  One launch instead of three:
-// small products are dominated by per-launch cost.
-template <int THREADS>
-__device__ __forceinline__ void oz_prep_rows(const SrcView &v, int rows, int K, int Rp, int Kp, int *expo, double *ss,
-                                             int *scale, uint8_t *X8, float *gpart, int planes, int rblk,
-                                             int *status)
+// Each CTA owns four complete rows of one operand, 64 threads to a row and four
+// consecutive k per thread and pass of 256 k: a first pass over the K extent
+// gives the row statistics (maximum and sum of squares), a second writes P digit
+// planes, P the largest slice count the tolerance can call for (the slice count
+// itself is not known yet; the leading S planes of the P-digit balanced
+// expansion represent the row to within 16.5 * 2^(-5S) of its maximum, the same
+// bound as rounding at S digits); every CTA leaves a partial of the slice-count
+// statistic, from which the product kernel chooses S.  Four rows are one 32-byte
+// sector per k of a column-major operand, so its loads waste nothing, and up to
+// K = 256 (ONE) the elements stay in registers between the passes.  One launch
+// instead of three: small products are dominated by per-launch cost, and what is
+// left is the latency of a CTA.  With 16 rows per CTA, staged in shared memory
+// and read twice, a small operand pair (512 rows of 256) took 13.8 us on 32 CTAs,
+// now 5.2 us on 128; 4096 + 256 rows 12.5 us after 28 us.
+constexpr int OZ_PREP_ROWS = 4, OZ_PREP_THREADS = 256, OZ_PREP_PASS = 4 * OZ_PREP_THREADS / OZ_PREP_ROWS;
+
+template <bool ONE, bool SEL>
+__device__ __forceinline__ void oz_prep_rows(const OzPrepOp &o, int planes, int blk, int *status)
 {
-    static_assert(THREADS == 256 || THREADS == 512, "the statistics map 16 threads to a row of a 16-row block");
-    constexpr int PER = OZ_SPLIT_ROWS * 128 / THREADS;   // k per thread in the digit split
-    __shared__ double tile[OZ_SPLIT_ROWS][129];
-    __shared__ int s_ex[OZ_SPLIT_ROWS];       // the rows' exponents and sums of squares, also kept here
-    __shared__ double s_ss[OZ_SPLIT_ROWS];    // for the partial and the split (no global round trip)
-    const int r0 = rblk * OZ_SPLIT_ROWS;
-    const int rr = threadIdx.x >> 4, lane16 = threadIdx.x & 15;   // 16 threads per row
+    __shared__ SsAcc s_acc[OZ_PREP_THREADS / 32][OZ_PREP_ROWS];
+    __shared__ int s_ex[OZ_PREP_ROWS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int rr = threadIdx.x & (OZ_PREP_ROWS - 1), kq = (threadIdx.x / OZ_PREP_ROWS) * 4;
+    const int r = blk * OZ_PREP_ROWS + rr;
+    auto load = [&](int k0, unsigned long long (&x)[4]) {
+        if (!o.v.cplx && o.v.Ksplit >= o.K) {   // a real operand (uniform)
+            const double *src = o.v.row_k ? o.v.X + (long long)r * o.v.ld + k0 + kq
+                                          : o.v.X + (long long)(k0 + kq) * o.v.ld + r;
+            const long long step = o.v.row_k ? 1 : o.v.ld;
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                x[j] = r < o.rows && k0 + kq + j < o.K ? (unsigned long long)__double_as_longlong(src[j * step]) : 0ull;
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                x[j] = r < o.rows && k0 + kq + j < o.K
+                           ? (unsigned long long)__double_as_longlong(src_get(o.v, r, k0 + kq + j)) : 0ull;
+        }
+    };
     SsAcc acc;
     acc.init();
-    for (int k0 = 0; k0 < K; k0 += 128) {
-        if (!v.cplx && v.Ksplit >= K && r0 + OZ_SPLIT_ROWS <= rows && k0 + 128 <= K) {
-            // a full 16 x 128 block of a real operand (uniform): strided
-            // pointers, every load issued before the first store
-            constexpr int N = OZ_SPLIT_ROWS * 128 / THREADS;
-            double x[N];
-            if (v.row_k) {   // X[r * ld + k]: 128 consecutive k per row
-                constexpr int RS = THREADS / 128;
-                const int tr = threadIdx.x >> 7, kk = threadIdx.x & 127;
-                const double *src = v.X + (long long)(r0 + tr) * v.ld + k0 + kk;
+    unsigned long long x[4];
+    bool nonfinite = false;
+    for (int k0 = 0; k0 < o.Kp; k0 += OZ_PREP_PASS) {
+        load(k0, x);
 #pragma unroll
-                for (int i = 0; i < N; i++) x[i] = src[(long long)i * RS * v.ld];
-#pragma unroll
-                for (int i = 0; i < N; i++) tile[tr + i * RS][kk] = x[i];
-            } else {         // X[k * ld + r]: 16 consecutive rows per k
-                constexpr int KS = THREADS / OZ_SPLIT_ROWS;
-                const int tr = threadIdx.x & (OZ_SPLIT_ROWS - 1), kk = threadIdx.x / OZ_SPLIT_ROWS;
-                const double *src = v.X + (long long)(k0 + kk) * v.ld + r0 + tr;
-#pragma unroll
-                for (int i = 0; i < N; i++) x[i] = src[(long long)i * KS * v.ld];
-#pragma unroll
-                for (int i = 0; i < N; i++) tile[tr][kk + i * KS] = x[i];
-            }
-        } else {
-            for (int t = threadIdx.x; t < OZ_SPLIT_ROWS * 128; t += blockDim.x) {
-                int tr, kk;
-                if (v.row_k) { kk = t & 127; tr = t >> 7; }
-                else         { tr = t % OZ_SPLIT_ROWS; kk = t / OZ_SPLIT_ROWS; }
-                const int r = r0 + tr, k = k0 + kk;
-                tile[tr][kk] = (r < rows && k < K) ? src_get(v, r, k) : 0.0;
-            }
+        for (int j = 0; j < 4; j++) {
+            const unsigned long long b = x[j] & 0x7FFFFFFFFFFFFFFFull;
+            nonfinite |= (b >> 52) == 0x7FFull;
+            if constexpr (SEL) acc.add_sel(b);
+            else acc.add(b);
         }
-        __syncthreads();
-        if (threadIdx.x < 256) {   // warp-uniform: the first eight warps
-            bool nonfinite = false;
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-                const unsigned long long b = abs_bits(tile[rr][lane16 + 16 * j]);
-                nonfinite |= (b >> 52) == 0x7FFull;
-                if constexpr (THREADS == 512) acc.add_sel(b);
-                else acc.add(b);
-            }
-            if (nonfinite) atomicCAS(status, 0, OZ_NONFINITE);
-        }
-        __syncthreads();
+        if (ONE) break;
     }
-    if (threadIdx.x < 256) {
+    if (nonfinite) atomicCAS(status, 0, OZ_NONFINITE);
+    auto reduce = [&](SsAcc &a) {   // over the lanes of a row
 #pragma unroll
-        for (int o = 8; o; o >>= 1) {   // the 16 threads of a row are one half-warp
+        for (int m = 16; m >= OZ_PREP_ROWS; m >>= 1) {
             SsAcc t;
-            t.maxb = __shfl_xor_sync(0xffffffffu, acc.maxb, o);
-            t.mref = __shfl_xor_sync(0xffffffffu, acc.mref, o);
-            t.ss = __shfl_xor_sync(0xffffffffu, acc.ss, o);
-            acc.merge(t);
+            t.maxb = __shfl_xor_sync(0xffffffffu, a.maxb, m);
+            t.mref = __shfl_xor_sync(0xffffffffu, a.mref, m);
+            t.ss = __shfl_xor_sync(0xffffffffu, a.ss, m);
+            a.merge(t);
         }
-    }
-    const int r = r0 + rr;
-    if (threadIdx.x < 256 && lane16 == 0 && r < Rp) {
+    };
+    reduce(acc);
+    if (lane < OZ_PREP_ROWS) s_acc[warp][lane] = acc;
+    __syncthreads();
+    if (warp == 0) {
+        acc = s_acc[lane / OZ_PREP_ROWS][rr];
+        reduce(acc);
         int ex = 0;
         double sv = 0.0;
-        if (r < rows) {
-            acc.finish(ex, sv);
-            expo[r] = ex;
-            ss[r] = sv;
-            scale[r] = ex - 4;
-        } else {
-            scale[r] = 0;
+        const bool valid = r < o.rows;
+        if (valid) acc.finish(ex, sv);
+        if (lane < OZ_PREP_ROWS) {
+            if (valid) {
+                o.expo[r] = ex;
+                o.ss[r] = sv;
+            }
+            if (r < o.Rp) o.scale[r] = valid ? ex - 4 : 0;
+            s_ex[rr] = ex;
         }
-        s_ex[rr] = ex;
-        s_ss[rr] = sv;
+        if (o.gpart) {
+            // this block's partial of the slice-count statistic (oz_choose_S):
+            // (emax_c, sum 2^(2(e_i - emax_c)), sum 2^(2(e_i - emax_c)) ss_i)
+            const int e = valid ? ex : -100000;
+            int em = e;
+#pragma unroll
+            for (int m = 1; m < OZ_PREP_ROWS; m <<= 1) em = max(em, __shfl_xor_sync(0xffffffffu, em, m));
+            const int d = 2 * (e - em);
+            const float w = (!valid || d < -126) ? 0.f : __int_as_float((127 + d) << 23);
+            float nu = w, de = valid ? w * (float)sv : 0.f;
+#pragma unroll
+            for (int m = 1; m < OZ_PREP_ROWS; m <<= 1) {
+                nu += __shfl_xor_sync(0xffffffffu, nu, m);
+                de += __shfl_xor_sync(0xffffffffu, de, m);
+            }
+            if (lane == 0) {
+                o.gpart[3 * blk] = (float)em;
+                o.gpart[3 * blk + 1] = nu;
+                o.gpart[3 * blk + 2] = de;
+            }
+        }
     }
     __syncthreads();   // the row exponents are visible to the whole CTA
-    if (gpart && threadIdx.x < 32) {
-        // this block's partial of the slice-count statistic (oz_choose_S):
-        // (emax_c, sum 2^(2(e_i - emax_c)), sum 2^(2(e_i - emax_c)) ss_i)
-        const int rg = r0 + (threadIdx.x & 15);
-        const bool valid = threadIdx.x < 16 && rg < rows;
-        const int e = valid ? s_ex[threadIdx.x & 15] : -100000;
-        int em = e;
-#pragma unroll
-        for (int o = 16; o; o >>= 1) em = max(em, __shfl_xor_sync(0xffffffffu, em, o));
-        const int d = 2 * (e - em);
-        const float w = (!valid || d < -126) ? 0.f : __int_as_float((127 + d) << 23);
-        float nu = w, de = valid ? w * (float)s_ss[threadIdx.x & 15] : 0.f;
-#pragma unroll
-        for (int o = 16; o; o >>= 1) {
-            nu += __shfl_xor_sync(0xffffffffu, nu, o);
-            de += __shfl_xor_sync(0xffffffffu, de, o);
-        }
-        if (threadIdx.x == 0) {
-            gpart[3 * rblk] = (float)em;
-            gpart[3 * rblk + 1] = nu;
-            gpart[3 * rblk + 2] = de;
-        }
+    const int e = s_ex[rr];
+    for (int k0 = 0; k0 < o.Kp; k0 += OZ_PREP_PASS) {
+        if (!ONE) load(k0, x);
+        if (k0 + kq < o.Kp)
+            oz_digits<4, SEL>(x, e, planes, o.X8 + (size_t)r * o.Kp + k0 + kq, (size_t)o.Rp * o.Kp);
+        if (ONE) break;
     }
-    const int kblocks = Kp / 128;
-    if (kblocks == 1)   // the statistics pass left this block's only tile in shared memory
-        oz_split_tile<PER, THREADS == 512>(v, rows, K, Rp, Kp, expo, planes, X8, rblk, tile, s_ex);
-    else
-        for (int kb = 0; kb < kblocks; kb++)
-            oz_split_tile<PER, THREADS == 512>(v, rows, K, Rp, Kp, expo, planes, X8, rblk * kblocks + kb, nullptr,
-                                               s_ex);
 }
 
-template <int THREADS>
-__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 4 : 1)
+template <bool ONE, bool SEL>
+__global__ void __launch_bounds__(OZ_PREP_THREADS)
 oz_prep_small(OzPrepOp a, OzPrepOp b, int planes, int *status)
 {
     // the product kernel may be scheduled now: its set-up needs none of this
     // launch's results, and it waits for them (griddepcontrol.wait)
-    asm volatile("griddepcontrol.launch_dependents;");
-    const int na = a.Rp / OZ_SPLIT_ROWS;
-    if ((int)blockIdx.x < na)
-        oz_prep_rows<THREADS>(a.v, a.rows, a.K, a.Rp, a.Kp, a.expo, a.ss, a.scale, a.X8, a.gpart, planes, blockIdx.x,
-                              status);
-    else
-        oz_prep_rows<THREADS>(b.v, b.rows, b.K, b.Rp, b.Kp, b.expo, b.ss, b.scale, b.X8, b.gpart, planes, blockIdx.x - na,
-                     status);
+    gbx_launch::pdl_enter();
+    const int na = a.Rp / OZ_PREP_ROWS;
+    const bool is_a = (int)blockIdx.x < na;
+    oz_prep_rows<ONE, SEL>(is_a ? a : b, planes, is_a ? blockIdx.x : blockIdx.x - na, status);
 }
 
 // ---------------------------------------------------------------------------
@@ -1566,6 +1539,8 @@ oz_gemm_sk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     volatile int *status = p.status;
 
+    // the next call's preparation may be placed on the SMs this launch leaves
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (threadIdx.x == 0) {
         for (int i = 0; i < OZS_AMAX; i++) { mbar_init(&fullA[i], 1); mbar_init(&emptyA[i], 1); }
         for (int i = 0; i < OZS_BSTG; i++) { mbar_init(&fullB[i], 1); mbar_init(&emptyB[i], 1); }
@@ -2285,7 +2260,7 @@ struct OzBuffers {
     int *rsa, *csb;   // scale exponents e-4 (rows of op(A), columns of op(B))
     double *ssa, *ssb;
     long long *W;     // nW planes of Mp x Np 128-bit running sums
-    float *gpart;     // (Mp + Np) / 16 slice-count partials of the one-launch preparation
+    float *gpart;     // slice-count partials of the one-launch preparation, one per OZ_PREP_ROWS rows
     int *status;      // the context's status words
     int *status_host; // device address of their host mirror
 };
@@ -2301,7 +2276,7 @@ gbx_status oz_buffers(gbx_ctx *ctx, int Mp, int Np, int Kp, int nW, OzBuffers &b
     if ((st = gbx_ws(ctx, GBX_WS_OZ2, 2 * sizeof(long long) * (size_t)Mp * Np * nW, &p)) != GBX_OK) return st;
     b.W = (long long *)p;
     const size_t small = 256 + sizeof(int) * (size_t)(Mp + Np) + sizeof(double) * 4 * (size_t)(Mp + Np) + 1024 +
-                         3 * sizeof(double) * (size_t)((Mp + Np) / 16 + 2);
+                         3 * sizeof(float) * (size_t)((Mp + Np) / OZ_PREP_ROWS + 2);
     if ((st = gbx_ws(ctx, GBX_WS_OZ3, small, &p)) != GBX_OK) return st;
     uint8_t *q = (uint8_t *)p;
     if ((st = gbx_ctx_status(ctx, &b.status, &b.status_host)) != GBX_OK) return st;
@@ -2433,14 +2408,14 @@ gbx_status run_ozaki(gbx_ctx *ctx, const OzProblem &pr, double tol, int forced, 
             B8 = b.B8;
             csb = b.csb;
         }
-        const long long blocks = (long long)Mp / OZ_SPLIT_ROWS + (long long)Np / OZ_SPLIT_ROWS;
+        const long long blocks = (long long)Mp / OZ_PREP_ROWS + (long long)Np / OZ_PREP_ROWS;
         if (blocks > 0x7fffffffLL) return gbx_fail(ctx, GBX_ERR_UNSUPPORTED, "ozaki: operands too large");
         oa.gpart = b.gpart;
-        ob.gpart = b.gpart + 3 * (size_t)(Mp / OZ_SPLIT_ROWS);
-        if (blocks <= gbx_ctx_sms(ctx))
-            oz_prep_small<2 * OZ_SMALL_THREADS><<<(unsigned)blocks, 2 * OZ_SMALL_THREADS, 0, s>>>(oa, ob, planes, b.status);
-        else
-            oz_prep_small<OZ_SMALL_THREADS><<<(unsigned)blocks, OZ_SMALL_THREADS, 0, s>>>(oa, ob, planes, b.status);
+        ob.gpart = b.gpart + 3 * (size_t)(Mp / OZ_PREP_ROWS);
+        const bool one = Kp <= OZ_PREP_PASS, sel = blocks <= 4LL * gbx_ctx_sms(ctx);
+        gbx_launch::launch_pdl(one ? (sel ? oz_prep_small<true, true> : oz_prep_small<true, false>)
+                                   : (sel ? oz_prep_small<false, true> : oz_prep_small<false, false>),
+                               (unsigned)blocks, OZ_PREP_THREADS, 0, s, oa, ob, planes, b.status);
         gbx_count_launch(ctx, 1);
         if ((st = gbx_check_launch(ctx, "ozaki prepare")) != GBX_OK) return st;
     } else if ((st = oz_prepare(ctx, oa, ob, b_stats, tol, forced, b.status, (unsigned *)(b.S + 4), b.S)) !=
@@ -2486,9 +2461,9 @@ gbx_status run_ozaki(gbx_ctx *ctx, const OzProblem &pr, double tol, int forced, 
     p.status = b.status;
     p.status_host = b.status_host;
     p.gpa = b.gpart;
-    p.gpb = b.gpart + 3 * (size_t)(Mp / OZ_SPLIT_ROWS);
-    p.npa = Mp / OZ_SPLIT_ROWS;
-    p.npb = Np / OZ_SPLIT_ROWS;
+    p.gpb = b.gpart + 3 * (size_t)(Mp / OZ_PREP_ROWS);
+    p.npa = Mp / OZ_PREP_ROWS;
+    p.npb = Np / OZ_PREP_ROWS;
     p.K = pr.K;
     p.tol_bits = (float)(-log2(tol));
     p.forced = forced;
