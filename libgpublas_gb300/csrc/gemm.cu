@@ -120,6 +120,12 @@ static gbx_status choose_and_launch(gbx_ctx *ctx, GemmArgs<T> p, const char *wha
     };
     if constexpr (std::is_same<T, double>::value) {
         const int bm = gbx_dgemm_tile_choice(p.m, p.n, p.c_part != C_FULL, gbx_ctx_sms(ctx));
+        gbx_timer_begin(ctx, GBX_TIMER_GEMM_FP64);
+        if (launch_gemm_short(ctx, p, bm)) {
+            gbx_timer_end(ctx);
+            gbx_count_launch(ctx, 1);
+            return gbx_check_launch(ctx, what);
+        }
         if (bm == 64) return launch_gemm_tile<T, 4>(ctx, p, what);
         if (bm == 32) return launch_gemm_tile<T, 2>(ctx, p, what);
         return launch_gemm_tile<T, 1>(ctx, p, what);
