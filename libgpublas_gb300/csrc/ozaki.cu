@@ -666,30 +666,28 @@ struct OzParams {
     int s_lo;                  // lower bound of S from the tolerance alone (small-K kernel)
 };
 
-// The small-K product kernel's slice count, computed by every CTA from the
-// preparation's per-block partials of both operands (the same data in the
+// The small-K product kernel's slice count, computed in every CTA by nt threads
+// (tid in [0, nt), named barrier bar) from the preparation's per-block partials of both operands (the same data in the
 // same order in every CTA: one S per call) with the model oz_prep_finish
 // applies, clamped to the planes the preparation wrote; CTA 0 records it.
 // Returns 0 for a call to skip (the status word is set: a non-finite operand
-// or an earlier kernel's expired wait); every thread gets the same answer
-// before any copy or MMA is issued.  The status and up to two partials per
+// or an earlier kernel's expired wait); every thread gets the same answer.  The status and up to two partials per
 // thread and operand are read in one round of loads (a round costs about a
 // microsecond at the start of a call of a few tens of microseconds).
-__device__ int oz_choose_S(const OzParams &p)
+__device__ int oz_choose_S(const OzParams &p, int tid, int nt, int bar)
 {
     constexpr int R = 2;   // partials per thread and operand held in registers
     __shared__ int s_e[2][32];
     __shared__ float s_v[4][32];
     __shared__ int s_S;
-    const int nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nt = blockDim.x;
-    const int st = threadIdx.x == 0 ? *(volatile int *)p.status : 0;
+    const int nw = nt >> 5, warp = tid >> 5, lane = tid & 31;
+    const int st = tid == 0 ? *(volatile int *)p.status : 0;
     if (p.forced > 0) {
-        if (threadIdx.x == 0) {
+        if (tid == 0) {
             s_S = st ? 0 : min(p.forced, p.smax);
             if (blockIdx.x == 0 && s_S) *p.S = s_S;
         }
-        __syncthreads();
+        gbx_launch::bar_wait(bar, nt);
         return s_S;
     }
     // the partial i is handled by thread i mod nt, in increasing i: the
@@ -700,7 +698,7 @@ __device__ int oz_choose_S(const OzParams &p)
     if (regs) {
 #pragma unroll
         for (int r = 0; r < R; r++) {
-            const int i = threadIdx.x + r * nt;
+            const int i = tid + r * nt;
             const bool va = i < p.npa, vb = i < p.npb;
 #pragma unroll
             for (int c = 0; c < 3; c++) {
@@ -710,13 +708,13 @@ __device__ int oz_choose_S(const OzParams &p)
         }
 #pragma unroll
         for (int r = 0; r < R; r++) {
-            const int i = threadIdx.x + r * nt;
+            const int i = tid + r * nt;
             if (i < p.npa) ea = max(ea, (int)pa[r][0]);
             if (i < p.npb) eb = max(eb, (int)pb[r][0]);
         }
     } else {
-        for (int i = threadIdx.x; i < p.npa; i += nt) ea = max(ea, (int)__ldcg(p.gpa + 3 * i));
-        for (int i = threadIdx.x; i < p.npb; i += nt) eb = max(eb, (int)__ldcg(p.gpb + 3 * i));
+        for (int i = tid; i < p.npa; i += nt) ea = max(ea, (int)__ldcg(p.gpa + 3 * i));
+        for (int i = tid; i < p.npb; i += nt) eb = max(eb, (int)__ldcg(p.gpb + 3 * i));
     }
 #pragma unroll
     for (int o = 16; o; o >>= 1) {
@@ -724,7 +722,7 @@ __device__ int oz_choose_S(const OzParams &p)
         eb = max(eb, __shfl_xor_sync(0xffffffffu, eb, o));
     }
     if (lane == 0) { s_e[0][warp] = ea; s_e[1][warp] = eb; }
-    __syncthreads();
+    gbx_launch::bar_wait(bar, nt);
     ea = lane < nw ? s_e[0][lane] : -100000;   // nw <= 32
     eb = lane < nw ? s_e[1][lane] : -100000;
 #pragma unroll
@@ -740,7 +738,7 @@ __device__ int oz_choose_S(const OzParams &p)
     if (regs) {
 #pragma unroll
         for (int r = 0; r < R; r++) {
-            const int i = threadIdx.x + r * nt;
+            const int i = tid + r * nt;
             if (i < p.npa) {
                 const float w = weight((int)pa[r][0], ea);
                 v[0] = fmaf(w, pa[r][1], v[0]);
@@ -749,7 +747,7 @@ __device__ int oz_choose_S(const OzParams &p)
         }
 #pragma unroll
         for (int r = 0; r < R; r++) {
-            const int i = threadIdx.x + r * nt;
+            const int i = tid + r * nt;
             if (i < p.npb) {
                 const float w = weight((int)pb[r][0], eb);
                 v[2] = fmaf(w, pb[r][1], v[2]);
@@ -757,12 +755,12 @@ __device__ int oz_choose_S(const OzParams &p)
             }
         }
     } else {
-        for (int i = threadIdx.x; i < p.npa; i += nt) {
+        for (int i = tid; i < p.npa; i += nt) {
             const float w = weight((int)__ldcg(p.gpa + 3 * i), ea);
             v[0] = fmaf(w, __ldcg(p.gpa + 3 * i + 1), v[0]);
             v[1] = fmaf(w, __ldcg(p.gpa + 3 * i + 2), v[1]);
         }
-        for (int i = threadIdx.x; i < p.npb; i += nt) {
+        for (int i = tid; i < p.npb; i += nt) {
             const float w = weight((int)__ldcg(p.gpb + 3 * i), eb);
             v[2] = fmaf(w, __ldcg(p.gpb + 3 * i + 1), v[2]);
             v[3] = fmaf(w, __ldcg(p.gpb + 3 * i + 2), v[3]);
@@ -774,7 +772,7 @@ __device__ int oz_choose_S(const OzParams &p)
         for (int o = 16; o; o >>= 1) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
         if (lane == 0) s_v[j][warp] = v[j];
     }
-    __syncthreads();
+    gbx_launch::bar_wait(bar, nt);
     if (warp == 0) {
         float t[4];
 #pragma unroll
@@ -793,7 +791,7 @@ __device__ int oz_choose_S(const OzParams &p)
             if (blockIdx.x == 0 && !st) *p.S = S;
         }
     }
-    __syncthreads();
+    gbx_launch::bar_wait(bar, nt);
     return s_S;
 }
 
@@ -1482,15 +1480,19 @@ oz_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 // 128 (N = 256: 128 cycles; measured by gbx_diag_mma_issue), so S(S+1)/2 products of
 // N = 32 would leave the tensor pipe three quarters idle; concatenated, a
 // 128-wide k block of a tile is sum_s ceil(32(S - s) / 256) * 4 MMAs (48 for
-// S = 10 instead of 220).  The A slices (16 KB each) stream through a ring
-// of up to eight stages: an A slice whose product has a narrow N is used
-// up in a few hundred cycles, so with K > 128 the ring depth, not the tensor
-// pipe, set the pace at four stages.  The B stage is double-buffered so the
+// S = 10 instead of 220).  The A slices (16 KB each) stream through a
+// ring of up to six stages of two slices: one request, one wait and one release
+// per two slices, because the issuing warp's time per slice (about 600 cycles of
+// MMAs, wait and release, whatever their width) sets the pace, not the tensor
+// pipe.  The B stage is double-buffered so the
 // next k block's (or tile's) slices load under the current MMAs.  A TMA
 // request costs the issuing thread about 80 ns, so a B stage (all P
-// prepared planes, of which the MMAs read the first S) is one 3-D request,
-// and the first tile's B stage and first A slices are requested before the
-// slice count is chosen (S >= s_lo from the tolerance alone).
+// prepared planes, of which the MMAs read the first S) is one 3-D request.
+// The slice count takes 2 us to choose; the first tile's products by the slices
+// that any count needs (S >= s_lo from the tolerance alone) run meanwhile.
+// Measured, one call's kernel at K = 256, S = 10 (512 x 256 and 2048 x 256
+// outputs): 16 and 22 us with one lane issuing slice by slice after the choice,
+// now 12 and 17.
 //
 // The drain prefetches its row's C values and scale exponents while the
 // MMAs run, then decodes each FP32 sum on the FMA and integer pipes (oz_f2i22)
@@ -1509,14 +1511,15 @@ oz_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 // most half the SMs: a call that small is one tile per CTA, and its time is
 // the tile's chain (loads, MMAs, drain); half-width tiles halve the drain
 // (the longest step: 8 conversions per thread) and double the CTAs at work.
-constexpr int OZS_BN = 32, OZS_AMAX = 8, OZS_BSTG = 2, OZS_DRAIN_WARPS = 16;
+constexpr int OZS_BN = 32, OZS_AMAX = 6, OZS_BSTG = 2, OZS_DRAIN_WARPS = 16;
+constexpr int OZS_A2 = 2 * OZ_A_BYTES;                      // an A stage: two slices
 constexpr int OZS_B_BYTES = OZS_BN * OZ_BK;                 // 4 KB: one slice's 32 rows (BN = 32)
 constexpr int OZS_THREADS = 64 + 32 * OZS_DRAIN_WARPS;
 // Dynamic shared memory: the two B stages (S x 4 KB each) and as many 16 KB
 // A stages as fit (8 for S <= 10, 6 for S = 14), barriers at the end.
 constexpr size_t OZS_SMEM = 220 * 1024;
 constexpr size_t OZS_DATA = OZS_SMEM - 1024 - 512;   // alignment slack, barriers
-static_assert(OZS_DATA >= 2 * OZ_SMAX * OZS_B_BYTES + 4 * (size_t)OZ_A_BYTES, "small-K stages");
+static_assert(OZS_DATA >= 2 * OZ_SMAX * OZS_B_BYTES + 2 * (size_t)OZS_A2, "small-K stages");
 constexpr int OZS_KMAX = 1024;
 static_assert((long long)OZ_SMAX * OZS_KMAX * 256 < (1LL << 22), "small-K diagonal sums must stay below 2^22");
 static_assert(OZ_SMAX * OZS_BN <= 512, "small-K accumulators must fit TMEM");
@@ -1534,7 +1537,9 @@ oz_gemm_sk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     uint64_t *fullA = bars, *emptyA = fullA + OZS_AMAX;
     uint64_t *fullB = emptyA + OZS_AMAX, *emptyB = fullB + OZS_BSTG;
     uint64_t *tfull = emptyB + OZS_BSTG, *tempty = tfull + 2;   // two accumulator sets
-    uint32_t *tmem_slot = (uint32_t *)(tempty + 2);
+    uint64_t *chosen = tempty + 2;                              // the slice count is known
+    uint32_t *tmem_slot = (uint32_t *)(chosen + 1);
+    __shared__ int s_count;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     volatile int *status = p.status;
@@ -1548,6 +1553,7 @@ oz_gemm_sk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             mbar_init(&tfull[i], 1);
             mbar_init(&tempty[i], 32 * OZS_DRAIN_WARPS);
         }
+        mbar_init(chosen, 1);
         fence_barrier_init();
         prefetch_tmap(&tmA);
         prefetch_tmap(&tmB);
@@ -1568,79 +1574,55 @@ oz_gemm_sk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     const int P = p.smax;   // digit planes prepared: S <= P
     const int nkb = p.Kp / OZ_BK;
     // B stages first (all P slices of BN rows each: a stage can be requested
-    // before S is known; the MMAs read the first S), then the A ring
+    // before S is known; the MMAs read the first S), then the ring of A stages of
+    // two slices each (one request, one wait and one release per two slices)
     const int bstage = P * B_BYTES;
     uint8_t *sB = smem;
     uint8_t *sA = smem + OZS_BSTG * bstage;
-    const int nA = min(OZS_AMAX, (int)((OZS_DATA - (size_t)OZS_BSTG * bstage) / OZ_A_BYTES));
+    const int nA = min(OZS_AMAX, (int)((OZS_DATA - (size_t)OZS_BSTG * bstage) / OZS_A2));
     const int ntiles = p.tiles_m * p.tiles_n;
-    // The first tile's first B stage and A slices 0..spec-1 (S >= p.s_lo, a
-    // bound from the tolerance alone) are requested before the slice count
-    // is chosen, so that these loads overlap the choice.
-    int t_first = -1, spec = 0;
-    if (warp == 0 && lane == 0) {
-        for (int t = blockIdx.x; t < ntiles; t += gridDim.x)
-            if (tile_needed(p, t / p.tiles_n, t % p.tiles_n, OZ_BM, BN)) { t_first = t; break; }
-        if (t_first >= 0) {
-            const int tm = t_first / p.tiles_n, tn = t_first % p.tiles_n;
-            spec = min(min(nA, p.s_lo), 3);   // a TMA request costs the thread ~80 ns
-            mbar_arrive_expect_tx(&fullB[0], (uint32_t)(P * B_BYTES));
-            tma_load_3d(sB, &tmB, &fullB[0], 0, tn * BN, 0);
-            for (int sa = 0; sa < spec; sa++) {
-                mbar_arrive_expect_tx(&fullA[sa], OZ_A_BYTES);
-                tma_load_2d(sA + sa * OZ_A_BYTES, &tmA, &fullA[sa], 0, sa * p.Mp + tm * OZ_BM);
-            }
-        }
-    }
-    const int S = oz_choose_S(p);   // 0: skip this call
-    if (S == 0) {
-        // the early loads land before the CTA leaves (a wait bounded by time
-        // only: the status word is set on this path)
-        if (warp == 0 && lane == 0 && t_first >= 0) {
-            const uint64_t t0 = globaltimer();
-            while (!mbar_try_wait(&fullB[0], 0u) && globaltimer() - t0 < WAIT_LIMIT_NS) {}
-            for (int sa = 0; sa < spec; sa++)
-                while (!mbar_try_wait(&fullA[sa], 0u) && globaltimer() - t0 < WAIT_LIMIT_NS) {}
-        }
-        if (warp == 1) {
-            tc_fence_after();
-            tmem_dealloc(tmem_base, 512);
-        }
-        __syncthreads();
-        oz_report(p);
-        return;
-    }
-    // Accumulator sets in TMEM: two of 256 columns when a tile's S diagonals
-    // fit (S * BN <= 256: always for BN = 16), so that a tile's MMAs run while
+    // The slice count takes the drain warps about 2 us to choose, but it is
+    // at least s_lo, a bound from the tolerance alone: the first tile's first
+    // B stage and the A stages of slices 0 .. s_lo - 1 are loaded and multiplied
+    // meanwhile, by all P planes of B (diagonals from S on are not read), whatever
+    // the status word says; then both roles wait for the count, and for 0 (skip
+    // this call) end with everything they started complete.
+    const int early = p.s_lo / 2;
+    // Accumulator sets in TMEM: two of 256 columns when a tile's P diagonals
+    // fit (P * BN <= 256: always for BN = 16), so that a tile's MMAs run while
     // the previous tile's sums are read out; else one
-    const int nbuf = S * BN <= 256 ? 2 : 1;
+    const int nbuf = P * BN <= 256 ? 2 : 1;
+    auto wait_count = [&]() {
+        return mbar_wait_timed(chosen, 0u, status, TC_TIMEOUT_FULL) ? *(volatile int *)&s_count : 0;
+    };
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         if (lane == 0) {
-            int as = 0, bs = 0;
+            int as = 0, bs = 0, S = -1;
             uint32_t ap = 0, bp = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
                 const int tm = t / p.tiles_n, tn = t % p.tiles_n;
                 if (!tile_needed(p, tm, tn, OZ_BM, BN)) continue;
                 for (int kb = 0; kb < nkb && ok; kb++) {
-                    // requested before the slice count was chosen
-                    const bool early = t == t_first && kb == 0;
-                    // the B stage: slices 0..P-1 of the tile's BN columns, side by side
-                    if (!early) {
-                        if (!mbar_wait(&emptyB[bs], bp ^ 1u, status, TC_TIMEOUT_EMPTY)) { ok = false; break; }
-                        mbar_arrive_expect_tx(&fullB[bs], (uint32_t)(P * B_BYTES));
-                        tma_load_3d(sB + bs * bstage, &tmB, &fullB[bs], kb * OZ_BK, tn * BN, 0);   // P planes
-                    }
+                    // the B stage: all planes of the tile's BN columns, side by side
+                    if (!mbar_wait(&emptyB[bs], bp ^ 1u, status, TC_TIMEOUT_EMPTY)) { ok = false; break; }
+                    mbar_arrive_expect_tx(&fullB[bs], (uint32_t)(P * B_BYTES));
+                    tma_load_3d(sB + bs * bstage, &tmB, &fullB[bs], kb * OZ_BK, tn * BN, 0);
                     if (++bs == OZS_BSTG) { bs = 0; bp ^= 1u; }
-                    // then the A slices
-                    for (int sa = 0; sa < S; sa++) {
-                        if (!(early && sa < spec)) {
-                            if (!mbar_wait(&emptyA[as], ap ^ 1u, status, TC_TIMEOUT_EMPTY)) { ok = false; break; }
-                            mbar_arrive_expect_tx(&fullA[as], OZ_A_BYTES);
-                            tma_load_2d(sA + as * OZ_A_BYTES, &tmA, &fullA[as], kb * OZ_BK, sa * p.Mp + tm * OZ_BM);
+                    // then the A slices, two at a time (a plane beyond S is loaded
+                    // with the last odd one and not used)
+                    for (int a2 = 0;; a2++) {
+                        if (S < 0 && a2 >= early) {
+                            S = wait_count();
+                            if (S == 0) ok = false;
                         }
+                        if (!ok || (S >= 0 && 2 * a2 >= S)) break;
+                        if (!(S < 0 ? mbar_wait_timed(&emptyA[as], ap ^ 1u, status, TC_TIMEOUT_EMPTY)
+                                    : mbar_wait(&emptyA[as], ap ^ 1u, status, TC_TIMEOUT_EMPTY))) { ok = false; break; }
+                        mbar_arrive_expect_tx(&fullA[as], OZS_A2);
+                        tma_load_3d(sA + as * OZS_A2, &tmA, &fullA[as], kb * OZ_BK, tm * OZ_BM, 2 * a2);
                         if (++as == nA) { as = 0; ap ^= 1u; }
                     }
                 }
@@ -1656,56 +1638,78 @@ oz_gemm_sk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            int as = 0, bs = 0, tbuf = 0;
-            uint32_t ap = 0, bp = 0, tp = 0;
-            bool ok = true;
-            const uint32_t a_base = smem_u32(sA), b_base = smem_u32(sB);
-            for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
-                const int tm = t / p.tiles_n, tn = t % p.tiles_n;
-                if (!tile_needed(p, tm, tn, OZ_BM, BN)) continue;
-                // this accumulator set's previous sums have been read out of TMEM
-                if (!mbar_wait(&tempty[tbuf], tp ^ 1u, status, TC_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
-                tc_fence_after();
-                for (int kb = 0; kb < nkb && ok; kb++) {
-                    if (!mbar_wait(&fullB[bs], bp, status, TC_TIMEOUT_FULL)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint32_t b_addr = b_base + bs * bstage;
-                    for (int sa = 0; sa < S; sa++) {
-                        if (!mbar_wait(&fullA[as], ap, status, TC_TIMEOUT_FULL)) { ok = false; break; }
-                        tc_fence_after();
-                        const uint32_t a_addr = a_base + as * OZ_A_BYTES;
-                        // A_s against B_0..B_{S-1-s}: columns BN s.. of TMEM, N <= 256 per MMA.
-                        // Descriptors are built once per stage and advanced by 32 bytes
-                        // (2 in the address field) per k step: the issuing thread shares
-                        // its SMSP with four drain warps, so its instructions are few.
-                        const uint64_t a_d = smem_desc_k128(a_addr);
-                        // the first k block's s = 0 products start every diagonal
-                        const uint32_t acc0 = (kb == 0 && sa == 0) ? 0u : 1u;
-                        const int ntot = BN * (S - sa);
-                        for (int c0 = 0; c0 < ntot; c0 += 256) {
-                            const int n = min(256, ntot - c0);
-                            const uint32_t idesc = idesc_e4m3_f32(OZ_BM, n);
-                            const uint32_t d_tmem = tmem_base + (uint32_t)(tbuf * 256 + BN * sa + c0);
-                            const uint64_t b_d = smem_desc_k128(b_addr + (uint32_t)c0 * OZ_BK);
+        // ---------------- MMA issuer (the whole warp, one lane elected) ----------------
+        int as = 0, bs = 0, tbuf = 0, S = -1;
+        uint32_t ap = 0, bp = 0, tp = 0;
+        bool ok = true;
+        auto all = [](bool v) { return __all_sync(0xffffffffu, v) != 0; };   // uniform
+        const uint64_t a_desc = smem_desc_k128(__shfl_sync(0xffffffffu, smem_u32(sA), 0));
+        const uint64_t b_desc = smem_desc_k128(__shfl_sync(0xffffffffu, smem_u32(sB), 0));
+        const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+        // A_s against B_0..B_{W-1-s} (W = S, or P while S is not known): columns
+        // BN s.. of TMEM, N <= 256 per MMA
+        auto slice = [&](int sa, int W, uint64_t a_d, uint64_t b_d, uint32_t acc0) {
+            const int ntot = BN * (W - sa);
+            for (int c0 = 0; c0 < ntot; c0 += 256) {
+                const uint32_t idesc = idesc_e4m3_f32(OZ_BM, min(256, ntot - c0));
+                const uint32_t d = tmem + (uint32_t)(tbuf * 256 + BN * sa + c0);
+                const uint64_t b = b_d + (uint64_t)((c0 * OZ_BK) >> 4);
 #pragma unroll
-                            for (int kk = 0; kk < OZ_BK / 32; kk++)
-                                mma_f8f6f4(d_tmem, a_d + 2 * kk, b_d + 2 * kk, idesc, kk == 0 ? acc0 : 1u);
+                for (int kk = 0; kk < OZ_BK / 32; kk++) mma_f8f6f4(d, a_d + 2 * kk, b + 2 * kk, idesc, kk == 0 ? acc0 : 1u);
+            }
+        };
+        for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
+            const int tm = t / p.tiles_n, tn = t % p.tiles_n;
+            if (!tile_needed(p, tm, tn, OZ_BM, BN)) continue;
+            // this accumulator set's previous sums have been read out of TMEM
+            ok = all(mbar_wait(&tempty[tbuf], tp ^ 1u, status, TC_TIMEOUT_TMEM_EMPTY));
+            for (int kb = 0; kb < nkb && ok; kb++) {
+                ok = all(S < 0 ? mbar_wait_timed(&fullB[bs], bp, status, TC_TIMEOUT_FULL)
+                               : mbar_wait(&fullB[bs], bp, status, TC_TIMEOUT_FULL));
+                const uint64_t b_d = b_desc + (uint64_t)((bs * bstage) >> 4);
+                for (int a2 = 0; ok; a2++) {
+                    if (S < 0 && a2 >= early) {
+                        S = __shfl_sync(0xffffffffu, wait_count(), 0);
+                        if (S == 0) {
+                            // what was issued completes before TMEM is given back
+                            if (elect_one()) mma_commit(&tfull[tbuf]);
+                            __syncwarp();
+                            mbar_wait_timed(&tfull[tbuf], tp, status, TC_TIMEOUT_FULL);
+                            ok = false;
                         }
-                        mma_commit(&emptyA[as]);
-                        if (++as == nA) { as = 0; ap ^= 1u; }
                     }
+                    if (!ok || (S >= 0 && 2 * a2 >= S)) break;
+                    ok = all(S < 0 ? mbar_wait_timed(&fullA[as], ap, status, TC_TIMEOUT_FULL)
+                                   : mbar_wait(&fullA[as], ap, status, TC_TIMEOUT_FULL));
                     if (!ok) break;
-                    mma_commit(&emptyB[bs]);
-                    if (++bs == OZS_BSTG) { bs = 0; bp ^= 1u; }
+                    tc_fence_after();
+                    const uint64_t a_d = a_desc + (uint64_t)((as * OZS_A2) >> 4);
+                    const int W = S < 0 ? P : S, sa = 2 * a2;
+                    if (elect_one()) {
+                        // the first k block's s = 0 products start every diagonal
+                        slice(sa, W, a_d, b_d, (kb == 0 && sa == 0) ? 0u : 1u);
+                        if (sa + 1 < W) slice(sa + 1, W, a_d + (OZ_A_BYTES >> 4), b_d, 1u);
+                        mma_commit(&emptyA[as]);
+                    }
+                    __syncwarp();
+                    if (++as == nA) { as = 0; ap ^= 1u; }
                 }
                 if (!ok) break;
-                mma_commit(&tfull[tbuf]);
-                if (++tbuf == nbuf) { tbuf = 0; tp ^= 1u; }
+                if (elect_one()) mma_commit(&emptyB[bs]);
+                __syncwarp();
+                if (++bs == OZS_BSTG) { bs = 0; bp ^= 1u; }
             }
+            if (!ok) break;
+            if (elect_one()) mma_commit(&tfull[tbuf]);
+            __syncwarp();
+            if (++tbuf == nbuf) { tbuf = 0; tp ^= 1u; }
         }
     } else {
+        const int S = oz_choose_S(p, (int)threadIdx.x - 64, 32 * OZS_DRAIN_WARPS, 1);   // 0: skip this call
+        if (threadIdx.x == 64) {
+            s_count = S;
+            mbar_arrive(chosen);
+        }
         // ---------------- drain (warps 2..17) ----------------
         const int quarter = warp & 3;               // TMEM lane window of this warp
         const int cg = (warp - 2) >> 2;             // columns cg*DCOLS .. of the tile
@@ -1715,7 +1719,7 @@ oz_gemm_sk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         const int lsh = 5 * (S - g);                // weight of the high half over the low one
         uint32_t tp = 0;
         int tbuf = 0;
-        bool ok = true;
+        bool ok = S > 0;
         for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
             const int tm = t / p.tiles_n, tn = t % p.tiles_n;
             if (!tile_needed(p, tm, tn, OZ_BM, BN)) continue;
@@ -2429,7 +2433,8 @@ gbx_status run_ozaki(gbx_ctx *ctx, const OzProblem &pr, double tol, int forced, 
     // wide tiles: also a half-width B box for the half tiles of the last wave
     const bool wide = !small_k && !pair;
     const int inner = wide ? OZ_WBK : OZ_BK;
-    if (!make_map(&tmA, b.A8, (long long)OZ_SMAX * Mp, Kp, OZ_BM, inner) ||
+    if (!(small_k ? make_map(&tmA, b.A8, Mp, Kp, -(OZ_BM * 256 + 2))
+                  : make_map(&tmA, b.A8, (long long)OZ_SMAX * Mp, Kp, OZ_BM, inner)) ||
         !(small_k ? make_map(&tmB, B8, Np, Kp, -(bn * 256 + planes))
                   : make_map(&tmB, B8, (long long)OZ_SMAX * Np, Kp, pair ? 128 : (mc ? bn / 2 : bn), inner)) ||
         (wide && !make_map(&tmBh, B8, (long long)OZ_SMAX * Np, Kp, mc ? bn / 4 : bn / 2, inner)) ||

@@ -90,6 +90,31 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
     }
 }
 
+// The same wait for work that is in flight whatever the status word says: only
+// the deadline ends it.
+__device__ __forceinline__ bool mbar_wait_timed(uint64_t *bar, uint32_t parity, volatile int *status, int code)
+{
+    if (mbar_try_wait(bar, parity)) return true;
+    const uint64_t t0 = globaltimer();
+    while (!mbar_try_wait(bar, parity))
+        if (globaltimer() - t0 > WAIT_LIMIT_NS) {
+            atomicCAS((int *)status, TC_OK, code);
+            return false;
+        }
+    return true;
+}
+
+// One lane of a converged warp, the same one every time.  A warp that issues
+// MMAs runs its loop as a whole and elects a lane for them: the loop's values are
+// then uniform, and an MMA's descriptors need no move from a lane's registers
+// (one lane running the loop alone took 150 cycles per MMA, this form 125).
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
+}
+
 // 2-D TMA tile load into shared memory, completion on an mbarrier.
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, uint64_t *bar, int x, int y)
 {
