@@ -1358,52 +1358,56 @@ oz_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            int stage = 0, buf = 0;
-            uint32_t phase = 0, tphase = 0;
-            bool ok = true;
-            const uint32_t smem_base = smem_u32(smem);
-            for (int u = unit0; u < p.nunits && ok; u += ustep) {
-                int tm, tn, col_off;
-                bool narrow;
-                oz_unit(p, u, BN, MROWS, rank, tm, tn, col_off, narrow);
-                if (!MC && !oz_unit_needed(p, tm, tn, col_off, narrow, BN)) continue;
-                const uint32_t idesc = narrow ? idesc_e4m3_f32(OZ_BM, BN / 2) : idesc_e4m3_f32(OZ_BM, BN);
-                for (int q = 0; q < gp.S && ok; q++) {
-                    const int s_lo = max(0, q - (gp.S - 1)), s_hi = min(q, gp.S - 1);
-                    const int nitems = (s_hi - s_lo + 1) * gp.nchunks;
-                    const int ng = gp.ngroups(nitems);
-                    for (int g = 0; g < ng && ok; g++) {
-                        const int g0 = gp.gbegin(nitems, ng, g), g1 = gp.gbegin(nitems, ng, g + 1);
-                        if (!mbar_wait(&tempty[buf], tphase ^ 1u, status, TC_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
-                        tc_fence_after();
-                        const uint32_t d_tmem = tmem_base + (uint32_t)(buf * BN);
-                        uint32_t acc = 0;
-                        for (int it = g0; it < g1 && ok; it++) {
-                            const int ch = it % gp.nchunks;
-                            const int kb0 = ch * gp.kch_blocks, kb1 = min(gp.nkb, kb0 + gp.kch_blocks);
-                            for (int kb = kb0; kb < kb1; kb++) {
-                                if (!mbar_wait(&full[stage], phase, status, TC_TIMEOUT_FULL)) { ok = false; break; }
-                                tc_fence_after();
-                                const uint32_t a_addr = smem_base + stage * STAGE_BYTES;
-                                // descriptors built once per stage, advanced by 32 bytes
-                                // (2 in the address field) per k step
-                                const uint64_t a_d = smem_desc_kmaj<Cfg::BK>(a_addr);
-                                const uint64_t b_d = smem_desc_kmaj<Cfg::BK>(a_addr + Cfg::A_BYTES);
+        // ---------------- MMA issuer (the whole warp, one lane elected) ----------------
+        int stage = 0, buf = 0;
+        uint32_t phase = 0, tphase = 0;
+        bool ok = true;
+        auto all = [](bool v) { return __all_sync(0xffffffffu, v) != 0; };   // uniform
+        const uint64_t s_desc = smem_desc_kmaj<Cfg::BK>(__shfl_sync(0xffffffffu, smem_u32(smem), 0));
+        const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+        for (int u = unit0; u < p.nunits && ok; u += ustep) {
+            int tm, tn, col_off;
+            bool narrow;
+            oz_unit(p, u, BN, MROWS, rank, tm, tn, col_off, narrow);
+            if (!MC && !oz_unit_needed(p, tm, tn, col_off, narrow, BN)) continue;
+            const uint32_t idesc = narrow ? idesc_e4m3_f32(OZ_BM, BN / 2) : idesc_e4m3_f32(OZ_BM, BN);
+            for (int q = 0; q < gp.S && ok; q++) {
+                const int s_lo = max(0, q - (gp.S - 1)), s_hi = min(q, gp.S - 1);
+                const int nitems = (s_hi - s_lo + 1) * gp.nchunks;
+                const int ng = gp.ngroups(nitems);
+                for (int g = 0; g < ng && ok; g++) {
+                    const int g0 = gp.gbegin(nitems, ng, g), g1 = gp.gbegin(nitems, ng, g + 1);
+                    ok = all(mbar_wait(&tempty[buf], tphase ^ 1u, status, TC_TIMEOUT_TMEM_EMPTY));
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t d_tmem = tmem + (uint32_t)(buf * BN);
+                    uint32_t acc = 0;
+                    for (int it = g0; it < g1 && ok; it++) {
+                        const int ch = it % gp.nchunks;
+                        const int kb0 = ch * gp.kch_blocks, kb1 = min(gp.nkb, kb0 + gp.kch_blocks);
+                        for (int kb = kb0; kb < kb1; kb++) {
+                            ok = all(mbar_wait(&full[stage], phase, status, TC_TIMEOUT_FULL));
+                            if (!ok) break;
+                            tc_fence_after();
+                            // one descriptor, advanced by the stage and by 32 bytes
+                            // (2 in the address field) per k step
+                            const uint64_t a_d = s_desc + (uint64_t)((stage * STAGE_BYTES) >> 4);
+                            const uint64_t b_d = a_d + (uint64_t)(Cfg::A_BYTES >> 4);
+                            if (elect_one()) {
 #pragma unroll
-                                for (int kk = 0; kk < Cfg::BK / 32; kk++) {
-                                    mma_f8f6f4(d_tmem, a_d + 2 * kk, b_d + 2 * kk, idesc, acc);
-                                    acc = 1;
-                                }
+                                for (int kk = 0; kk < Cfg::BK / 32; kk++)
+                                    mma_f8f6f4(d_tmem, a_d + 2 * kk, b_d + 2 * kk, idesc, kk ? 1u : acc);
                                 if (MC) mma_commit_mc(&empty[stage], (uint16_t)3u);
                                 else mma_commit(&empty[stage]);
-                                if (++stage == STAGES) { stage = 0; phase ^= 1u; }
                             }
+                            __syncwarp();
+                            acc = 1;
+                            if (++stage == STAGES) { stage = 0; phase ^= 1u; }
                         }
-                        mma_commit(&tfull[buf]);
-                        if (++buf == NBUF) { buf = 0; tphase ^= 1u; }
                     }
+                    if (elect_one()) mma_commit(&tfull[buf]);
+                    __syncwarp();
+                    if (++buf == NBUF) { buf = 0; tphase ^= 1u; }
                 }
             }
         }
@@ -1957,12 +1961,15 @@ oz_gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer (even CTA only) ----------------
-        if (leader && lane == 0) {
+        // ---------------- MMA issuer (the even CTA's whole warp, one lane elected) ----------------
+        if (leader) {
             int stage = 0, buf = 0;
             uint32_t phase = 0, tphase = 0;
             bool ok = true;
-            const uint32_t smem_base = smem_u32(smem);
+            auto all = [](bool v) { return __all_sync(0xffffffffu, v) != 0; };   // uniform
+            const uint64_t s_desc = smem_desc_k128(__shfl_sync(0xffffffffu, smem_u32(smem), 0));
+            const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+            const uint16_t mask = (uint16_t)(3u << __shfl_sync(0xffffffffu, leader_rank, 0));
             for (int u = pair; u < p.nunits && ok; u += npairs) {
                 int tm, tn, col_off;
                 bool narrow;
@@ -1975,29 +1982,33 @@ oz_gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     const int ng = gp.ngroups(nitems);
                     for (int g = 0; g < ng && ok; g++) {
                         const int g0 = gp.gbegin(nitems, ng, g), g1 = gp.gbegin(nitems, ng, g + 1);
-                        if (!mbar_wait_cl(&tempty[buf], tphase ^ 1u, status, TC_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
+                        ok = all(mbar_wait_cl(&tempty[buf], tphase ^ 1u, status, TC_TIMEOUT_TMEM_EMPTY));
+                        if (!ok) break;
                         tc_fence_after();
-                        const uint32_t d_tmem = tmem_base + (uint32_t)(buf * OZ_BN);
+                        const uint32_t d_tmem = tmem + (uint32_t)(buf * OZ_BN);
                         uint32_t acc = 0;
                         for (int it = g0; it < g1 && ok; it++) {
                             const int ch = it % gp.nchunks;
                             const int kb0 = ch * gp.kch_blocks, kb1 = min(gp.nkb, kb0 + gp.kch_blocks);
                             for (int kb = kb0; kb < kb1; kb++) {
-                                if (!mbar_wait_cl(&full[stage], phase, status, TC_TIMEOUT_FULL)) { ok = false; break; }
+                                ok = all(mbar_wait_cl(&full[stage], phase, status, TC_TIMEOUT_FULL));
+                                if (!ok) break;
                                 tc_fence_after();
-                                const uint32_t a_addr = smem_base + stage * OZ2_STAGE_BYTES;
-                                const uint64_t a_d = smem_desc_k128(a_addr);
-                                const uint64_t b_d = smem_desc_k128(a_addr + OZ2_HALF);
+                                const uint64_t a_d = s_desc + (uint64_t)((stage * OZ2_STAGE_BYTES) >> 4);
+                                const uint64_t b_d = a_d + (uint64_t)(OZ2_HALF >> 4);
+                                if (elect_one()) {
 #pragma unroll
-                                for (int kk = 0; kk < OZ_BK / 32; kk++) {
-                                    mma_f8f6f4_pair(d_tmem, a_d + 2 * kk, b_d + 2 * kk, idesc, acc);
-                                    acc = 1;
+                                    for (int kk = 0; kk < OZ_BK / 32; kk++)
+                                        mma_f8f6f4_pair(d_tmem, a_d + 2 * kk, b_d + 2 * kk, idesc, kk ? 1u : acc);
+                                    mma_commit_pair_mc(&empty[stage], mask);
                                 }
-                                mma_commit_pair_mc(&empty[stage], (uint16_t)(3u << leader_rank));
+                                __syncwarp();
+                                acc = 1;
                                 if (++stage == OZ2_STAGES) { stage = 0; phase ^= 1u; }
                             }
                         }
-                        mma_commit_pair_mc(&tfull[buf], (uint16_t)(3u << leader_rank));
+                        if (elect_one()) mma_commit_pair_mc(&tfull[buf], mask);
+                        __syncwarp();
                         if (++buf == 2) { buf = 0; tphase ^= 1u; }
                     }
                 }
@@ -2224,14 +2235,13 @@ bool oz_small_k(int K)
     return env != 0 && K <= 1024;
 }
 
-// The CTA-pair kernel takes the products (K > 1024) of at most four waves of
-// its 256 x 256 tiles: measured one after another on one GB300 it ran 2048^3
-// in 0.50 ms against 0.70 ms and 4096^3 in 2.90 against 3.07 ms of the
-// one-CTA kernel; from 8192 on (calls of 20 ms and more under the power
-// cap) it draws more power, the SM clock falls further, and it ties (8192)
-// or loses (16384: 185-194 against 163 ms).  GBX_OZAKI_PAIR=1 selects it
-// for every product with more than one 128-row tile (small K included),
-// GBX_OZAKI_PAIR=0 never.
+// The CTA-pair kernel takes the products (K > 1024) of at most ten waves of
+// its 256 x 256 tiles.  Whole calls, pair / one-CTA kernel, uniform operands:
+// 2048^3 0.45 / 0.70 ms, 4096^3 2.64 / 3.07, 5120^3 4.84 / 5.41, 6144^3 8.4 / 9.0,
+// 7168^3 (10.3 waves) 13.8 / 14.2; at 8192 (calls of 20 ms and more under the
+// power cap) it draws more power, the SM clock falls further, and it loses by
+// 1.5 %.  GBX_OZAKI_PAIR=1 selects it for every product with more than one
+// 128-row tile (small K included), GBX_OZAKI_PAIR=0 never.
 bool oz_use_pair(int M, int N, int K, int sms)
 {
     static int env = [] {
@@ -2242,7 +2252,7 @@ bool oz_use_pair(int M, int N, int K, int sms)
     if (env > 0) return true;
     if (rup(std::max(K, 1), OZ_BK) <= OZS_KMAX && oz_small_k(K)) return false;
     const long long tiles = (long long)((M + OZ2_BM - 1) / OZ2_BM) * ((N + OZ_BN - 1) / OZ_BN);
-    return tiles <= 4LL * std::max(1, sms / 2);
+    return tiles <= 10LL * std::max(1, sms / 2);
 }
 
 // Column tile: 128 when N fits in it (the rank-nb updates of blocked
