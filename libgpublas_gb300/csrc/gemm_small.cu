@@ -1,8 +1,9 @@
-// gemm_small.cu — FP64 GEMM launches of at most a few waves: the core's tiles
+// gemm_small.cu — FP64 GEMM launches of at most one CTA per SM: the core's tiles
 // launched so that they overlap the end of the kernel before them, and a
-// half-height tile for products that would leave most SMs idle.  (Kernels of
-// their own: the overlap's two instructions per CTA cost 0.2 % of a long launch,
-// DGEMM 2999 x 2500 x 2777.)
+// half-height tile for products that would leave most SMs idle.  (Not larger
+// ones: CTAs placed while the kernel before still runs spread unevenly over the
+// SMs, and the FP64 pipe of the fullest SM sets the time: DGEMM 756 x 330 x 1710,
+// 1008 tiles, took 873 us overlapped and 769 not.)
 #include "gbx_internal.h"
 #include "gemm_host.h"
 #include "launch.cuh"
@@ -102,7 +103,7 @@ namespace gbx_gemm {
 
 // The FP64 launches this file takes; bm: the core's tile (64, 32, 16).  Half-
 // height tiles when 16 x 16 tiles would leave half the SMs idle and the operands
-// are plain; otherwise the core's tile, overlapping, up to eight CTAs per SM.
+// are plain; otherwise the core's tile, overlapping, up to one CTA per SM.
 bool launch_gemm_short(gbx_ctx *ctx, GemmArgs<double> p, int bm)
 {
     const int sms = gbx_ctx_sms(ctx);
@@ -119,7 +120,7 @@ bool launch_gemm_short(gbx_ctx *ctx, GemmArgs<double> p, int bm)
     p.tiles_n = (p.n + bm - 1) / bm;
     const long long blocks = p.c_part == C_FULL ? (long long)p.tiles_m * p.tiles_n
                                                 : (long long)p.tiles_m * (p.tiles_m + 1) / 2;
-    if (blocks > 8LL * sms || (p.c_part != C_FULL && p.m != p.n)) return false;
+    if (blocks > sms || (p.c_part != C_FULL && p.m != p.n)) return false;
     launch_pdl(bm == 64 ? gemm_overlap_kernel<4, 8> : (bm == 32 ? gemm_overlap_kernel<2, 8> : gemm_overlap_kernel<1, 16>),
                (unsigned)blocks, GEMM_THREADS, 0, s, p);
     return true;
