@@ -17,9 +17,10 @@ using gbx_launch::pdl_enter;
 namespace {
 
 // 8 x 16 tile of a full C = alpha op(A) op(B) + beta C by 128 threads, one
-// element each.  An FP64 warp instruction takes 64 cycles on its SM sub-
-// partition, so the eight warps of the core's 16 x 16 tile take 128 cycles per
-// k and the four of this one 64, the latency of the FMA chain itself; what is
+// element each.  A warp has one FP64 instruction in flight, 65 cycles each, and
+// the SM's pipe takes 16 to 19 cycles per warp: the eight warps of the core's
+// 16 x 16 tile take 128 to 150 cycles per k and the four of this one 65 to 77,
+// the latency of the FMA chain itself; what is
 // left is the latency of the loads, so a panel is 64 k deep (one round of loads
 // up to K = 64) and C is fetched under the products.  Each element is one FMA
 // chain over k in increasing order and the core's epilogue: the bits of any

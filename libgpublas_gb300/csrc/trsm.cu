@@ -15,9 +15,12 @@
 // (transa 'C') conjugates the inverted blocks and the GEMM operands.
 #include "gbx_internal.h"
 #include "gemm_host.h"
+#include "launch.cuh"
+#include "tri_inverse.cuh"
 
 #include <cuda_runtime.h>
 #include <algorithm>
+#include <type_traits>
 
 using namespace gbx_gemm;
 
@@ -81,6 +84,89 @@ trinv_blocks(int na, const T *__restrict__ A, long long lda, int tr, int cj, int
     for (int i = 0; i < NB; i++) out[(long long)j * NB + i] = X[i * NB + j];
 }
 
+// The same for double, by 256 threads per block (gbx_tri::invert64): a thread
+// per column stepping through 64 rows took 165 us (a warp has one FP64
+// instruction in flight, 65 cycles each), now 29.  An upper triangle is inverted
+// as the lower one it becomes when rows and columns are reversed.
+constexpr size_t TRINV64_SMEM = sizeof(double) * (2 * gbx_tri::NB * gbx_tri::LD + 32 * 33);
+__global__ void __launch_bounds__(256)
+trinv64_blocks(int na, const double *__restrict__ A, long long lda, int tr, int lower, int unit,
+               double *__restrict__ Inv)
+{
+    extern __shared__ __align__(16) unsigned char sm_raw[];
+    double *D = (double *)sm_raw, *X = D + NB * gbx_tri::LD, *W = X + NB * gbx_tri::LD;
+    const int r0 = blockIdx.x * NB, nbb = min(NB, na - r0);
+    // position p of the reversed block is row (column) NB - 1 - p; identity beyond na
+    for (int t = threadIdx.x; t < NB * NB; t += blockDim.x) {
+        const int u = t & 63, v = t >> 6;
+        const int r = tr ? v : u, c = tr ? u : v;   // row, column of op(A)'s block
+        double d = r == c ? 1.0 : 0.0;
+        if (r < nbb && c < nbb && (lower ? c <= r : c >= r) && !(unit && r == c))
+            d = tr ? A[(long long)(r0 + r) * lda + r0 + c] : A[(long long)(r0 + c) * lda + r0 + r];
+        const int i = lower ? r : NB - 1 - r, k = lower ? c : NB - 1 - c;
+        D[k * gbx_tri::LD + i] = d;
+    }
+    __syncthreads();
+    gbx_tri::invert64(D, X, W);
+    double *out = Inv + (long long)blockIdx.x * NB * NB;
+    for (int t = threadIdx.x; t < NB * NB; t += blockDim.x) {
+        const int i = t & 63, k = t >> 6;
+        out[t] = lower ? X[k * gbx_tri::LD + i] : X[(NB - 1 - k) * gbx_tri::LD + NB - 1 - i];
+    }
+}
+
+// Leaf of a double solve, in place: B(64 rows, n) = inv B (left) or B(m, 64
+// columns) = B inv (right), inv the 64 x 64 inverted diagonal block (triangular,
+// lower or upper), TL_V vectors of 64 (columns, or rows) per CTA.  Thread (i, q):
+// element i of TL_V / 4 vectors; a warp skips the half of k that is zero for its
+// 32 elements.  Eight vectors per CTA, or four where that still leaves no SM a
+// second CTA.  For 1024 vectors the FP64 pipe alone takes 7 us; DTRSM 8192 x 1024
+// lost 4 us per leaf to a GEMM into scratch and a copy back instead.
+template <int TL_V>
+__global__ void __launch_bounds__(256)
+trsm_leaf(int len, int nvec, int right, int lower, const double *__restrict__ inv, double *__restrict__ B,
+          long long ldb)
+{
+    gbx_launch::pdl_enter();
+    __shared__ double sI[NB][NB + 1];    // [k][i]: coefficient of input k in output i
+    __shared__ double sB[TL_V][NB];
+    const int v0 = blockIdx.x * TL_V;
+    for (int t = threadIdx.x; t < NB * NB; t += 256) {
+        const int a = t & 63, b = t >> 6;   // inv is column-major: element (a, b)
+        // left: out_i = sum_k inv(i, k) in_k; right: out_i = sum_k in_k inv(k, i)
+        if (right) sI[a][b] = inv[t];
+        else sI[b][a] = inv[t];
+    }
+    auto at = [&](int v, int i) { return B + (right ? (long long)i * ldb + v0 + v : (long long)(v0 + v) * ldb + i); };
+    for (int t = threadIdx.x; t < NB * TL_V; t += 256) {
+        const int i = right ? t / TL_V : t % NB, v = right ? t % TL_V : t / NB;   // contiguous index fastest
+        sB[v][i] = i < len && v0 + v < nvec ? *at(v, i) : 0.0;
+    }
+    __syncthreads();
+    const int i = threadIdx.x & 63, q = threadIdx.x >> 6;
+    constexpr int PER = TL_V / 4;
+    double acc[PER];
+#pragma unroll
+    for (int j = 0; j < PER; j++) acc[j] = 0.0;
+    // out_i uses inputs k <= i (lower from the left, upper from the right) or k >= i
+    const bool below = (lower != 0) != (right != 0);
+    const int k0 = !below && i >= 32 ? 32 : 0, k1 = below && i < 32 ? 32 : NB;
+#pragma unroll 8
+    for (int k = k0; k < k1; k++) {
+        const double c = sI[k][i];
+#pragma unroll
+        for (int j = 0; j < PER; j++) acc[j] = fma(c, sB[q * PER + j][k], acc[j]);
+    }
+    __syncthreads();   // every input is read
+#pragma unroll
+    for (int j = 0; j < PER; j++) sB[q * PER + j][i] = acc[j];
+    __syncthreads();
+    for (int t = threadIdx.x; t < NB * TL_V; t += 256) {
+        const int o = right ? t / TL_V : t % NB, v = right ? t % TL_V : t / NB;
+        if (o < len && v0 + v < nvec) *at(v, o) = sB[v][o];
+    }
+}
+
 template <typename T>
 struct Trsm {
     gbx_ctx *ctx;
@@ -92,7 +178,7 @@ struct Trsm {
     T *B;
     long long ldb;
     const T *Inv;
-    T *Tw;   // NB x n (left) or m x NB (right)
+    T *Tw;   // NB x n (left) or m x NB (right); none for double, whose leaves are in place
 
     // op(A)[r0:, c0:] as a GEMM operand: pointer and transposition flag
     const T *opA(int r0, int c0, int &t) const
@@ -115,6 +201,15 @@ struct Trsm {
         return launch_gemm<T>(ctx, p, nm);
     }
 
+    gbx_status leaf(int right_side, int len, int nvec, const double *inv, double *Bp)
+    {
+        const int v = (nvec + 3) / 4 <= gbx_ctx_sms(ctx) ? 4 : 8;
+        gbx_launch::launch_pdl(v == 4 ? trsm_leaf<4> : trsm_leaf<8>, (unsigned)((nvec + v - 1) / v), 256, 0, S(ctx), len,
+                               nvec, right_side, lower, inv, Bp, ldb);
+        gbx_count_launch(ctx, 1);
+        return gbx_check_launch(ctx, nm);
+    }
+
     gbx_status copy_back(T *dst, long long ldd, const T *src, long long lds, int rows, int cols)
     {
         cudaError_t e = cudaMemcpy2DAsync(dst, sizeof(T) * ldd, src, sizeof(T) * lds, sizeof(T) * rows, cols,
@@ -134,6 +229,7 @@ struct Trsm {
         gbx_status st;
         if (len <= NB) {
             const T *inv = Inv + (long long)(r0 / NB) * NB * NB;
+            if constexpr (std::is_same<T, double>::value) return leaf(0, len, n, inv, B + r0);
             if ((st = gemm(len, n, len, one(), inv, NB, 0, 0, B + r0, ldb, 0, 0, T{}, Tw, NB)) != GBX_OK) return st;
             return copy_back(B + r0, ldb, Tw, NB, len, n);
         }
@@ -160,6 +256,7 @@ struct Trsm {
         gbx_status st;
         if (len <= NB) {
             const T *inv = Inv + (long long)(c0 / NB) * NB * NB;
+            if constexpr (std::is_same<T, double>::value) return leaf(1, len, m, inv, B + (long long)c0 * ldb);
             if ((st = gemm(m, len, len, one(), B + (long long)c0 * ldb, ldb, 0, 0, inv, NB, 0, 0, T{}, Tw, m)) !=
                 GBX_OK)
                 return st;
@@ -206,17 +303,23 @@ gbx_status trsm_t(gbx_ctx *ctx, const char *nm, char side, char uplo, char ta, c
     t.lower = (tri & TRI_LOWER) != 0;
     t.B = B; t.ldb = ldb;
     const int nblk = (t.na + NB - 1) / NB;
-    T *inv, *tmp;
+    T *inv, *tmp = nullptr;
     if ((st = gbx_ws(ctx, GBX_WS_TMP1, sizeof(T) * (size_t)nblk * NB * NB, (void **)&inv)) != GBX_OK) return st;
-    if ((st = gbx_ws(ctx, GBX_WS_TMP2, sizeof(T) * (size_t)NB * (lside ? n : m), (void **)&tmp)) != GBX_OK)
+    if (!std::is_same<T, double>::value &&
+        (st = gbx_ws(ctx, GBX_WS_TMP2, sizeof(T) * (size_t)NB * (lside ? n : m), (void **)&tmp)) != GBX_OK)
         return st;
     t.Inv = inv;
     t.Tw = tmp;
 
-    const size_t smem = sizeof(T) * (NB * (NB + 1) + NB * NB);
     // a per-device function attribute; setting it is a cheap host call
-    cudaFuncSetAttribute(trinv_blocks<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    trinv_blocks<T><<<nblk, NB, smem, S(ctx)>>>(t.na, A, lda, t.tr, t.cj, t.lower, (tri & TRI_UNIT) != 0, inv);
+    if constexpr (std::is_same<T, double>::value) {
+        cudaFuncSetAttribute(trinv64_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TRINV64_SMEM);
+        trinv64_blocks<<<nblk, 256, TRINV64_SMEM, S(ctx)>>>(t.na, A, lda, t.tr, t.lower, (tri & TRI_UNIT) != 0, inv);
+    } else {
+        const size_t smem = sizeof(T) * (NB * (NB + 1) + NB * NB);
+        cudaFuncSetAttribute(trinv_blocks<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        trinv_blocks<T><<<nblk, NB, smem, S(ctx)>>>(t.na, A, lda, t.tr, t.cj, t.lower, (tri & TRI_UNIT) != 0, inv);
+    }
     gbx_count_launch(ctx, 1);
     if ((st = gbx_check_launch(ctx, nm)) != GBX_OK) return st;
     return lside ? t.left(0, m) : t.right(0, n);
