@@ -202,10 +202,15 @@ symv_finish(int n, int nb, const double *__restrict__ part, double alpha, double
 }
 
 // ------------------------------------------------------------------ DTRSV
-constexpr int TV_NB = gbx_tri::NB, TV_LD = gbx_tri::LD, TV_THREADS = 256, TV_STAGES = 3;
+constexpr int TV_NB = gbx_tri::NB, TV_LD = gbx_tri::LD, TV_THREADS = 256;
 constexpr int TV_TILE = TV_NB * TV_LD;
-constexpr size_t TV_SMEM = sizeof(double) * ((TV_STAGES + 1) * TV_TILE + 4 * TV_NB + TV_NB + 8 * 16);
-constexpr int TV_FOLD = 24;
+constexpr int TV_R = 16, TV_SL = TV_NB / TV_R, TV_RLD = TV_R + 1;   // rows and number of a block's slices
+constexpr int TV_STAGES = 8, TV_WT = 8 * TV_RLD;   // a warp's ring: 16 rows x 8 columns per stage
+constexpr int TV_RED = TV_R * 18;
+constexpr int TV_W1 = 3 * TV_NB * TV_RLD + 8 * TV_STAGES * TV_WT + 2 * TV_RED;   // for a slice
+constexpr int TV_W2 = 2 * TV_TILE + 32 * 33;                                    // to invert a block
+constexpr size_t TV_SMEM = sizeof(double) * (TV_TILE + (TV_W1 > TV_W2 ? TV_W1 : TV_W2));
+constexpr int TV_FOLD = 8;
 constexpr unsigned long long TV_TIMEOUT_NS = 2000000000ull;
 constexpr int TV_TIMEOUT_CODE = 9;
 
@@ -215,6 +220,9 @@ struct TrsvArgs {
     long long lda;
     double *x;          // element 0 of the vector
     double *xw;         // solution in solve order, nblk * 64 values, all bits set until known
+    double *zw;         // b - (the blocks subtracted one by one), likewise
+    double *inv;        // inverted diagonal blocks, element (i, k) at [64 k + i]
+    int *ready;         // per block: all bits set until its inverse is there
     int *status, *status_host;
 };
 
@@ -260,145 +268,282 @@ __device__ __forceinline__ void tv_fetch(const TrsvArgs &a, double *dst, int s, 
     }
 }
 
-// This warp's 16 values of solution block K (columns 16 q .. of it): lanes
-// 0-15 hold them in v once known.  The values themselves are the flags: a
-// block's owner stores them over the "all bits set" pattern.  A wait that
-// lasts 2 s gives up: the status word is set and the values become NaN, so
-// that every later block still finishes.
-__device__ __forceinline__ double tv_load(const double *p, int lane)
+// Row of its block that is row r of slice sl: eight from the block's upper half
+// and eight from the lower, so that the triangular work of the slices is equal.
+__device__ __forceinline__ int tv_row(int sl, int r) { return r < 8 ? 8 * sl + r : 48 - 8 * sl + r; }
+
+// A lane's share of the copy of a slice's 16 x 8 parts, columns c0 + 64 K .. of
+// block row s, to dst[k * 17 + i]: four elements whose addresses differ by
+// off[], 64 columns further per block.
+struct TvPart {
+    const double *src, *any;
+    long long off[3], kstep;
+    int dst, dstep, ok;
+
+    __device__ __forceinline__ TvPart(const TrsvArgs &a, int s, int sl, int c0, int lane)
+    {
+        const int k0 = a.tr ? lane & 7 : lane >> 4, i0 = a.tr ? lane >> 3 : lane & 15;
+        const long long col = a.fwd ? a.lda : -a.lda;   // one column (N) or row (T) on
+        any = a.A;
+        ok = 0;
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (s * TV_NB + tv_row(sl, i0 + (a.tr ? 4 * u : 0)) < a.n) ok |= 1 << u;
+        // (a lane whose first row is beyond n reads nothing)
+        src = tv_at(a, min(s * TV_NB + tv_row(sl, i0), a.n - 1), c0 + k0);
+#pragma unroll
+        for (int u = 1; u < 4; u++)
+            off[u - 1] = col * (a.tr ? tv_row(sl, i0 + 4 * u) - tv_row(sl, i0) : 2 * u);
+        kstep = TV_NB * (a.tr ? (a.fwd ? 1 : -1) : col);
+        dst = k0 * TV_RLD + i0;
+        dstep = a.tr ? 4 : 2 * TV_RLD;
+    }
+    // the next block's part
+    __device__ __forceinline__ void fetch(double *ring)
+    {
+        double *d = ring + dst;
+        tv_copy8(d, ok & 1 ? src : any, ok & 1);
+#pragma unroll
+        for (int u = 1; u < 4; u++) tv_copy8(d + u * dstep, ok >> u & 1 ? src + off[u - 1] : any, ok >> u & 1);
+        src += kstep;
+    }
+};
+
+// Values that other CTAs publish are their own flags: a value is stored over
+// the "all bits set" pattern.  Waits until the lanes of `mask` hold theirs
+// (v: loaded before, p: this lane's address).  A wait that lasts 2 s gives
+// up: the status word is set and the values become NaN, so that every later
+// block still finishes.
+__device__ __forceinline__ double tv_load(const double *p) { return *(const volatile double *)p; }
+__device__ __forceinline__ void tv_timeout(const TrsvArgs &a)
 {
-    return lane < 16 ? *(const volatile double *)(p + lane) : 0.0;
+    atomicCAS(a.status, 0, TV_TIMEOUT_CODE);
+    *(volatile int *)a.status_host = TV_TIMEOUT_CODE;
+    __threadfence_system();
 }
-__device__ __forceinline__ double tv_wait(const TrsvArgs &a, const double *p, double v, int lane)
+__device__ __forceinline__ double tv_wait(const TrsvArgs &a, const double *p, double v, unsigned mask, int lane)
 {
-    if (__all_sync(0xffffffffu, __double_as_longlong(v) != -1ll)) return v;
+    const bool mine = mask >> lane & 1;
+    if (!__any_sync(0xffffffffu, mine && __double_as_longlong(v) == -1ll)) return v;
     const unsigned long long t0 = tv_now();
     while (true) {
-        if (__double_as_longlong(v) == -1ll) v = tv_load(p, lane);
-        if (__all_sync(0xffffffffu, __double_as_longlong(v) != -1ll)) return v;
+        if (mine && __double_as_longlong(v) == -1ll) v = tv_load(p);
+        if (!__any_sync(0xffffffffu, mine && __double_as_longlong(v) == -1ll)) return v;
         if (__any_sync(0xffffffffu, tv_now() - t0 > TV_TIMEOUT_NS)) {
-            if (lane == 0) {
-                atomicCAS(a.status, 0, TV_TIMEOUT_CODE);
-                *(volatile int *)a.status_host = TV_TIMEOUT_CODE;
-                __threadfence_system();
-            }
+            if (lane == 0) tv_timeout(a);
             return __longlong_as_double(0x7ff8000000000000ll);
         }
     }
 }
+__device__ __forceinline__ void tv_publish(double *p, double r)
+{
+    // the "not yet known" pattern is a NaN: another NaN in its place
+    *(volatile double *)p = __double_as_longlong(r) == -1ll ? __longlong_as_double(0x7ff8000000000000ll) : r;
+}
 
-// x := T^-1 x, blocks of 64 rows in solve order; CTA b owns blocks b,
-// b + gridDim.x, ...  All CTAs are resident (cooperative launch), and a block
-// waits only for earlier ones.  For its block s a CTA
-//   * inverts the diagonal block (while it waits anyway, except the first);
-//   * subtracts T(s, K) x_K for every earlier block K as x_K appears, the
-//     64 x 64 blocks of T prefetched three deep into shared memory (they do
-//     not depend on x), 16 of the products per thread and block;
-//   * x_s = inv (b - sum) goes to the later blocks through xw and to x.
+// Waits for the inverse of block s and starts the copy of the slice's rows of
+// it to dst[k * 17 + i]; by the whole CTA.
+__device__ __forceinline__ void tv_fetch_inv(const TrsvArgs &a, double *dst, int s, int sl)
+{
+    const int tid = threadIdx.x;
+    if (tid == 0) {
+        const unsigned long long t0 = tv_now();
+        while (*(volatile int *)(a.ready + s) != 0)
+            if (tv_now() - t0 > TV_TIMEOUT_NS) {
+                tv_timeout(a);
+                break;
+            }
+        __threadfence();
+    }
+    __syncthreads();
+    const double *src = a.inv + (size_t)s * TV_NB * TV_NB + tv_row(sl, tid & 15);
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const int k = (tid >> 4) + 16 * u;
+        tv_copy8(dst + k * TV_RLD + (tid & 15), src + k * TV_NB, 1);
+    }
+}
+
+// Sum over the CTA of the 16 values that its threads (row lane & 15, columns
+// 4 (2 warp + lane / 16) ..) have for each row: in warps 0-3, lanes 4 r' + ..:
+// row 4 warp + (lane & 3).
+__device__ __forceinline__ double tv_sum(double *red, double v, int lane, int warp)
+{
+    red[(2 * warp + (lane >> 4)) * 18 + (lane & 15)] = v;
+    __syncthreads();
+    double r = 0.0;
+    if (warp < 4) {
+        const double *q = red + 2 * (lane >> 2) * 18 + 4 * warp + (lane & 3);
+        r = q[0] + q[18];
+        r += __shfl_xor_sync(0xffffffffu, r, 4);
+        r += __shfl_xor_sync(0xffffffffu, r, 8);
+        r += __shfl_xor_sync(0xffffffffu, r, 16);
+    }
+    return r;
+}
+
+// x := T^-1 x, blocks of 64 rows in solve order, each in four slices of 16
+// rows (tv_row); CTA b owns slices b, b + gridDim.x, ...  All CTAs are resident
+// (cooperative launch).  A slice waits for earlier blocks and for sums of its
+// own block's slices, which wait for earlier blocks only.
+//   * The CTAs invert the diagonal blocks first, CTA b block b (again before
+//     every fourth slice, for as many blocks as the next four rounds reach).
+//   * A slice subtracts T(s, K) x_K for every earlier block K as x_K appears:
+//     warp w columns 8 w .. 8 w + 7 of each, prefetched seven blocks deep into
+//     its own ring (they do not depend on x), without barriers.
+//   * The four slices exchange z = b - sum through zw; x_s = inv z goes to the
+//     later blocks through xw and to x.
+//   * From block TV_FOLD on M = inv T(s, s-1) is formed beforehand, so that
+//     x_s = inv (b - sum over K < s-1) - M x_(s-1): the exchange and the
+//     inverse lie before x_(s-1), which needs one product.
 // What bounds it: the chain over the blocks, each link one hand-over through
-// L2 (about 1 us) and the products between x_(s-1) and x_s, 1 us per 64 x 64
-// on the SM's two FP64 lanes.  From the 24th block on there is time to form
-// M = inv T(s, s-1) beforehand, so that x_s = inv (b - sum over K < s-1) -
-// M x_(s-1) needs one product after x_(s-1) instead of two (M costs 47 us,
-// by which the chain has come to that block).  64 rows per block: half of it
-// would double the hand-overs, double of it the products per link.
-// n = 8192: 300 us for N or T; one launch per 64 rows, each forming
-// x_s in every CTA, took 4.1 ms.
+// L2 and the product with x_(s-1), 1.2 us; for the last blocks the FP64 pipe,
+// which takes 0.33 us for each 16 x 64 part and 11 us for M.  (With a block per
+// CTA, 1.3 us of the pipe for each 64 x 64 part, a link took 2.3 us; two CTAs
+// per SM fill the pipe but share it with the link: n = 8192 6 % slower, 16000
+// 10 % faster.)  n = 8192: N or T 300 us with a block per CTA, now 214.  M for
+// every block from the 8th on: from the 12th n = 2000 is 3 us slower, from the
+// 6th all sizes the same.
 __global__ void __launch_bounds__(TV_THREADS)
 trsv_solve(TrsvArgs a)
 {
     extern __shared__ __align__(16) double tv_sm[];
-    double *stage = tv_sm;                          // TV_STAGES blocks
-    double *X = stage + TV_STAGES * TV_TILE;        // inverse of the diagonal block
-    double *red = X + TV_TILE;                      // [4][64]
-    double *st = red + 4 * TV_NB;                   // [64]
+    double *T1 = tv_sm;                              // T(s, s-1)
+    double *work = T1 + TV_TILE;                     // to invert a block
+    double *Ia = work;                               // the slice's rows of the inverse, [k * 17 + i]: two
+    double *Ms = Ia + 2 * TV_NB * TV_RLD;            // of M, likewise
+    double *ring = Ms + TV_NB * TV_RLD;
+    double *red = ring + 8 * TV_STAGES * TV_WT;      // two sums
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int i = tid & 63, q = tid >> 6;           // row, quarter of the columns
-    double *xs = st + TV_NB + 16 * warp;            // this warp's 16 solution values
+    const int i = lane & 15, h4 = 4 * (lane >> 4);   // row; columns 8 warp + h4 .. + 3
+    ring += warp * TV_STAGES * TV_WT;
+    const int r16 = (4 * warp + (lane & 3)) & 15;    // row of the sums, warps 0-3
+    const bool out = warp < 4 && lane < 4;
 
-    for (int s = blockIdx.x; s < a.nblk; s += gridDim.x) {
-        const int p = s * TV_NB + i;
-        // diagonal block into stage 0 (identity beyond n)
-        for (int t = tid; t < TV_NB * TV_NB; t += TV_THREADS) {
-            const int u = t & 63, v = t >> 6;
-            const int r = a.tr ? v : u, k = a.tr ? u : v;
-            const int pr = s * TV_NB + r, pk = s * TV_NB + k;
-            double d = r == k ? 1.0 : 0.0;
-            if (k <= r && pr < a.n && !(a.unit && r == k)) d = *tv_at(a, pr, pk);
-            stage[k * TV_LD + r] = d;
-        }
-        const bool fold = s >= TV_FOLD;
-        if (fold) tv_fetch(a, stage + TV_TILE, s, s - 1);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        const double b = p < a.n ? a.x[(long long)(a.fwd ? p : a.n - 1 - p) * a.incx] : 0.0;
-        __syncthreads();
-        gbx_tri::invert64(stage, X, stage + 2 * TV_TILE);
-        double M[16];
-        if (fold) {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-            __syncthreads();
-            // M(i, 16 q ..): row i of the inverse reaches column i at most
-            const double *T1 = stage + TV_TILE + 16 * q * TV_LD;
+    int round = 0;
+    for (int t = blockIdx.x; t < TV_SL * a.nblk; t += gridDim.x, round++) {
+        const int ib = blockIdx.x + round / TV_SL * gridDim.x;
+        if (round % TV_SL == 0 && ib < a.nblk) {
+            double *D = work, *X = D + TV_TILE;
 #pragma unroll
-            for (int k = 0; k < 16; k++) M[k] = 0.0;
-            const int jend = (warp & 1) ? 64 : 32;
-            for (int j = 0; j < jend; j++) {
-                const double v = X[j * TV_LD + i];
-#pragma unroll
-                for (int k = 0; k < 16; k++) M[k] = fma(v, T1[k * TV_LD + j], M[k]);
+            for (int f = 0; f < TV_NB * TV_NB / TV_THREADS; f++) {   // identity beyond n
+                const int e = tid + f * TV_THREADS, u = e & 63, v = e >> 6;
+                const int r = a.tr ? v : u, k = a.tr ? u : v;
+                const int pr = ib * TV_NB + r, pk = ib * TV_NB + k;
+                const int in = k <= r && pr < a.n && !(a.unit && r == k);
+                if (in) tv_copy8(D + k * TV_LD + r, tv_at(a, pr, pk), 1);
+                else D[k * TV_LD + r] = r == k ? 1.0 : 0.0;
             }
+            asm volatile("cp.async.wait_all;" ::: "memory");
             __syncthreads();
+            gbx_tri::invert64(D, X, X + TV_TILE);
+            double *o = a.inv + (size_t)ib * TV_NB * TV_NB;
+            for (int e = tid; e < TV_NB * TV_NB; e += TV_THREADS) o[e] = X[(e >> 6) * TV_LD + (e & 63)];
+            __threadfence();
+            __syncthreads();
+            if (tid == 0) *(volatile int *)(a.ready + ib) = 0;
         }
-        const int nk = fold ? s - 1 : s;   // blocks subtracted one by one
-#pragma unroll
+        const int s = t / TV_SL, sl = t % TV_SL;
+        const int row = s * TV_NB + tv_row(sl, r16);
+        const bool fold = s >= TV_FOLD;
+        double *I = Ia + (round & 1) * TV_NB * TV_RLD;
+        if (fold && round == 0) tv_fetch(a, T1, s, s - 1);
+        if (round % TV_SL == 0) tv_fetch_inv(a, I, s, sl);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const int nk = fold ? s - 1 : s;                 // blocks subtracted one by one
+        TvPart part(a, s, sl, 8 * warp, lane);
+#pragma unroll 1
         for (int f = 0; f < TV_STAGES - 1; f++) {
-            if (f < nk) tv_fetch(a, stage + f * TV_TILE, s, f);
+            if (f < nk) part.fetch(ring + f * TV_WT);
             asm volatile("cp.async.commit_group;" ::: "memory");
         }
-        double acc = 0.0, xv = 0.0;
-        if (s > 0) xv = tv_load(a.xw + 16 * q, lane);
+        double b = 0.0;
+        const long long xi = (long long)(a.fwd ? row : a.n - 1 - row) * a.incx;
+        if (out && row < a.n) b = a.x[xi];
+        asm volatile("cp.async.wait_group %0;" ::"n"(TV_STAGES - 1) : "memory");   // T1, I
+        __syncthreads();
+        double M[4];
+        if (fold) {
+            // warps 0-3 have the slice's upper eight rows, 4-7 the lower: the
+            // inverse is lower triangular.  Thread: one row, four columns.
+            const int m8 = (lane & 7) + 8 * (warp >> 2), c4 = 16 * (warp & 3) + 4 * (lane >> 3);
+            const int jend = 8 * (warp < 4 ? sl + 1 : 8 - sl);
+            const double *c = T1 + c4 * TV_LD;
+#pragma unroll
+            for (int k = 0; k < 4; k++) M[k] = 0.0;
+            for (int j = 0; j < jend; j++) {
+                const double v = I[j * TV_RLD + m8];
+#pragma unroll
+                for (int k = 0; k < 4; k++) M[k] = fma(v, c[k * TV_LD + j], M[k]);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) Ms[(c4 + k) * TV_RLD + m8] = M[k];
+        }
+        __syncthreads();
+        if (fold) {
+#pragma unroll
+            for (int k = 0; k < 4; k++) M[k] = -Ms[(8 * warp + h4 + k) * TV_RLD + i];
+        }
+        const int sn = (t + gridDim.x) / TV_SL;          // the next slice's
+        if (sn < a.nblk && sn >= TV_FOLD) tv_fetch(a, T1, sn, sn - 1);
+        if (sn < a.nblk && (round + 1) % TV_SL != 0)
+            tv_fetch_inv(a, Ia + ((round + 1) & 1) * TV_NB * TV_RLD, sn, sl);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        // x of four blocks at a time: lane 8 u + c has column 8 warp + c of block 4 g + u
+        const double *xp = a.xw + (lane >> 3) * TV_NB + 8 * warp + (lane & 7);
+        double acc0 = 0.0, acc1 = 0.0, xv = 0.0, xn = 0.0;
+        if ((lane >> 3) < s) xn = tv_load(xp);
+        auto x_of = [&](int K) {   // this warp's eight values of x_K are in lanes 8 (K & 3) ..
+            if ((K & 3) == 0) {
+                xv = xn;
+                if (K + 4 + (lane >> 3) < s) xn = tv_load(xp + (long long)(K + 4) * TV_NB);
+            }
+            xv = tv_wait(a, xp + (long long)(K & ~3) * TV_NB, xv, 0xffu << 8 * (K & 3), lane);
+        };
         for (int K = 0; K < nk; K++) {
-            asm volatile("cp.async.wait_group %0;" :: "n"(TV_STAGES - 2) : "memory");
-            __syncthreads();   // block K is in, block K - 1 consumed
-            if (K + TV_STAGES - 1 < nk)
-                tv_fetch(a, stage + ((K + TV_STAGES - 1) % TV_STAGES) * TV_TILE, s, K + TV_STAGES - 1);
+            if (K + TV_STAGES - 1 < nk) part.fetch(ring + (K + TV_STAGES - 1) % TV_STAGES * TV_WT);
             asm volatile("cp.async.commit_group;" ::: "memory");
-            xv = tv_wait(a, a.xw + (long long)K * TV_NB + 16 * q, xv, lane);
+            x_of(K);
+            asm volatile("cp.async.wait_group %0;" ::"n"(TV_STAGES - 1) : "memory");
             __syncwarp();
-            if (lane < 16) xs[lane] = xv;
-            __syncwarp();
-            if (K + 1 < s) xv = tv_load(a.xw + (long long)(K + 1) * TV_NB + 16 * q, lane);
-            const double *T = stage + (K % TV_STAGES) * TV_TILE + 16 * q * TV_LD + i;
-#pragma unroll
-            for (int k = 0; k < 16; k++) acc = fma(T[k * TV_LD], xs[k], acc);
+            const double *T = ring + K % TV_STAGES * TV_WT + h4 * TV_RLD + i;
+            const int l = 8 * (K & 3) + h4;
+            acc0 = fma(T[0], __shfl_sync(0xffffffffu, xv, l), acc0);
+            acc1 = fma(T[TV_RLD], __shfl_sync(0xffffffffu, xv, l + 1), acc1);
+            acc0 = fma(T[2 * TV_RLD], __shfl_sync(0xffffffffu, xv, l + 2), acc0);
+            acc1 = fma(T[3 * TV_RLD], __shfl_sync(0xffffffffu, xv, l + 3), acc1);
+            __syncwarp();   // the stage may be overwritten
         }
-        red[q * TV_NB + i] = acc;
-        __syncthreads();
-        if (tid < TV_NB) st[i] = b - ((red[i] + red[TV_NB + i]) + (red[2 * TV_NB + i] + red[3 * TV_NB + i]));
-        __syncthreads();
-        double v = 0.0;
-        if ((warp & 1) || q < 2) {   // rows < 32 end at column 31
-#pragma unroll
-            for (int k = 0; k < 16; k++) v = fma(X[(16 * q + k) * TV_LD + i], st[16 * q + k], v);
+        const double sum = tv_sum(red, acc0 + acc1, lane, warp);
+        if (out) tv_publish(a.zw + row, b - sum);
+        double v0 = 0.0, v1 = 0.0;
+        if (warp < 8 - sl) {   // the rows end at column 63 - 8 sl
+            const double *zp = a.zw + (long long)s * TV_NB + 8 * warp + (lane & 7);
+            const double z = tv_wait(a, zp, tv_load(zp), 0xffffffffu, lane);
+            const double *c = I + (8 * warp + h4) * TV_RLD + i;
+            v0 = fma(c[0], __shfl_sync(0xffffffffu, z, h4), v0);
+            v1 = fma(c[TV_RLD], __shfl_sync(0xffffffffu, z, h4 + 1), v1);
+            v0 = fma(c[2 * TV_RLD], __shfl_sync(0xffffffffu, z, h4 + 2), v0);
+            v1 = fma(c[3 * TV_RLD], __shfl_sync(0xffffffffu, z, h4 + 3), v1);
+            v0 += v1;
+            v1 = 0.0;
         }
         if (fold) {
-            xv = tv_wait(a, a.xw + (long long)(s - 1) * TV_NB + 16 * q, xv, lane);
-            __syncwarp();
-            if (lane < 16) xs[lane] = xv;
-            __syncwarp();
-#pragma unroll
-            for (int k = 0; k < 16; k++) v = fma(-M[k], xs[k], v);
+            x_of(s - 1);
+            const int l = 8 * ((s - 1) & 3) + h4;
+            v0 = fma(M[0], __shfl_sync(0xffffffffu, xv, l), v0);
+            v1 = M[1] * __shfl_sync(0xffffffffu, xv, l + 1);
+            v0 = fma(M[2], __shfl_sync(0xffffffffu, xv, l + 2), v0);
+            v1 = fma(M[3], __shfl_sync(0xffffffffu, xv, l + 3), v1);
+            v0 += v1;
         }
-        red[q * TV_NB + i] = v;
-        __syncthreads();
-        if (tid < TV_NB) {
-            const double r = (red[i] + red[TV_NB + i]) + (red[2 * TV_NB + i] + red[3 * TV_NB + i]);
-            // the "not yet known" pattern is a NaN: publish another NaN in its place
-            const double o = __double_as_longlong(r) == -1ll ? __longlong_as_double(0x7ff8000000000000ll) : r;
-            *(volatile double *)(a.xw + p) = o;
-            if (p < a.n) a.x[(long long)(a.fwd ? p : a.n - 1 - p) * a.incx] = r;
+        const double r = tv_sum(red + TV_RED, v0, lane, warp);
+        if (out) {
+            tv_publish(a.xw + row, r);
+            if (row < a.n) a.x[xi] = r;
         }
-        __syncthreads();   // shared memory is reused by the next block
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();   // shared memory is reused by the next slice
     }
 }
 
@@ -495,7 +640,11 @@ extern "C" gbx_status gbx_dtrsv(gbx_ctx *ctx, char uplo, char trans, char diag, 
     double *xw;
     TrsvArgs p{};
     gbx_status st;
-    if ((st = gbx_ws(ctx, GBX_WS_TMP2, sizeof(double) * (size_t)nblk * TV_NB, (void **)&xw)) != GBX_OK) return st;
+    // x and z in solve order and the blocks' ready words (eight bytes each)
+    const size_t wbytes = sizeof(double) * (size_t)nblk * (2 * TV_NB + 1);
+    if ((st = gbx_ws(ctx, GBX_WS_TMP1, sizeof(double) * (size_t)nblk * TV_NB * TV_NB, (void **)&p.inv)) != GBX_OK)
+        return st;
+    if ((st = gbx_ws(ctx, GBX_WS_TMP2, wbytes, (void **)&xw)) != GBX_OK) return st;
     if ((st = gbx_ctx_status(ctx, &p.status, &p.status_host)) != GBX_OK) return st;
     p.n = n;
     p.nblk = nblk;
@@ -507,13 +656,16 @@ extern "C" gbx_status gbx_dtrsv(gbx_ctx *ctx, char uplo, char trans, char diag, 
     p.x = x + base_off(n, incx);
     p.incx = incx;
     p.xw = xw;
+    p.zw = xw + (size_t)nblk * TV_NB;
+    p.ready = (int *)(p.zw + (size_t)nblk * TV_NB);
     // every value "not yet known" (all bits set)
-    cudaError_t e = cudaMemsetAsync(xw, 0xFF, sizeof(double) * (size_t)nblk * TV_NB, S(ctx));
+    cudaError_t e = cudaMemsetAsync(xw, 0xFF, wbytes, S(ctx));
     // a per-device function attribute; setting it is a cheap host call
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(trsv_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TV_SMEM);
     if (e != cudaSuccess) return gbx_fail(ctx, GBX_ERR_CUDA, "dtrsv: %s", cudaGetErrorString(e));
-    const int grid = std::min(nblk, gbx_ctx_sms(ctx));   // one CTA per SM is always resident
+    // one CTA per SM is always resident; whole blocks, so that a block's slices run side by side
+    const int grid = TV_SL * std::min(nblk, std::max(1, gbx_ctx_sms(ctx) / TV_SL));
     void *args[] = {&p};
     gbx_timer_begin(ctx, GBX_TIMER_GEMV);
     e = cudaLaunchCooperativeKernel((const void *)trsv_solve, dim3(grid), dim3(TV_THREADS), args, TV_SMEM, S(ctx));

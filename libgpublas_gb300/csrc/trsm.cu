@@ -86,7 +86,7 @@ trinv_blocks(int na, const T *__restrict__ A, long long lda, int tr, int cj, int
 
 // The same for double, by 256 threads per block (gbx_tri::invert64): a thread
 // per column stepping through 64 rows took 165 us (a warp has one FP64
-// instruction in flight, 65 cycles each), now 29.  An upper triangle is inverted
+// instruction in flight, 65 cycles each), now 22.  An upper triangle is inverted
 // as the lower one it becomes when rows and columns are reversed.
 constexpr size_t TRINV64_SMEM = sizeof(double) * (2 * gbx_tri::NB * gbx_tri::LD + 32 * 33);
 __global__ void __launch_bounds__(256)
@@ -97,8 +97,9 @@ trinv64_blocks(int na, const double *__restrict__ A, long long lda, int tr, int 
     double *D = (double *)sm_raw, *X = D + NB * gbx_tri::LD, *W = X + NB * gbx_tri::LD;
     const int r0 = blockIdx.x * NB, nbb = min(NB, na - r0);
     // position p of the reversed block is row (column) NB - 1 - p; identity beyond na
-    for (int t = threadIdx.x; t < NB * NB; t += blockDim.x) {
-        const int u = t & 63, v = t >> 6;
+#pragma unroll
+    for (int f = 0; f < NB * NB / 256; f++) {
+        const int t = threadIdx.x + f * 256, u = t & 63, v = t >> 6;
         const int r = tr ? v : u, c = tr ? u : v;   // row, column of op(A)'s block
         double d = r == c ? 1.0 : 0.0;
         if (r < nbb && c < nbb && (lower ? c <= r : c >= r) && !(unit && r == c))
