@@ -13,7 +13,7 @@
 //     FMAs per 8 bytes: on GB300's FP64 pipe (2 lanes per clock per SM) that
 //     is the bound, not HBM.  Per-tile partial vectors are summed in a fixed
 //     order by a second kernel (deterministic).
-//   * DTRSV: one cooperative launch in which every CTA owns a 64-row block
+//   * DTRSV: one cooperative launch in which every CTA owns 16 rows of a block
 //     and passes its part of the solution to the later blocks through global
 //     memory as soon as it is known (see trsv_solve).
 #include "gbx_internal.h"

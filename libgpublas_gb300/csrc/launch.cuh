@@ -21,11 +21,10 @@ __device__ __forceinline__ void pdl_enter()
 }
 
 // Hand-over between the warps of a CTA on named barrier id (1-15) of `threads`
-// threads: the producing warp arrives without waiting, the others wait.
+// threads: the producing warp arrives without waiting, the others wait and then
+// see what it stored.
 __device__ __forceinline__ void bar_arrive(int id, int threads)
 {
-    __threadfence_block();
-    __syncwarp();
     asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 __device__ __forceinline__ void bar_wait(int id, int threads)
