@@ -84,7 +84,9 @@ __device__ __forceinline__ bool last_block(unsigned *counter)
     return s_last != 0u;
 }
 
-__device__ __forceinline__ double2 ldg2(const double2 *p) { return __ldg(p); }
+// A plain load: the vectors may be results of the call before, which still runs
+// when the CTA is placed, so loads through the non-coherent path are not for them.
+__device__ __forceinline__ double2 ldg2(const double2 *p) { return *p; }
 
 static __global__ void zero_result(double *res) { *res = 0.0; }
 static __global__ void zero_index(int *res) { *res = 0; }
@@ -94,7 +96,7 @@ static __global__ void zero_index(int *res) { *res = 0; }
 // double2 (128-bit) accesses after peeling one leading element; otherwise it
 // falls back to 64-bit accesses.
 static __global__ void __launch_bounds__(L1_THREADS)
-axpy_unit(int n, double a, const double *__restrict__ x, double *__restrict__ y)
+axpy_unit(int n, double a, const double *x, double *__restrict__ y)
 {
     gbx_launch::pdl_enter();
     const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -121,13 +123,13 @@ axpy_unit(int n, double a, const double *__restrict__ x, double *__restrict__ y)
         }
         if (((n - peel) & 1) && tid == 0) y[n - 1] = fma(a, x[n - 1], y[n - 1]);
     } else {
-        for (long long i = tid; i < n; i += stride) y[i] = fma(a, __ldg(x + i), y[i]);
+        for (long long i = tid; i < n; i += stride) y[i] = fma(a, x[i], y[i]);
     }
 }
 
 // Any increments; x and y point at element 0 of the logical vectors.
 static __global__ void __launch_bounds__(L1_THREADS)
-axpy_strided(int n, double a, const double *__restrict__ x, int incx, double *__restrict__ y, int incy)
+axpy_strided(int n, double a, const double *x, int incx, double *__restrict__ y, int incy)
 {
     gbx_launch::pdl_enter();
     const long long stride = (long long)gridDim.x * blockDim.x;
@@ -148,7 +150,7 @@ scal_kernel(int n, double a, double *__restrict__ x, int incx)
 
 // ----------------------------------------------------------------- ddot ---
 static __global__ void __launch_bounds__(L1_THREADS)
-dot_kernel(int n, const double *__restrict__ x, int incx, const double *__restrict__ y, int incy,
+dot_kernel(int n, const double *x, int incx, const double *y, int incy,
            double *__restrict__ part, unsigned *counter, double *__restrict__ res)
 {
     gbx_launch::pdl_enter();
@@ -341,7 +343,7 @@ __device__ __forceinline__ double blue_finish(double asml, double amed, double a
 }
 
 static __global__ void __launch_bounds__(L1_THREADS)
-nrm2_kernel(int n, const double *__restrict__ x, int incx, double *__restrict__ part, unsigned *counter,
+nrm2_kernel(int n, const double *x, int incx, double *__restrict__ part, unsigned *counter,
             double *__restrict__ res)
 {
     gbx_launch::pdl_enter();
@@ -453,7 +455,7 @@ __device__ __forceinline__ void block_best(unsigned long long &k, long long &i)
 
 template <bool IS_MIN>
 static __global__ void __launch_bounds__(L1_THREADS)
-iamax_kernel(int n, const double *__restrict__ x, int incx, unsigned long long *__restrict__ keys,
+iamax_kernel(int n, const double *x, int incx, unsigned long long *__restrict__ keys,
              long long *__restrict__ idx, unsigned *counter, int *__restrict__ res)
 {
     gbx_launch::pdl_enter();

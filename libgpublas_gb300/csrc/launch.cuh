@@ -2,7 +2,10 @@
 // (programmatic stream serialisation).  A kernel launched with launch_pdl may
 // have its CTAs placed on the SMs before the kernel ahead of it in the stream
 // has finished; every thread of it calls pdl_enter() before it touches memory,
-// which waits until that kernel is complete and its writes are visible.
+// which waits until that kernel is complete and its writes are visible.  What
+// that kernel may have written is read with plain loads, not through __ldg or a
+// const __restrict__ parameter: such loads assume that nothing writes the data
+// from the launch on.
 // Without it each of a program's short calls pays its launch, about 2 us, after
 // the call before has drained.
 #pragma once

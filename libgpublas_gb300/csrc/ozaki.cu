@@ -1790,7 +1790,7 @@ oz_gemm_sk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 #pragma unroll
             for (int j = 0; j < DCOLS; j++) {
                 cold[j] = (row_ok && as.beta_on && oz_c_keep(p, grow, gc0 + j)) ? cp[(size_t)j * p.ldc] : 0.0;
-                ecol[j] = __ldg(p.col_exp + gc0 + j);
+                ecol[j] = p.col_exp[gc0 + j];
             }
             const int erow = row_ok ? p.row_exp[grow] - 5 * (S - 1) : 0;
 
@@ -2775,7 +2775,7 @@ oz_trinv_diag(OzTriView L, int unit, double *__restrict__ D)
 }
 
 __global__ void __launch_bounds__(OZ_TI_NMAX)
-oz_trinv_kernel(OzTriView L, int trans, const double *__restrict__ D, double *__restrict__ X, long long ldx)
+oz_trinv_kernel(OzTriView L, int trans, const double *D, double *X, long long ldx)
 {
     gbx_launch::pdl_enter();
     __shared__ double st[2][OZ_TI_BLK], sx[2][OZ_TI_BLK];

@@ -221,7 +221,7 @@ potrf_step(int n, int j0, double *__restrict__ A, long long lda, int *__restrict
 // lower triangle per CTA, blockIdx.x enumerating the tiles (ti >= tj) row by
 // row; the two 16 x PB row blocks of A21 are staged in shared memory.
 __global__ void __launch_bounds__(256)
-potrf_syrk(int m, const double *__restrict__ A21, double *__restrict__ A22, long long lda)
+potrf_syrk(int m, const double *A21, double *A22, long long lda)
 {
     pdl_enter();
     __shared__ double Li[16][PB + 1], Lj[16][PB + 1];

@@ -125,8 +125,7 @@ trinv64_blocks(int na, const double *__restrict__ A, long long lda, int tr, int 
 // lost 4 us per leaf to a GEMM into scratch and a copy back instead.
 template <int TL_V>
 __global__ void __launch_bounds__(256)
-trsm_leaf(int len, int nvec, int right, int lower, const double *__restrict__ inv, double *__restrict__ B,
-          long long ldb)
+trsm_leaf(int len, int nvec, int right, int lower, const double *inv, double *B, long long ldb)
 {
     gbx_launch::pdl_enter();
     __shared__ double sI[NB][NB + 1];    // [k][i]: coefficient of input k in output i
