@@ -18,6 +18,7 @@
 //     memory as soon as it is known (see trsv_solve).
 #include "gbx_internal.h"
 #include "gemm_host.h"
+#include "launch.cuh"
 #include "tri_inverse.cuh"
 
 #include <cuda_runtime.h>
@@ -25,6 +26,8 @@
 #include <algorithm>
 
 namespace {
+
+using gbx_launch::launch_pdl_short;
 
 inline cudaStream_t S(gbx_ctx *ctx) { return (cudaStream_t)gbx_ctx_get_stream(ctx); }
 inline long long base_off(int n, int inc) { return inc >= 0 ? 0 : (long long)(n - 1) * (-inc); }
@@ -42,15 +45,16 @@ constexpr int GER_ROWS = 512, GER_COLS = 32;
 // vec: A is 16-byte aligned and lda even, so that a thread's two adjacent
 // rows are one 128-bit access in every column.
 __global__ void __launch_bounds__(256)
-ger_kernel(int m, int n, double alpha, const double *__restrict__ x, int incx, const double *__restrict__ y,
-           int incy, double *__restrict__ A, long long lda, int vec)
+ger_kernel(int m, int n, double alpha, const double *x, int incx, const double *y,
+           int incy, double *A, long long lda, int vec)
 {
+    gbx_launch::pdl_enter();
     __shared__ double coef[GER_COLS];
     __shared__ unsigned s_keep;
     const int c0 = blockIdx.y * GER_COLS, cols = min(GER_COLS, n - c0);
     const int tid = threadIdx.x;
     if (tid < 32) {
-        const double yj = tid < cols ? __ldg(y + (long long)(c0 + tid) * incy) : 0.0;
+        const double yj = tid < cols ? y[(long long)(c0 + tid) * incy] : 0.0;
         coef[tid] = alpha * yj;
         // y_j != 0 on the bit pattern (NaN counts as nonzero)
         const unsigned keep = __ballot_sync(0xffffffffu, (__double_as_longlong(yj) << 1) != 0);
@@ -63,8 +67,8 @@ ger_kernel(int m, int n, double alpha, const double *__restrict__ x, int incx, c
     const int r2 = vec ? r + 1 : r + 256;
     if (r >= m) return;
     double *ap = A + (long long)c0 * lda + r;
-    const double x0 = __ldg(x + (long long)r * incx);
-    const double x1 = r2 < m ? __ldg(x + (long long)r2 * incx) : 0.0;
+    const double x0 = x[(long long)r * incx];
+    const double x1 = r2 < m ? x[(long long)r2 * incx] : 0.0;
     if (keep == 0xffffffffu >> (GER_COLS - cols) && r2 < m) {   // no column is skipped
         if (vec) {
 #pragma unroll 1
@@ -120,9 +124,10 @@ constexpr int SY_T = 64;
 // to part[I][J] and, off the diagonal, the column partial (A_IJ^T x_I) to
 // part[J][I]; part[b][q] is the q-th partial of output block b.
 __global__ void __launch_bounds__(256)
-symv_tiles(int n, int nb, int lower, const double *__restrict__ A, long long lda, const double *__restrict__ x,
-           int incx, double *__restrict__ part)
+symv_tiles(int n, int nb, int lower, const double *A, long long lda, const double *x,
+           int incx, double *part)
 {
+    gbx_launch::pdl_enter();
     __shared__ double s[SY_T][SY_T + 1];
     __shared__ double sxI[SY_T], sxJ[SY_T];
     __shared__ double red[4][SY_T];
@@ -182,9 +187,10 @@ symv_tiles(int n, int nb, int lower, const double *__restrict__ A, long long lda
 // partials in order with eight loads in flight (one thread per row walking
 // all 128 partials of n = 8192 took 19.6 us, now 6.8 us).
 __global__ void __launch_bounds__(4 * SY_T)
-symv_finish(int n, int nb, const double *__restrict__ part, double alpha, double beta, double *__restrict__ y,
+symv_finish(int n, int nb, const double *part, double alpha, double beta, double *y,
             int incy)
 {
+    gbx_launch::pdl_enter();
     __shared__ double red[4][SY_T];
     const int b = blockIdx.x, l = threadIdx.x & (SY_T - 1), g = threadIdx.x / SY_T;
     const int q0 = (int)((long long)nb * g / 4), q1 = (int)((long long)nb * (g + 1) / 4);
@@ -593,8 +599,8 @@ extern "C" gbx_status gbx_dger(gbx_ctx *ctx, int m, int n, double alpha, const d
     if (g.y > 65535) return gbx_fail(ctx, GBX_ERR_UNSUPPORTED, "DGER: n too large");
     gbx_timer_begin(ctx, GBX_TIMER_GEMV);
     const int vec = (((uintptr_t)A) & 15) == 0 && lda % 2 == 0;
-    ger_kernel<<<g, 256, 0, S(ctx)>>>(m, n, alpha, x + base_off(m, incx), incx, y + base_off(n, incy), incy, A,
-                                      lda, vec);
+    launch_pdl_short(gbx_ctx_sms(ctx), ger_kernel, g, 256, S(ctx), m, n, alpha, x + base_off(m, incx), incx,
+                     y + base_off(n, incy), incy, A, lda, vec);
     gbx_timer_end(ctx);
     gbx_count_launch(ctx, 1);
     return gbx_check_launch(ctx, "dger");
@@ -617,13 +623,14 @@ extern "C" gbx_status gbx_dsymv(gbx_ctx *ctx, char uplo, int n, double alpha, co
     if (tiles > 0x7fffffffLL) return gbx_fail(ctx, GBX_ERR_UNSUPPORTED, "DSYMV: n too large");
     if (alpha != 0.0) {
         gbx_timer_begin(ctx, GBX_TIMER_GEMV);
-        symv_tiles<<<(unsigned)tiles, 256, 0, S(ctx)>>>(n, nb, gbx_lsame(uplo, 'L'), A, lda, xb, incx, part);
+        launch_pdl_short(gbx_ctx_sms(ctx), symv_tiles, dim3((unsigned)tiles), 256, S(ctx), n, nb, gbx_lsame(uplo, 'L'), A,
+                         lda, xb, incx, part);
         gbx_timer_end(ctx);
         gbx_count_launch(ctx, 1);
     } else {
         cudaMemsetAsync(part, 0, sizeof(double) * (size_t)nb * nb * SY_T, S(ctx));
     }
-    symv_finish<<<nb, 4 * SY_T, 0, S(ctx)>>>(n, nb, part, alpha, beta, yb, incy);
+    launch_pdl_short(gbx_ctx_sms(ctx), symv_finish, dim3(nb), 4 * SY_T, S(ctx), n, nb, part, alpha, beta, yb, incy);
     gbx_count_launch(ctx, 1);
     return gbx_check_launch(ctx, "dsymv");
 }
