@@ -86,18 +86,21 @@ gemv_n_partial(int m, int n, int chunk, const double *A, long long lda,
     if (r + 1 < m) pp[r + 1] = s1;
 }
 
-// 64 rows per CTA, four threads per row, each summing a quarter of the partials
-// in order with eight loads in flight (one thread per row on 32 CTAs took 10 us
-// for m = 8192, 38 partials), and placed while the partials are computed: DGEMV N
-// of 8192 x 8192 takes 124.5 us in a stream of calls, 129.6 without either.
-constexpr int FIN_ROWS = 64;
-__global__ void __launch_bounds__(4 * FIN_ROWS)
+// ROWS rows per CTA, 256 / ROWS threads per row, each summing its share of the
+// partials in order with eight loads in flight, placed while the partials are
+// computed.  64 rows per CTA: DGEMV N of 8192 x 8192 (38 partials) takes 124.5 us
+// in a stream of calls, with one thread per row in a launch that waits 129.6.
+// 16 where one CTA per SM does (few rows have many partials): 300 rows, 250
+// partials 13.5 us with 64, 9 with 16.
+template <int ROWS>
+__global__ void __launch_bounds__(GEMV_THREADS)
 gemv_n_finish(int m, int nchunks, const double *part, double alpha, double beta, double *y, int incy)
 {
     gbx_launch::pdl_enter();
-    __shared__ double red[4][FIN_ROWS];
-    const int l = threadIdx.x & (FIN_ROWS - 1), g = threadIdx.x / FIN_ROWS, i = blockIdx.x * FIN_ROWS + l;
-    const int c0 = (int)((long long)nchunks * g / 4), c1 = (int)((long long)nchunks * (g + 1) / 4);
+    constexpr int G = GEMV_THREADS / ROWS;
+    __shared__ double red[G][ROWS];
+    const int l = threadIdx.x % ROWS, g = threadIdx.x / ROWS, i = blockIdx.x * ROWS + l;
+    const int c0 = (int)((long long)nchunks * g / G), c1 = (int)((long long)nchunks * (g + 1) / G);
     double s = 0.0;
     if (i < m) {
 #pragma unroll 8
@@ -106,7 +109,9 @@ gemv_n_finish(int m, int nchunks, const double *part, double alpha, double beta,
     red[g][l] = s;
     __syncthreads();
     if (g || i >= m) return;
-    s = (red[0][l] + red[1][l]) + (red[2][l] + red[3][l]);
+    s = 0.0;
+#pragma unroll
+    for (int q = 0; q < G; q += 4) s += (red[q][l] + red[q + 1][l]) + (red[q + 2][l] + red[q + 3][l]);
     double *yp = y + (long long)i * incy;
     *yp = (beta == 0.0) ? alpha * s : fma(beta, *yp, alpha * s);
 }
@@ -240,8 +245,9 @@ extern "C" gbx_status gbx_dgemv(gbx_ctx *ctx, char trans, int m, int n, double a
         launch_pdl_short(sms, overlap ? gemv_n_partial<true> : gemv_n_partial<false>, g, GEMV_THREADS, S(ctx), m, n,
                          chunk, A, lda, xb, incx, part, vec);
         gbx_timer_end(ctx);
-        launch_pdl_short(sms, gemv_n_finish, dim3((m + FIN_ROWS - 1) / FIN_ROWS), 4 * FIN_ROWS, S(ctx), m, nchunks,
-                         part, alpha, beta, yb, incy);
+        const int fin = (m + 15) / 16 <= sms ? 16 : 64;
+        launch_pdl_short(sms, fin == 16 ? gemv_n_finish<16> : gemv_n_finish<64>, dim3((m + fin - 1) / fin), GEMV_THREADS,
+                         S(ctx), m, nchunks, part, alpha, beta, yb, incy);
         gbx_count_launch(ctx, 2);
         return gbx_check_launch(ctx, "dgemv");
     }

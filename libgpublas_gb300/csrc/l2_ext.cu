@@ -35,23 +35,25 @@ inline long long base_off(int n, int inc) { return inc >= 0 ? 0 : (long long)(n 
 // ------------------------------------------------------------------- DGER
 constexpr int GER_ROWS = 512, GER_COLS = 32;
 
-// 512 rows x 32 columns per CTA, two rows per thread, eight columns' loads in
-// flight.  The bound is HBM (16 bytes per element and one DFMA: the FP64
-// pipe alone would take two thirds of that time), so nothing else per
+// 512 rows x `width` (at most 32) columns per CTA, two rows per thread, eight
+// columns' loads in flight.  The bound is HBM (16 bytes per element and one DFMA:
+// the FP64 pipe alone would take two thirds of that time), so nothing else per
 // element may use the FP64 pipe: alpha y_j is formed once per CTA and the
 // test for a zero y_j (netlib leaves that column alone) is a bit in an
 // integer mask.  With the product and the test per element the FP64 pipe was
-// the bound: 8192 x 8192 took 387 us, now 162 us (1.07 GB, 6.6 TB/s).
+// the bound: 8192 x 8192 took 387 us, now 156 us (1.07 GB, 6.9 TB/s).
+// A row count that leaves threads without their second row, or zeros in y, takes
+// the same batches of eight: one column at a time, 300 x 4000 took 25 us, now 11.
 // vec: A is 16-byte aligned and lda even, so that a thread's two adjacent
 // rows are one 128-bit access in every column.
 __global__ void __launch_bounds__(256)
-ger_kernel(int m, int n, double alpha, const double *x, int incx, const double *y,
-           int incy, double *A, long long lda, int vec)
+ger_kernel(int m, int n, int width, double alpha, const double *x, int incx, const double *y, int incy, double *A,
+           long long lda, int vec)
 {
     gbx_launch::pdl_enter();
     __shared__ double coef[GER_COLS];
     __shared__ unsigned s_keep;
-    const int c0 = blockIdx.y * GER_COLS, cols = min(GER_COLS, n - c0);
+    const int c0 = blockIdx.y * width, cols = min(width, n - c0);
     const int tid = threadIdx.x;
     if (tid < 32) {
         const double yj = tid < cols ? y[(long long)(c0 + tid) * incy] : 0.0;
@@ -61,58 +63,49 @@ ger_kernel(int m, int n, double alpha, const double *x, int incx, const double *
         if (tid == 0) s_keep = keep;
     }
     __syncthreads();
-    const unsigned keep = s_keep;
+    const unsigned keep = s_keep;   // no bit beyond cols
     // vec: rows r, r + 1 with r even; otherwise rows r and r + 256
     const int r = blockIdx.x * GER_ROWS + (vec ? 2 * tid : tid);
     const int r2 = vec ? r + 1 : r + 256;
     if (r >= m) return;
     double *ap = A + (long long)c0 * lda + r;
+    const bool two = r2 < m;
     const double x0 = x[(long long)r * incx];
-    const double x1 = r2 < m ? x[(long long)r2 * incx] : 0.0;
-    if (keep == 0xffffffffu >> (GER_COLS - cols) && r2 < m) {   // no column is skipped
-        if (vec) {
+    const double x1 = two ? x[(long long)r2 * incx] : 0.0;
+    if (vec && two) {
 #pragma unroll 1
-            for (int j = 0; j < cols; j += 8) {
-                double2 v[8];
+        for (int j = 0; j < cols; j += 8) {
+            double2 v[8];
 #pragma unroll
-                for (int u = 0; u < 8; u++)
-                    if (j + u < cols) v[u] = *(const double2 *)(ap + (j + u) * lda);
+            for (int u = 0; u < 8; u++)
+                if (keep >> (j + u) & 1) v[u] = *(const double2 *)(ap + (j + u) * lda);
 #pragma unroll
-                for (int u = 0; u < 8; u++)
-                    if (j + u < cols) {
-                        const double c = coef[j + u];
-                        v[u].x = fma(x0, c, v[u].x);
-                        v[u].y = fma(x1, c, v[u].y);
-                        *(double2 *)(ap + (j + u) * lda) = v[u];
-                    }
-            }
-        } else {
-#pragma unroll 1
-            for (int j = 0; j < cols; j += 8) {
-                double v[8], w[8];
-#pragma unroll
-                for (int u = 0; u < 8; u++)
-                    if (j + u < cols) {
-                        v[u] = ap[(j + u) * lda];
-                        w[u] = ap[(j + u) * lda + 256];
-                    }
-#pragma unroll
-                for (int u = 0; u < 8; u++)
-                    if (j + u < cols) {
-                        const double c = coef[j + u];
-                        ap[(j + u) * lda] = fma(x0, c, v[u]);
-                        ap[(j + u) * lda + 256] = fma(x1, c, w[u]);
-                    }
-            }
+            for (int u = 0; u < 8; u++)
+                if (keep >> (j + u) & 1) {
+                    const double c = coef[j + u];
+                    v[u].x = fma(x0, c, v[u].x);
+                    v[u].y = fma(x1, c, v[u].y);
+                    *(double2 *)(ap + (j + u) * lda) = v[u];
+                }
         }
         return;
     }
-    for (int j = 0; j < cols; j++) {
-        if (!((keep >> j) & 1)) continue;
-        double *q = ap + j * lda;
-        const double c = coef[j];
-        *q = fma(x0, c, *q);
-        if (r2 < m) q[r2 - r] = fma(x1, c, q[r2 - r]);
+#pragma unroll 1
+    for (int j = 0; j < cols; j += 8) {
+        double v[8], w[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            if (keep >> (j + u) & 1) {
+                v[u] = ap[(j + u) * lda];
+                if (two) w[u] = ap[(j + u) * lda + 256];
+            }
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            if (keep >> (j + u) & 1) {
+                const double c = coef[j + u];
+                ap[(j + u) * lda] = fma(x0, c, v[u]);
+                if (two) ap[(j + u) * lda + 256] = fma(x1, c, w[u]);
+            }
     }
 }
 
@@ -134,7 +127,7 @@ symv_tiles(int n, int nb, int lower, const double *A, long long lda, const doubl
     // tile index -> (I, J) with I >= J (lower) in row-major triangle order
     // (FP32 square root and integer correction: an FP64 one by every thread
     // cost the FP64 pipe nearly half as much as the tile's products:
-    // n = 8192 took 198 us, now 136 us)
+    // n = 8192 took 198 us, then 136)
     const int t = blockIdx.x;
     int I = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
     while ((long long)(I + 1) * (I + 2) / 2 <= t) I++;
@@ -143,19 +136,20 @@ symv_tiles(int n, int nb, int lower, const double *A, long long lda, const doubl
     if (!lower) { const int tmp = I; I = J; J = tmp; }   // upper: I <= J
     const int r0 = I * SY_T, c0 = J * SY_T;
     const int tid = threadIdx.x;
-    for (int q = tid; q < SY_T * SY_T; q += blockDim.x) {
-        const int i = q % SY_T, j = q / SY_T;
+    double v[SY_T * SY_T / 256];   // all loads in flight before the first store to shared memory:
+    // n = 300 7.3 us instead of 13.9, n = 8192 125 instead of 136
+#pragma unroll
+    for (int f = 0; f < SY_T * SY_T / 256; f++) {
+        const int q = tid + f * 256, i = q % SY_T, j = q / SY_T;
         const int gi = r0 + i, gj = c0 + j;
-        double v = 0.0;
+        v[f] = 0.0;
         if (gi < n && gj < n) {
-            if (I != J) v = A[(long long)gj * lda + gi];
-            else {
-                const bool stored = lower ? gi >= gj : gi <= gj;
-                v = stored ? A[(long long)gj * lda + gi] : A[(long long)gi * lda + gj];   // mirror
-            }
+            const bool stored = I != J || (lower ? gi >= gj : gi <= gj);   // else its mirror image
+            v[f] = stored ? A[(long long)gj * lda + gi] : A[(long long)gi * lda + gj];
         }
-        s[i][j] = v;
     }
+#pragma unroll
+    for (int f = 0; f < SY_T * SY_T / 256; f++) s[(tid + f * 256) % SY_T][(tid + f * 256) / SY_T] = v[f];
     if (tid < SY_T) {
         sxJ[tid] = (c0 + tid < n) ? x[(long long)(c0 + tid) * incx] : 0.0;
         sxI[tid] = (r0 + tid < n) ? x[(long long)(r0 + tid) * incx] : 0.0;
@@ -595,11 +589,16 @@ extern "C" gbx_status gbx_dger(gbx_ctx *ctx, int m, int n, double alpha, const d
     const int info = gbx_check_ger_args(m, n, incx, incy, lda);
     if (info) return gbx_fail(ctx, GBX_ERR_ARG, "DGER parameter %d", info);
     if (m == 0 || n == 0 || alpha == 0.0) return GBX_OK;
+    // 32 columns per CTA, 16 or 8 as long as there is at most one CTA per SM
+    // (1000 x 800: 9.6 us with 32, 6.7 with 16)
     dim3 g((m + GER_ROWS - 1) / GER_ROWS, (n + GER_COLS - 1) / GER_COLS);
+    int width = GER_COLS;
+    while (width > 8 && (long long)g.x * ((n + width / 2 - 1) / (width / 2)) <= gbx_ctx_sms(ctx)) width /= 2;
+    g.y = (n + width - 1) / width;
     if (g.y > 65535) return gbx_fail(ctx, GBX_ERR_UNSUPPORTED, "DGER: n too large");
     gbx_timer_begin(ctx, GBX_TIMER_GEMV);
     const int vec = (((uintptr_t)A) & 15) == 0 && lda % 2 == 0;
-    launch_pdl_short(gbx_ctx_sms(ctx), ger_kernel, g, 256, S(ctx), m, n, alpha, x + base_off(m, incx), incx,
+    launch_pdl_short(gbx_ctx_sms(ctx), ger_kernel, g, 256, S(ctx), m, n, width, alpha, x + base_off(m, incx), incx,
                      y + base_off(n, incy), incy, A, lda, vec);
     gbx_timer_end(ctx);
     gbx_count_launch(ctx, 1);

@@ -70,3 +70,31 @@ def test_symmetric_products(dev, n, uplo):
     for i in range(4):
         ref = a @ ref
         assert float((x[i + 1] - ref).norm()) <= 64 * (n + 8) * 2.0 ** -53
+
+
+@pytest.mark.parametrize("m,n", [(1, 9), (255, 8), (256, 9), (257, 33), (300, 1208), (511, 1209), (512, 2424), (513, 608),
+                                 (1000, 609), (1000, 1217), (700, 4865)])
+@pytest.mark.parametrize("pad", [0, 1])
+def test_update_widths(dev, m, n, pad):
+    """8, 16 or 32 columns per CTA, second rows that end inside a CTA, columns
+    left alone (y_j = 0).  Two roundings of values below 2: 2^-51."""
+    import torch
+    from libgpublas_gb300._lib import _dp
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(7 * m + n + pad)
+
+    def uni(*s):
+        return torch.rand(*s, dtype=torch.float64, device="cuda", generator=gen) * 2 - 1
+    a, x, y = uni(n, m + pad), uni(m), uni(n)
+    y[torch.rand(n, device="cuda", generator=gen) < 0.2] = 0.0
+    a[y == 0.0, 0] = float("inf")
+    ref = a.clone()
+    live = y != 0.0
+    ref[live, :m] += 0.75 * y[live][:, None] * x[None, :]
+    torch.cuda.synchronize()
+    assert dev.L.gbx_dger(dev.ctx, m, n, 0.75, _dp(x), 1, _dp(y), 1, _dp(a), m + pad) == 0
+    dev.sync()
+    fin = torch.isfinite(ref)
+    assert torch.equal(torch.isfinite(a), fin)
+    assert torch.equal(a[~live], ref[~live]) and torch.equal(a[:, m:], ref[:, m:])
+    assert float((a[fin] - ref[fin]).abs().max()) <= 2.0 ** -51
