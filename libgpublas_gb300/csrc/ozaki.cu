@@ -35,6 +35,7 @@
 #include "gemm_host.h"
 #include "launch.cuh"
 #include "tc_ptx.cuh"
+#include "tri_inverse.cuh"
 
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -2700,7 +2701,7 @@ namespace {
 // U is handled as the lower triangle L' = P U P (P the order-reversing
 // permutation; U^-1 = P L'^-1 P); X = W = L'^-1, or W^T for op = 'T'/'C'.
 // Two launches:
-//   * oz_trinv_diag: the 32 x 32 diagonal blocks, one CTA of four warps each;
+//   * oz_trinv_diag: the 32 x 32 diagonal blocks, one CTA each (tri_inverse.cuh);
 //   * oz_trinv_kernel: forward substitution by blocks of 32 rows, two columns
 //     of the inverse per CTA (j and n - 1 - j: together they have about n rows
 //     to solve whatever j is), one thread per row.  Block I of both columns is
@@ -2708,7 +2709,7 @@ namespace {
 //     row below subtracts its 32 products, from columns of L' that were loaded
 //     during the block before.
 // The bound is the FP64 pipe (2 lanes per clock per SM, n^2 / 2 FMAs per CTA: 16
-// us at n = 256) and eight block steps.  n = 256: 15 + 22 us; one warp
+// us at n = 256) and eight block steps.  n = 256: 10 + 22 us; one warp
 // per column stepping through its 256 rows one by one took 235 us.
 constexpr int OZ_TI_NMAX = 256, OZ_TI_BLK = 32;
 
@@ -2724,54 +2725,35 @@ struct OzTriView {
     }
 };
 
-// D: per block 32 x 32, column-major.  Lane j substitutes for column j, warp w
-// holding rows 4u + w; the warp of row i + 1 finishes and publishes it before
-// its other rows and does not wait for the other warps (a warp has one FP64
-// instruction in flight, 65 cycles each: a single warp took 24 us).
+// D: per block 32 x 32, column-major; the two 16 x 16 halves by a warp each, then
+// joined (10 us; substitution on 32 rows by four warps, a hand-over per
+// row, took 15).
 __global__ void __launch_bounds__(128)
-oz_trinv_diag(OzTriView L, int unit, double *__restrict__ D)
+oz_trinv_diag(OzTriView L, int unit, double *D)
 {
-    using namespace gbx_launch;
-    pdl_enter();
-    __shared__ double sL[OZ_TI_BLK][OZ_TI_BLK + 1];   // [column][row]
-    __shared__ double sw[OZ_TI_BLK][OZ_TI_BLK + 1];   // row i of the inverse
-    __shared__ double ri[OZ_TI_BLK];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r0 = blockIdx.x * OZ_TI_BLK;
+    gbx_launch::pdl_enter();
+    constexpr int LD = OZ_TI_BLK + 1;
+    __shared__ double sL[OZ_TI_BLK * LD], sX[OZ_TI_BLK * LD], sW[16 * 17];   // [column][row]
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, r0 = blockIdx.x * OZ_TI_BLK;
     const int m = min(OZ_TI_BLK, L.n - r0);
+    double v[8];
 #pragma unroll
     for (int q = 0; q < 8; q++) {   // identity beyond n
         const int c = 4 * q + warp;
-        double v = lane == c ? 1.0 : 0.0;
-        if (c <= lane && lane < m && !(unit && lane == c)) v = L(r0 + lane, r0 + c);
-        sL[c][lane] = v;
-        if (lane == c) ri[c] = 1.0 / v;
+        v[q] = lane == c ? 1.0 : 0.0;
+        if (c <= lane && lane < m && !(unit && lane == c)) v[q] = L(r0 + lane, r0 + c);
     }
+#pragma unroll
+    for (int q = 0; q < 8; q++) sL[(4 * q + warp) * LD + lane] = v[q];
     __syncthreads();
-    double s[8];
-#pragma unroll
-    for (int u = 0; u < 8; u++) s[u] = 4 * u + warp == lane ? 1.0 : 0.0;
-    auto publish = [&](int i) {
-        sw[i][lane] = s[i >> 2] * ri[i];
-        bar_arrive(1 + (i & 7), 128);
-    };
-    if (warp == 0) publish(0);
-#pragma unroll
-    for (int i = 0; i < OZ_TI_BLK - 1; i++) {
-        if (warp != (i & 3)) bar_wait(1 + (i & 7), 128);
-        const double w = sw[i][lane];
-        if (warp == ((i + 1) & 3)) {
-            s[(i + 1) >> 2] = fma(-sL[i][i + 1], w, s[(i + 1) >> 2]);
-            publish(i + 1);
-        }
-#pragma unroll
-        for (int u = 0; u < 8; u++)
-            if (4 * u + 3 > i && 4 * u + warp > i + (warp == ((i + 1) & 3) ? 1 : 0))
-                s[u] = fma(-sL[i][4 * u + warp], w, s[u]);
-    }
-    if (warp != ((OZ_TI_BLK - 1) & 3)) bar_wait(1 + ((OZ_TI_BLK - 1) & 7), 128);
+    if (warp < 2) gbx_tri::invert16<LD>(sL, sX, 16 * warp);
+    __syncthreads();
+    gbx_tri::join32_w<LD>(sL, sX, sW, 0, t);
+    __syncthreads();
+    gbx_tri::join32_x<LD>(sX, sW, 0, t);
     __syncthreads();
     double *d = D + (size_t)blockIdx.x * OZ_TI_BLK * OZ_TI_BLK;
-    for (int t = threadIdx.x; t < OZ_TI_BLK * OZ_TI_BLK; t += 128) d[t] = sw[t & 31][t >> 5];
+    for (int e = t; e < OZ_TI_BLK * OZ_TI_BLK; e += 128) d[e] = sX[(e >> 5) * LD + (e & 31)];
 }
 
 __global__ void __launch_bounds__(OZ_TI_NMAX)
