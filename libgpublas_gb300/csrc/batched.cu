@@ -162,7 +162,7 @@ template <bool BIG>
 __global__ void __launch_bounds__(BT_THREADS, BIG ? 2 : 4)
 grouped_kernel(const DevOp *__restrict__ ops, const Item *__restrict__ items, int nitems, int *counter)
 {
-    __shared__ __align__(16) double smem[TRSM_MAX_ORDER * TRSM_SYS];
+    __shared__ __align__(16) double smem[gbx_grouped::trsm_smem(TRSM_MAX_ORDER, TRSM_SYS)];
     __shared__ int s_item;
     static_assert(sizeof smem >= sizeof(double) * 4 * 8 * 64, "two stages of two 8 x 64 panels");
     int it = blockIdx.x;
@@ -278,7 +278,7 @@ void tile_items(const DevOp &o, int opi, int variant, std::vector<Item> &items, 
         const int order = o.left ? o.m : o.n;
         for (int s = 0; s * TRSM_SYS < nsys; s++) {
             items.push_back({opi, s, 0, 0});
-            cost.push_back((double)order * order * TRSM_SYS * 4.0);   // serial substitution
+            cost.push_back((double)order * order * TRSM_SYS / 2.0 + 1000.0 * order);   // and the chain of its blocks
         }
         return;
     }

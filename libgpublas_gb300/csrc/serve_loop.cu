@@ -60,7 +60,7 @@ constexpr int LOOP_MAX_MN = 512, LOOP_MAX_K = 4096;   // larger products run as 
                                                       // the slot streams, with every SM at their disposal
 constexpr int LOOP_TRSM_SYS = 16;
 constexpr int LOOP_TRSM_ORDER = 256;
-constexpr size_t LOOP_DSMEM = sizeof(double) * LOOP_TRSM_ORDER * LOOP_TRSM_SYS;   // 32 KB
+constexpr size_t LOOP_DSMEM = sizeof(double) * gbx_grouped::trsm_smem(LOOP_TRSM_ORDER, LOOP_TRSM_SYS);   // 38.4 KB
 constexpr int LOOP_POLLERS = 8;                 // CTAs that watch the ring for new requests
 constexpr unsigned long long LOOP_IDLE_NS = 20000000ull;    // 20 ms without work: the CTA leaves
 constexpr unsigned long long LOOP_WAIT_NS = 1000000000ull;  // 1 s for a reserved queue item
@@ -142,7 +142,7 @@ __device__ void finish(RingSlot *ring, unsigned long long ticket, int status)
 __global__ void __launch_bounds__(LOOP_THREADS, 1)
 serve_loop_kernel(LoopState *st, RingSlot *ring, const LoopCtl *ctl)
 {
-    extern __shared__ __align__(16) double tsm[];   // triangular solves: LOOP_TRSM_ORDER x LOOP_TRSM_SYS
+    extern __shared__ __align__(16) double tsm[];   // triangular solves
     __shared__ unsigned long long s_ticket, s_base;
     __shared__ int s_action, s_item, s_n, s_qi;
     unsigned long long idle0 = gbx_tc::globaltimer();
