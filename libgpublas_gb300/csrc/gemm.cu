@@ -130,6 +130,12 @@ static gbx_status choose_and_launch(gbx_ctx *ctx, GemmArgs<T> p, const char *wha
         if (bm == 32) return launch_gemm_tile<T, 2>(ctx, p, what);
         return launch_gemm_tile<T, 1>(ctx, p, what);
     } else if constexpr (sizeof(T) <= 8) {
+        if constexpr (std::is_same<T, float>::value) {
+            if (!flag && launch_gemm_short(ctx, p)) {
+                gbx_count_launch(ctx, 1);
+                return gbx_check_launch(ctx, what);
+            }
+        }
         if (tiles(128) >= want) return launch_gemm_tile<T, 8>(ctx, p, what, flag, epoch);
         if (tiles(64) >= want) return launch_gemm_tile<T, 4>(ctx, p, what, flag, epoch);
         if (tiles(32) >= want) return launch_gemm_tile<T, 2>(ctx, p, what, flag, epoch);

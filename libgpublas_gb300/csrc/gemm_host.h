@@ -8,8 +8,9 @@
 namespace gbx_gemm {
 template <typename T>
 gbx_status launch_gemm(gbx_ctx *ctx, GemmArgs<T> p, const char *what);
-// FP64 launches of few waves (gemm_small.cu); false: not one of them.
+// FP64 launches of few waves and small SGEMMs (gemm_small.cu); false: not one of them.
 bool launch_gemm_short(gbx_ctx *ctx, GemmArgs<double> p, int bm);
+bool launch_gemm_short(gbx_ctx *ctx, GemmArgs<float> p);
 // The SIMT SGEMM of a full C, which does nothing unless *flag == epoch when it runs.
 gbx_status launch_gemm_if(gbx_ctx *ctx, GemmArgs<float> p, const char *what, const int *flag, int epoch);
 // SGEMM on the tensor cores (sgemm_tc.cu); *done: the call was taken.

@@ -28,20 +28,21 @@ namespace {
 // with this one (the rate at which Python issues the calls).
 constexpr int SM_BM = 8, SM_BN = 16, SM_BK = 64, SM_THREADS = SM_BM * SM_BN;
 
+template <typename T>
 __global__ void __launch_bounds__(SM_THREADS)
-gemm_small_kernel(GemmArgs<double> p)
+gemm_small_kernel(GemmArgs<T> p)
 {
     pdl_enter();
-    __shared__ double As[2][SM_BK][SM_BM], Bs[2][SM_BK][SM_BN];
+    __shared__ T As[2][SM_BK][SM_BM], Bs[2][SM_BK][SM_BN];
     const int m0 = (int)(blockIdx.x % p.tiles_m) * SM_BM, n0 = (int)(blockIdx.x / p.tiles_m) * SM_BN;
     const int tid = threadIdx.x, tx = tid % SM_BN, ty = tid / SM_BN;
     const int row = m0 + ty, col = n0 + tx;
-    double *cp = p.C + (long long)col * p.ldc + row;
-    const bool beta0 = Ops<double>::is_zero(p.beta);
+    T *cp = p.C + (long long)col * p.ldc + row;
+    const bool beta0 = Ops<T>::is_zero(p.beta);
     const bool live = row < p.m && col < p.n;
-    const double cold = live && !beta0 ? *cp : 0.0;
+    const T cold = live && !beta0 ? *cp : T(0);
     constexpr int NA = SM_BM * SM_BK / SM_THREADS, NB = SM_BN * SM_BK / SM_THREADS;
-    double ra[NA], rb[NB];
+    T ra[NA], rb[NB];
     // neighbouring threads along the contiguous index: rows of A or k for A^T,
     // k for B or columns for B^T
     auto load = [&](int k0) {
@@ -49,13 +50,13 @@ gemm_small_kernel(GemmArgs<double> p)
         for (int q = 0; q < NA; q++) {
             const int t = tid + q * SM_THREADS;
             const int r = m0 + (p.ta ? t / SM_BK : t % SM_BM), k = k0 + (p.ta ? t % SM_BK : t / SM_BM);
-            ra[q] = r < p.m && k < p.k ? p.A[p.ta ? (long long)r * p.lda + k : (long long)k * p.lda + r] : 0.0;
+            ra[q] = r < p.m && k < p.k ? p.A[p.ta ? (long long)r * p.lda + k : (long long)k * p.lda + r] : T(0);
         }
 #pragma unroll
         for (int q = 0; q < NB; q++) {
             const int t = tid + q * SM_THREADS;
             const int c = n0 + (p.tb ? t % SM_BN : t / SM_BK), k = k0 + (p.tb ? t / SM_BN : t % SM_BK);
-            rb[q] = c < p.n && k < p.k ? p.B[p.tb ? (long long)k * p.ldb + c : (long long)c * p.ldb + k] : 0.0;
+            rb[q] = c < p.n && k < p.k ? p.B[p.tb ? (long long)k * p.ldb + c : (long long)c * p.ldb + k] : T(0);
         }
     };
     auto store = [&](int s) {
@@ -70,7 +71,7 @@ gemm_small_kernel(GemmArgs<double> p)
             Bs[s][p.tb ? t / SM_BN : t % SM_BK][p.tb ? t % SM_BN : t / SM_BK] = rb[q];
         }
     };
-    double acc = 0.0;
+    T acc = T(0);
     load(0);
     store(0);
     __syncthreads();
@@ -87,7 +88,7 @@ gemm_small_kernel(GemmArgs<double> p)
             __syncthreads();
         }
     }
-    if (live) *cp = beta0 ? Ops<double>::mul(p.alpha, acc) : Ops<double>::axpby(p.alpha, acc, p.beta, cold);
+    if (live) *cp = beta0 ? Ops<T>::mul(p.alpha, acc) : Ops<T>::axpby(p.alpha, acc, p.beta, cold);
 }
 
 template <int TM, int BK>
@@ -114,7 +115,7 @@ bool launch_gemm_short(gbx_ctx *ctx, GemmArgs<double> p, int bm)
     if (bm == 16 && plain && 2 * t16 <= sms) {
         p.tiles_m = (p.m + SM_BM - 1) / SM_BM;
         p.tiles_n = (p.n + SM_BN - 1) / SM_BN;
-        launch_pdl(gemm_small_kernel, (unsigned)(p.tiles_m * p.tiles_n), SM_THREADS, 0, s, p);
+        launch_pdl(gemm_small_kernel<double>, (unsigned)(p.tiles_m * p.tiles_n), SM_THREADS, 0, s, p);
         return true;
     }
     p.tiles_m = (p.m + bm - 1) / bm;
@@ -124,6 +125,20 @@ bool launch_gemm_short(gbx_ctx *ctx, GemmArgs<double> p, int bm)
     if (blocks > sms || (p.c_part != C_FULL && p.m != p.n)) return false;
     launch_pdl(bm == 64 ? gemm_overlap_kernel<4, 8> : (bm == 32 ? gemm_overlap_kernel<2, 8> : gemm_overlap_kernel<1, 16>),
                (unsigned)blocks, GEMM_THREADS, 0, s, p);
+    return true;
+}
+
+// SGEMM where the core's 16 x 16 tiles would leave half the SMs idle (the same
+// bits again; the core loads 8 k per panel).  Through sgemm_, which waits for the
+// result: 134 x 76 x 125 25 -> 22 us, 60 x 50 x 1000 56 -> 39.
+bool launch_gemm_short(gbx_ctx *ctx, GemmArgs<float> p)
+{
+    const long long t16 = ((p.m + 15LL) / 16) * ((p.n + 15) / 16);
+    if (p.c_part != C_FULL || p.tri_a || p.tri_b || p.sym_a || p.sym_b || 2 * t16 > gbx_ctx_sms(ctx)) return false;
+    p.tiles_m = (p.m + SM_BM - 1) / SM_BM;
+    p.tiles_n = (p.n + SM_BN - 1) / SM_BN;
+    launch_pdl(gemm_small_kernel<float>, (unsigned)(p.tiles_m * p.tiles_n), SM_THREADS, 0,
+               (cudaStream_t)gbx_ctx_get_stream(ctx), p);
     return true;
 }
 
