@@ -1,6 +1,6 @@
 // gemm_small.cu — FP64 GEMM launches of at most one CTA per SM: the core's tiles
 // launched so that they overlap the end of the kernel before them, and a
-// half-height tile for products that would leave most SMs idle.  (Not larger
+// half-height tile for products (SGEMM's too) that would leave most SMs idle.  (Not larger
 // ones: CTAs placed while the kernel before still runs spread unevenly over the
 // SMs, and the FP64 pipe of the fullest SM sets the time: DGEMM 756 x 330 x 1710,
 // 1008 tiles, took 873 us overlapped and 769 not.)
