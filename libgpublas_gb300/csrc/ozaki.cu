@@ -682,8 +682,8 @@ template <bool ONE, bool SEL>
 __global__ void __launch_bounds__(OZ_PREP_THREADS)
 oz_prep_small(OzPrepOp a, OzPrepOp b, int planes, int *status)
 {
-    // the product kernel may be scheduled now: its set-up needs none of this
-    // launch's results, and it waits for them (griddepcontrol.wait)
+    // the product kernel may be placed once this one runs: its set-up needs none
+    // of this launch's results, and it waits for them (griddepcontrol.wait)
     gbx_launch::pdl_enter();
     const int na = a.Rp / OZ_PREP_ROWS;
     const bool is_a = (int)blockIdx.x < na;
@@ -1602,8 +1602,6 @@ oz_gemm_sk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     volatile int *status = p.status;
 
-    // the next call's preparation may be placed on the SMs this launch leaves
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (threadIdx.x == 0) {
         for (int i = 0; i < OZS_AMAX; i++) { mbar_init(&fullA[i], 1); mbar_init(&emptyA[i], 1); }
         for (int i = 0; i < OZS_BSTG; i++) { mbar_init(&fullB[i], 1); mbar_init(&emptyB[i], 1); }
@@ -1629,6 +1627,8 @@ oz_gemm_sk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     // above overlaps its tail; its slices, scales and S are complete and
     // visible after this wait (a no-op for an ordinary launch).
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    // the next call's preparation may be placed on the SMs this launch leaves
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int P = p.smax;   // digit planes prepared: S <= P
     const int nkb = p.Kp / OZ_BK;
     // B stages first (all P slices of BN rows each: a stage can be requested
