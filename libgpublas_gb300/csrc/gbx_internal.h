@@ -35,15 +35,15 @@ gbx_status gbx_fail(gbx_ctx *ctx, gbx_status st, const char *fmt, ...);
 #define GBX_WS_BATCH    10  /* grouped/batched descriptors                  */
 #define GBX_WS_STAGE_D  11
 #define GBX_WS_TRSM_X   12  /* dtrsm_ozaki: inverse of the triangle          */
-#define GBX_WS_SGEMM    13  /* SGEMM: bf16 planes of both operands          */
+#define GBX_WS_SPARE13  13  /* unused                                       */
 #define GBX_WS_GEMV     14  /* gemv partial sums                            */
 #define GBX_WS_RED      15  /* reduction partials                           */
 gbx_status gbx_ws(gbx_ctx *ctx, int slot, size_t bytes, void **ptr);
-/* Whether gbx_ws would return without allocating. */
-int gbx_ws_ready(const gbx_ctx *ctx, int slot, size_t bytes);
-/* A number that differs from call to call on a context (a kernel's mark in
- * device memory is recognised by it, so the mark need not be reset). */
-int gbx_ctx_epoch(gbx_ctx *ctx);
+/* Scratch that one call uses between get and put, which comes after its last
+ * launch; calls of the context on other streams have other blocks.  Not for a
+ * stream that is being captured. */
+gbx_status gbx_scratch_get(gbx_ctx *ctx, size_t bytes, void **ptr, int *block);
+gbx_status gbx_scratch_put(gbx_ctx *ctx, int block);
 /* Pinned host scratch owned by the context (for small results). */
 gbx_status gbx_pinned(gbx_ctx *ctx, size_t bytes, void **ptr);
 void gbx_count_launch(gbx_ctx *ctx, int n);

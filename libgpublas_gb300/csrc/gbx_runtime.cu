@@ -32,6 +32,16 @@ struct gbx_timer_rec {
     int used;
 };
 
+#define GBX_SCRATCH_BLOCKS 4
+#define GBX_SCRATCH_MAX ((size_t)9 << 28)   // 2.25 GiB: one block of the largest kind, or several smaller ones
+struct gbx_scratch {
+    void *p;
+    size_t bytes;
+    unsigned long long stream;   // id of the stream that used it last
+    cudaEvent_t done;            // its last use has ended
+    uint64_t used;               // number of that use
+};
+
 struct gbx_ctx {
     int device;
     int sms;
@@ -39,10 +49,11 @@ struct gbx_ctx {
     cudaStream_t stream;
     void  *ws[GBX_WS_SLOTS];
     size_t ws_bytes[GBX_WS_SLOTS];
+    gbx_scratch scratch[GBX_SCRATCH_BLOCKS];
+    uint64_t scratch_uses;
     void  *pinned;
     size_t pinned_bytes;
     uint64_t launches;
-    int epoch;
     int *status_dev;     // device status words of kernels with bounded waits ([0]; [12] a counter)
     int *status_host;    // mapped pinned mirror of status_dev[0], written by the kernels on failure
     int *status_mirror;  // the mirror's device address
@@ -191,6 +202,13 @@ extern "C" gbx_status gbx_ctx_destroy(gbx_ctx *c)
     cudaStreamSynchronize(c->stream);
     for (int i = 0; i < GBX_WS_SLOTS; i++)
         if (c->ws[i]) cudaFree(c->ws[i]);
+    for (int i = 0; i < GBX_SCRATCH_BLOCKS; i++) {
+        gbx_scratch &b = c->scratch[i];
+        if (!b.done) continue;
+        cudaEventSynchronize(b.done);   // (its stream need not be the context's)
+        if (b.p) cudaFree(b.p);
+        cudaEventDestroy(b.done);
+    }
     if (c->pinned) cudaFreeHost(c->pinned);
     if (c->status_dev) cudaFree(c->status_dev);
     if (c->status_host) cudaFreeHost(c->status_host);
@@ -344,15 +362,84 @@ extern "C" gbx_status gbx_ws(gbx_ctx *c, int slot, size_t bytes, void **ptr)
     return GBX_OK;
 }
 
-extern "C" int gbx_ws_ready(const gbx_ctx *c, int slot, size_t bytes)
+// A call's own scratch.  Calls on one stream share a block (they run in turn); a
+// call on another stream takes a block that nobody uses any more, or a new one, so
+// that the two stay independent; only with all blocks in use, or GBX_SCRATCH_MAX
+// bytes held, it waits (on the device) for the block used longest ago.  Streams
+// are told apart by their ids, which are not reused as handles are, and the event
+// of a block's last use holds when its stream is gone.
+extern "C" gbx_status gbx_scratch_get(gbx_ctx *c, size_t bytes, void **ptr, int *block)
 {
-    return c && slot >= 0 && slot < GBX_WS_SLOTS && c->ws_bytes[slot] >= bytes;
+    if (!c) return GBX_ERR_ARG;
+    unsigned long long id;
+    cudaError_t e = cudaStreamGetId(c->stream, &id);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return gbx_fail(c, GBX_ERR_CUDA, "scratch: %s", cudaGetErrorString(e));
+    }
+    int pick = -1, idle = -1, unused = -1, oldest = -1;
+    size_t held = 0;
+    for (int i = 0; i < GBX_SCRATCH_BLOCKS; i++) {
+        const gbx_scratch &b = c->scratch[i];
+        held += b.bytes;
+        if (!b.done) unused = i;
+        else if (b.stream == id) pick = i;
+        if (b.done && (oldest < 0 || b.used < c->scratch[oldest].used)) oldest = i;
+    }
+    if (pick < 0) {
+        for (int i = 0; i < GBX_SCRATCH_BLOCKS; i++) {
+            const gbx_scratch &b = c->scratch[i];
+            if (!b.done) continue;
+            if (cudaEventQuery(b.done) != cudaSuccess) {
+                cudaGetLastError();   // not ready
+                continue;
+            }
+            // the smallest that is large enough, or the largest
+            const size_t now = idle < 0 ? 0 : c->scratch[idle].bytes;
+            if (idle < 0 || (b.bytes >= bytes ? now < bytes || b.bytes < now : b.bytes > now)) idle = i;
+        }
+        if (idle >= 0 && c->scratch[idle].bytes >= bytes) pick = idle;
+        else if (unused >= 0 && (oldest < 0 || held + bytes <= GBX_SCRATCH_MAX)) pick = unused;
+        else pick = idle >= 0 ? idle : oldest;
+    }
+    gbx_scratch &b = c->scratch[pick];
+    if (!b.done) {
+        e = cudaEventCreateWithFlags(&b.done, cudaEventDisableTiming);
+        if (e != cudaSuccess) b.done = nullptr;
+    } else if (b.stream != id) {
+        e = cudaStreamWaitEvent(c->stream, b.done, 0);
+    }
+    if (e == cudaSuccess && b.bytes < bytes) {
+        if (inject_alloc_failure()) return gbx_fail(c, GBX_ERR_ALLOC, "scratch: injected allocation failure");
+        // a capture on another thread is none of this allocation's business
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        e = cudaEventSynchronize(b.done);
+        if (b.p) cudaFree(b.p);
+        b.p = nullptr;
+        b.bytes = 0;
+        const size_t want = (bytes + std::min(bytes / 4, (size_t)64 << 20) + 4095) & ~(size_t)4095;
+        if (e == cudaSuccess) e = cudaMalloc(&b.p, want);
+        if (e == cudaSuccess) b.bytes = want;
+        else b.p = nullptr;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return gbx_fail(c, GBX_ERR_ALLOC, "scratch: %zu bytes: %s", bytes, cudaGetErrorString(e));
+    }
+    b.stream = id;
+    b.used = ++c->scratch_uses;
+    *ptr = b.p;
+    *block = pick;
+    return GBX_OK;
 }
 
-extern "C" int gbx_ctx_epoch(gbx_ctx *c)
+// After the call's last launch.
+extern "C" gbx_status gbx_scratch_put(gbx_ctx *c, int block)
 {
-    c->epoch = (int)((unsigned)c->epoch + 1u);
-    return c->epoch;
+    const cudaError_t e = cudaEventRecord(c->scratch[block].done, c->stream);
+    return e == cudaSuccess ? GBX_OK : gbx_fail(c, GBX_ERR_CUDA, "scratch: %s", cudaGetErrorString(e));
 }
 
 extern "C" gbx_status gbx_ctx_reserve(gbx_ctx *c, size_t bytes)

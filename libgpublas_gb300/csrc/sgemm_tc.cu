@@ -50,6 +50,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 
 using namespace gbx_gemm;
@@ -93,7 +94,8 @@ __device__ __forceinline__ float hi_f(uint32_t v) { return __uint_as_float(v & 0
 // contiguous index, written as 16-byte pieces along k.  Bound by memory: 4
 // bytes read and 6 written per element.
 __global__ void __launch_bounds__(256)
-split_bf16x3(SplitOp a, SplitOp b, int K, long long pitch, int blocks_a, int *flag, int epoch)
+split_bf16x3(SplitOp a, SplitOp b, int K, long long pitch, int blocks_a, unsigned *flag,
+             unsigned tag)
 {
     __shared__ float s[64][65];
     const bool is_a = (int)blockIdx.x < blocks_a;
@@ -119,7 +121,7 @@ split_bf16x3(SplitOp a, SplitOp b, int K, long long pitch, int blocks_a, int *fl
         else s[x][y] = v[u];
     }
     if (__syncthreads_or(bad)) {
-        if (t == 0) *flag = epoch;
+        if (t == 0) *flag = tag;
     }
     const size_t plane = (size_t)o.rows * pitch;
 #pragma unroll
@@ -150,8 +152,8 @@ struct StParams {
     float alpha, beta;
     float *C;
     long long ldc;
-    const int *flag;
-    int epoch;
+    const unsigned *flag;
+    unsigned tag;
     int *status, *status_host;
 };
 
@@ -217,7 +219,7 @@ __device__ __forceinline__ void st_store(const StParams &p, const float (&acc)[3
 __global__ void __launch_bounds__(ST_THREADS, 1)
 sgemm_bf16x3(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, StParams p)
 {
-    if (*p.flag == p.epoch) return;   // the SIMT kernel behind this one computes the product
+    if (*p.flag == p.tag) return;   // the SIMT kernel behind this one computes the product
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t *smB = smem + ST_ASLOTS * ST_PLANE;
@@ -442,6 +444,57 @@ size_t st_plane_bytes(int m, int n, int k, size_t *a_bytes)
     return a + 6 * (size_t)n * pitch;
 }
 
+// What the flag is set to: different in every call of the process, so that
+// scratch need not be cleared.  (Scratch that happens to hold it costs the SIMT
+// kernel's time, no more.)
+unsigned next_tag()
+{
+    static std::atomic<unsigned> n{0x9d3c5a7eu};
+    return ++n;
+}
+
+// The product with its scratch at ws.
+gbx_status run_planes(gbx_ctx *ctx, const GemmArgs<float> &g, const char *what, char *ws, size_t a_bytes, int *words,
+                      int *mirror)
+{
+    const long long pitch = ((long long)g.k + 7) / 8 * 8;
+    __nv_bfloat16 *pa = (__nv_bfloat16 *)(ws + 256), *pb = (__nv_bfloat16 *)(ws + 256 + a_bytes);
+    CUtensorMap tmA, tmB;
+    if (!plane_map(&tmA, pa, g.m, g.k, pitch, 1) || !plane_map(&tmB, pb, g.n, g.k, pitch, 3))
+        return gbx_fail(ctx, GBX_ERR_CUDA, "%s: cuTensorMapEncodeTiled failed", what);
+    unsigned *flag = (unsigned *)ws;
+    const unsigned tag = next_tag();
+
+    SplitOp a{}, b{};
+    a.X = g.A; a.ld = g.lda; a.row_k = g.ta; a.rows = g.m; a.P = pa; a.tiles_r = (g.m + 63) / 64;
+    b.X = g.B; b.ld = g.ldb; b.row_k = !g.tb; b.rows = g.n; b.P = pb; b.tiles_r = (g.n + 63) / 64;
+    const int kt = (g.k + 63) / 64;
+    split_bf16x3<<<(unsigned)(kt * (a.tiles_r + b.tiles_r)), 256, 0, S(ctx)>>>(a, b, g.k, pitch, kt * a.tiles_r, flag,
+                                                                               tag);
+    StParams p{};
+    p.M = g.m; p.N = g.n;
+    p.nkb = (g.k + ST_BK - 1) / ST_BK;
+    p.tiles_m = (g.m + ST_T - 1) / ST_T;
+    p.tiles_n = (g.n + ST_T - 1) / ST_T;
+    p.chunk = p.nkb > 4 ? 2 : 1;
+    p.alpha = g.alpha; p.beta = g.beta;
+    p.C = g.C; p.ldc = g.ldc;
+    p.flag = flag; p.tag = tag;
+    p.status = words + 4;
+    p.status_host = mirror;
+    // a per-device function attribute; setting it is a cheap host call
+    if (cudaFuncSetAttribute(sgemm_bf16x3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ST_SMEM) != cudaSuccess)
+        return gbx_fail(ctx, GBX_ERR_CUDA, "%s: shared memory attribute", what);
+    const int grid = std::min(p.tiles_m * p.tiles_n, gbx_ctx_sms(ctx));
+    gbx_timer_begin(ctx, GBX_TIMER_GEMM_FP64);
+    sgemm_bf16x3<<<grid, ST_THREADS, ST_SMEM, S(ctx)>>>(tmA, tmB, p);
+    gbx_timer_end(ctx);
+    gbx_count_launch(ctx, 2);
+    gbx_status st = gbx_check_launch(ctx, what);
+    if (st != GBX_OK) return st;
+    return launch_gemm_if(ctx, g, what, flag, tag);
+}
+
 }  // namespace
 
 // Whether an m x n x k product is faster on the tensor cores than on the SIMT
@@ -467,6 +520,14 @@ gbx_status sgemm_tensor(gbx_ctx *ctx, const GemmArgs<float> &g, const char *what
 {
     *done = false;
     if (!gbx_sgemm_tensor_choice(g.m, g.n, g.k, gbx_ctx_sms(ctx))) return GBX_OK;
+    // A capture gets the SIMT core: its replays outlive this call, may run on any
+    // stream, and must not use scratch that other calls use too.
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(S(ctx), &cap) != cudaSuccess) {
+        cudaGetLastError();
+        return GBX_OK;
+    }
+    if (cap != cudaStreamCaptureStatusNone) return GBX_OK;
     size_t a_bytes;
     const size_t planes = st_plane_bytes(g.m, g.n, g.k, &a_bytes);
     if (planes > ST_WS_MAX) {
@@ -495,53 +556,17 @@ gbx_status sgemm_tensor(gbx_ctx *ctx, const GemmArgs<float> &g, const char *what
         *done = true;
         return GBX_OK;
     }
-    // workspace: 256 bytes of flag, then the planes; without it (no memory, or
-    // a capture that must not allocate) the SIMT core takes the call
-    void *ws;
     int *words, *mirror;
-    if (!gbx_ws_ready(ctx, GBX_WS_SGEMM, 256 + planes)) {
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(S(ctx), &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return GBX_OK;
-    }
-    if (gbx_ws(ctx, GBX_WS_SGEMM, 256 + planes, &ws) != GBX_OK) return GBX_OK;
     if (gbx_ctx_status(ctx, &words, &mirror) != GBX_OK) return GBX_OK;
-    const long long pitch = ((long long)g.k + 7) / 8 * 8;
-    __nv_bfloat16 *pa = (__nv_bfloat16 *)((char *)ws + 256), *pb = (__nv_bfloat16 *)((char *)ws + 256 + a_bytes);
-    CUtensorMap tmA, tmB;
-    if (!plane_map(&tmA, pa, g.m, g.k, pitch, 1) || !plane_map(&tmB, pb, g.n, g.k, pitch, 3))
-        return gbx_fail(ctx, GBX_ERR_CUDA, "%s: cuTensorMapEncodeTiled failed", what);
+    // 256 bytes of flag, then the planes; where they cannot be had the SIMT core
+    // takes the call
+    void *ws;
+    int block;
+    if (gbx_scratch_get(ctx, 256 + planes, &ws, &block) != GBX_OK) return GBX_OK;
     *done = true;
-    int *flag = (int *)ws;
-    const int epoch = gbx_ctx_epoch(ctx);
-
-    SplitOp a{}, b{};
-    a.X = g.A; a.ld = g.lda; a.row_k = g.ta; a.rows = g.m; a.P = pa; a.tiles_r = (g.m + 63) / 64;
-    b.X = g.B; b.ld = g.ldb; b.row_k = !g.tb; b.rows = g.n; b.P = pb; b.tiles_r = (g.n + 63) / 64;
-    const int kt = (g.k + 63) / 64;
-    split_bf16x3<<<(unsigned)(kt * (a.tiles_r + b.tiles_r)), 256, 0, S(ctx)>>>(a, b, g.k, pitch, kt * a.tiles_r, flag,
-                                                                               epoch);
-    StParams p{};
-    p.M = g.m; p.N = g.n;
-    p.nkb = (g.k + ST_BK - 1) / ST_BK;
-    p.tiles_m = (g.m + ST_T - 1) / ST_T;
-    p.tiles_n = (g.n + ST_T - 1) / ST_T;
-    p.chunk = p.nkb > 4 ? 2 : 1;
-    p.alpha = g.alpha; p.beta = g.beta;
-    p.C = g.C; p.ldc = g.ldc;
-    p.flag = flag; p.epoch = epoch;
-    p.status = words + 4;
-    p.status_host = mirror;
-    // a per-device function attribute; setting it is a cheap host call
-    if (cudaFuncSetAttribute(sgemm_bf16x3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ST_SMEM) != cudaSuccess)
-        return gbx_fail(ctx, GBX_ERR_CUDA, "%s: shared memory attribute", what);
-    const int grid = std::min(p.tiles_m * p.tiles_n, gbx_ctx_sms(ctx));
-    gbx_timer_begin(ctx, GBX_TIMER_GEMM_FP64);
-    sgemm_bf16x3<<<grid, ST_THREADS, ST_SMEM, S(ctx)>>>(tmA, tmB, p);
-    gbx_timer_end(ctx);
-    gbx_count_launch(ctx, 2);
-    gbx_status st = gbx_check_launch(ctx, what);
-    if (st != GBX_OK) return st;
-    return launch_gemm_if(ctx, g, what, flag, epoch);
+    const gbx_status st = run_planes(ctx, g, what, (char *)ws, a_bytes, words, mirror);
+    const gbx_status put = gbx_scratch_put(ctx, block);
+    return st != GBX_OK ? st : put;
 }
 
 }  // namespace gbx_gemm
