@@ -44,6 +44,11 @@ gbx_status gbx_ws(gbx_ctx *ctx, int slot, size_t bytes, void **ptr);
  * stream that is being captured. */
 gbx_status gbx_scratch_get(gbx_ctx *ctx, size_t bytes, void **ptr, int *block);
 gbx_status gbx_scratch_put(gbx_ctx *ctx, int block);
+/* What a one-launch reduction on the context's stream uses besides its partials
+ * (part_bytes of them, the same in every call): the counter of finished blocks and,
+ * unless null, where its last block writes seq at its end. */
+typedef struct gbx_red { unsigned *counter, *done; unsigned seq; } gbx_red;
+gbx_status gbx_reduction(gbx_ctx *ctx, size_t part_bytes, void **part, gbx_red *red);
 /* Pinned host scratch owned by the context (for small results). */
 gbx_status gbx_pinned(gbx_ctx *ctx, size_t bytes, void **ptr);
 void gbx_count_launch(gbx_ctx *ctx, int n);
@@ -55,9 +60,8 @@ void gbx_timer_end(gbx_ctx *ctx);
  * mapped host mirror, which such kernels set to the status when it is
  * nonzero as they finish.  gbx_ctx_sync reports a nonzero mirror (5: a
  * non-finite Ozaki operand, GBX_ERR_ARG; else GBX_ERR_TIMEOUT) and clears
- * both.  Word 0 is the status, word 4 that of the SGEMM tensor kernel; words
- * 8 and 12 are last-CTA counters (reductions, the DPOTRF step), which the
- * kernels that use them reset. */
+ * both.  Word 0 is the status, word 4 that of the SGEMM tensor kernel; word
+ * 12 is the last-CTA counter of the DPOTRF step, which resets it. */
 gbx_status gbx_ctx_status(gbx_ctx *ctx, int **dev_status, int **host_mirror);
 /* Check cudaGetLastError after a launch, record and map it. */
 gbx_status gbx_check_launch(gbx_ctx *ctx, const char *what);

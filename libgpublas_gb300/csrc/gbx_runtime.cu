@@ -42,6 +42,15 @@ struct gbx_scratch {
     uint64_t used;               // number of that use
 };
 
+// What a stream's one-launch reductions use (gbx_reduction).
+#define GBX_RED_STREAMS 16
+#define GBX_RED_CAPTURED 4096
+struct gbx_red_stream {
+    unsigned long long id;       // of the stream
+    unsigned seq;                // number of its last reduction (0: the entry is unused)
+    uint64_t used;
+};
+
 struct gbx_ctx {
     int device;
     int sms;
@@ -51,6 +60,11 @@ struct gbx_ctx {
     size_t ws_bytes[GBX_WS_SLOTS];
     gbx_scratch scratch[GBX_SCRATCH_BLOCKS];
     uint64_t scratch_uses;
+    gbx_red_stream red[GBX_RED_STREAMS];
+    uint64_t red_uses;
+    int red_captured;              // counters given to captured reductions
+    volatile unsigned *red_done;   // mapped: per entry, the number of the last reduction that ended
+    unsigned *red_done_dev;        // its device address
     void  *pinned;
     size_t pinned_bytes;
     uint64_t launches;
@@ -209,6 +223,7 @@ extern "C" gbx_status gbx_ctx_destroy(gbx_ctx *c)
         if (b.p) cudaFree(b.p);
         cudaEventDestroy(b.done);
     }
+    if (c->red_done) cudaFreeHost((void *)c->red_done);
     if (c->pinned) cudaFreeHost(c->pinned);
     if (c->status_dev) cudaFree(c->status_dev);
     if (c->status_host) cudaFreeHost(c->status_host);
@@ -440,6 +455,83 @@ extern "C" gbx_status gbx_scratch_put(gbx_ctx *c, int block)
 {
     const cudaError_t e = cudaEventRecord(c->scratch[block].done, c->stream);
     return e == cudaSuccess ? GBX_OK : gbx_fail(c, GBX_ERR_CUDA, "scratch: %s", cudaGetErrorString(e));
+}
+
+// State of a one-launch reduction: the blocks' partials, the count of finished
+// blocks (zero between launches) and where its last block writes seq.  The
+// reductions of one stream run in turn and share an entry; another stream has
+// another, the entry of a stream whose last reduction has ended if none is unused.
+// A count shared by launches that overlap could stay nonzero for good, and every
+// later reduction would end too early or never.  So a captured reduction, whose
+// replays may overlap anything, has a counter that no other launch uses: the count
+// wraps at the grid's size, whatever its own replays do.  (Captured reductions of
+// one context share their partials, as calls on several streams did when there was
+// one array for all: their replays must not overlap.)
+extern "C" gbx_status gbx_reduction(gbx_ctx *c, size_t part_bytes, void **part, gbx_red *red)
+{
+    part_bytes = (part_bytes + 255) & ~(size_t)255;   // the same in every call
+    const size_t counters = part_bytes * (GBX_RED_STREAMS + 1);
+    const size_t count = GBX_RED_STREAMS + GBX_RED_CAPTURED;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    cudaError_t e = cudaStreamIsCapturing(c->stream, &cap);
+    if (e == cudaSuccess && cap == cudaStreamCaptureStatusNone) e = cudaStreamGetId(c->stream, &id);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return gbx_fail(c, GBX_ERR_CUDA, "reduction: %s", cudaGetErrorString(e));
+    }
+    char *base;
+    gbx_status st = gbx_ws(c, GBX_WS_RED, counters + sizeof(unsigned) * count, (void **)&base);
+    if (st != GBX_OK) return st;
+    if (!c->red_done) {
+        void *h = nullptr;
+        e = cudaMemsetAsync(base + counters, 0, sizeof(unsigned) * count, c->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+        if (e == cudaSuccess) e = cudaHostAlloc(&h, sizeof(unsigned) * GBX_RED_STREAMS, cudaHostAllocMapped);
+        if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&c->red_done_dev, h, 0);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            if (h) cudaFreeHost(h);
+            return gbx_fail(c, GBX_ERR_ALLOC, "reduction: %s", cudaGetErrorString(e));
+        }
+        memset(h, 0, sizeof(unsigned) * GBX_RED_STREAMS);
+        c->red_done = (volatile unsigned *)h;
+    }
+    red->done = nullptr;
+    red->seq = 0;
+    if (cap != cudaStreamCaptureStatusNone) {
+        *part = base + part_bytes * GBX_RED_STREAMS;
+        const bool fresh = c->red_captured < GBX_RED_CAPTURED - 1;
+        red->counter = (unsigned *)(base + counters) + GBX_RED_STREAMS + c->red_captured;
+        if (fresh) c->red_captured++;
+        else if (cudaMemsetAsync(red->counter, 0, sizeof(unsigned), c->stream) != cudaSuccess)   // the last one, cleared
+            return gbx_check_launch(c, "reduction counter");
+        return GBX_OK;
+    }
+    int pick = -1, oldest = 0;
+    for (int i = 0; i < GBX_RED_STREAMS; i++) {
+        const gbx_red_stream &r = c->red[i];
+        if (r.seq && r.id == id) {
+            pick = i;
+            break;
+        }
+        if (pick < 0 && c->red_done[i] == r.seq) pick = i;   // unused, or ended
+        if (r.used < c->red[oldest].used) oldest = i;
+    }
+    if (pick < 0) {
+        e = cudaDeviceSynchronize();   // reductions in flight on as many streams as there are entries
+        if (e != cudaSuccess) return gbx_fail(c, GBX_ERR_CUDA, "reduction: %s", cudaGetErrorString(e));
+        pick = oldest;
+    }
+    gbx_red_stream &r = c->red[pick];
+    r.id = id;
+    r.used = ++c->red_uses;
+    if (++r.seq == 0) r.seq = 1;
+    *part = base + part_bytes * pick;
+    red->counter = (unsigned *)(base + counters) + pick;
+    red->done = c->red_done_dev + pick;
+    red->seq = r.seq;
+    return GBX_OK;
 }
 
 extern "C" gbx_status gbx_ctx_reserve(gbx_ctx *c, size_t bytes)

@@ -35,16 +35,15 @@ inline cudaStream_t S(gbx_ctx *ctx) { return (cudaStream_t)gbx_ctx_get_stream(ct
 // vector of 10,000 on five of them).  Long vectors fill the grid either way.
 constexpr int RED_PER_THREAD = 2;
 
-// Workspace of a reduction: the blocks' partials and the count of finished
-// blocks (a status word, zero between launches).
+// Partials (at most three values per block) and counter of a reduction.  One block
+// needs neither.
 template <typename P>
-gbx_status reduction_ws(gbx_ctx *ctx, size_t bytes, P **part, unsigned **counter)
+gbx_status reduction_ws(gbx_ctx *ctx, int g, P **part, gbx_red *red)
 {
-    int *words, *mirror;
-    gbx_status st = gbx_ws(ctx, GBX_WS_RED, bytes, (void **)part);
-    if (st == GBX_OK) st = gbx_ctx_status(ctx, &words, &mirror);
-    if (st == GBX_OK) *counter = (unsigned *)(words + 8);
-    return st;
+    *part = nullptr;
+    *red = gbx_red{};
+    if (g == 1) return GBX_OK;
+    return gbx_reduction(ctx, 3 * sizeof(double) * (size_t)gbx_ctx_sms(ctx) * L1_BLOCKS_PER_SM, (void **)part, red);
 }
 
 // element offset of the first element a kernel should touch: netlib walks a
@@ -92,12 +91,11 @@ extern "C" gbx_status gbx_ddot(gbx_ctx *ctx, int n, const double *x, int incx,
     }
     const int g = grid_for(ctx, n, RED_PER_THREAD);
     double *part;
-    unsigned *counter;
-    gbx_status st = reduction_ws(ctx, sizeof(double) * (size_t)g, &part, &counter);
+    gbx_red red;
+    gbx_status st = reduction_ws(ctx, g, &part, &red);
     if (st != GBX_OK) return st;
     gbx_timer_begin(ctx, GBX_TIMER_LEVEL1);
-    launch_pdl(dot_kernel, g, L1_THREADS, 0, S(ctx), n, x + base_off(n, incx), incx, y + base_off(n, incy), incy, part, counter,
-                                             res);
+    launch_pdl(dot_kernel, g, L1_THREADS, 0, S(ctx), n, x + base_off(n, incx), incx, y + base_off(n, incy), incy, part, red, res);
     gbx_timer_end(ctx);
     gbx_count_launch(ctx, 1);
     return gbx_check_launch(ctx, "ddot");
@@ -113,11 +111,11 @@ extern "C" gbx_status gbx_dnrm2(gbx_ctx *ctx, int n, const double *x, int incx, 
     }
     const int g = grid_for(ctx, n, RED_PER_THREAD);
     double *part;
-    unsigned *counter;
-    gbx_status st = reduction_ws(ctx, 3 * sizeof(double) * (size_t)g, &part, &counter);
+    gbx_red red;
+    gbx_status st = reduction_ws(ctx, g, &part, &red);
     if (st != GBX_OK) return st;
     gbx_timer_begin(ctx, GBX_TIMER_LEVEL1);
-    launch_pdl(nrm2_kernel, g, L1_THREADS, 0, S(ctx), n, x, incx, part, counter, res);
+    launch_pdl(nrm2_kernel, g, L1_THREADS, 0, S(ctx), n, x, incx, part, red, res);
     gbx_timer_end(ctx);
     gbx_count_launch(ctx, 1);
     return gbx_check_launch(ctx, "dnrm2");
@@ -133,13 +131,13 @@ static gbx_status iamax_common(gbx_ctx *ctx, int n, const double *x, int incx, i
     }
     const int g = grid_for(ctx, n, RED_PER_THREAD);
     unsigned long long *keys;
-    unsigned *counter;
-    gbx_status st = reduction_ws(ctx, 2 * sizeof(unsigned long long) * (size_t)g, &keys, &counter);
+    gbx_red red;
+    gbx_status st = reduction_ws(ctx, g, &keys, &red);
     if (st != GBX_OK) return st;
-    long long *idx = (long long *)(keys + g);
+    long long *idx = g > 1 ? (long long *)(keys + g) : nullptr;
     gbx_timer_begin(ctx, GBX_TIMER_LEVEL1);
-    if (is_min) launch_pdl(iamax_kernel<true>, g, L1_THREADS, 0, S(ctx), n, x, incx, keys, idx, counter, res);
-    else launch_pdl(iamax_kernel<false>, g, L1_THREADS, 0, S(ctx), n, x, incx, keys, idx, counter, res);
+    if (is_min) launch_pdl(iamax_kernel<true>, g, L1_THREADS, 0, S(ctx), n, x, incx, keys, idx, red, res);
+    else launch_pdl(iamax_kernel<false>, g, L1_THREADS, 0, S(ctx), n, x, incx, keys, idx, red, res);
     gbx_timer_end(ctx);
     gbx_count_launch(ctx, 1);
     return gbx_check_launch(ctx, is_min ? "idamin" : "idamax");

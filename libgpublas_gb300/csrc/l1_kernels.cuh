@@ -1,6 +1,7 @@
 // l1_kernels.cuh — device code of the Level-1 routines (included by l1.cu).
 #pragma once
 
+#include "gbx_internal.h"
 #include "launch.cuh"
 
 #include <cuda_runtime.h>
@@ -69,19 +70,23 @@ __device__ __forceinline__ void block_sum3(double &a, double &b, double &c)
 // Second half of a reduction in the same launch: true in every thread of the
 // block that finishes last, once the partials that the blocks' threads 0 wrote
 // before the call can be read (with __ldcg).  The counter is zero before the
-// launch and again after it.  A second launch cost 2 to 4 us a call, as much as
-// a short vector's whole first pass.
-__device__ __forceinline__ bool last_block(unsigned *counter)
+// launch and again after it (it wraps).  A second launch cost 2 to 4 us a call, as
+// much as a short vector's whole first pass.
+__device__ __forceinline__ bool last_block(const gbx_red &red)
 {
     __shared__ unsigned s_last;
     if (threadIdx.x == 0) {
         __threadfence();
-        s_last = atomicAdd(counter, 1u) == gridDim.x - 1;
-        if (s_last) *counter = 0u;
+        s_last = atomicInc(red.counter, gridDim.x - 1) == gridDim.x - 1;
         __threadfence();
     }
     __syncthreads();
     return s_last != 0u;
+}
+// By one thread of that block, after its last read of the partials.
+__device__ __forceinline__ void reduction_ended(const gbx_red &red)
+{
+    if (red.done) *(volatile unsigned *)red.done = red.seq;
 }
 
 // A plain load: the vectors may be results of the call before, which still runs
@@ -151,7 +156,7 @@ scal_kernel(int n, double a, double *__restrict__ x, int incx)
 // ----------------------------------------------------------------- ddot ---
 static __global__ void __launch_bounds__(L1_THREADS)
 dot_kernel(int n, const double *x, int incx, const double *y, int incy,
-           double *__restrict__ part, unsigned *counter, double *__restrict__ res)
+           double *__restrict__ part, gbx_red red, double *__restrict__ res)
 {
     gbx_launch::pdl_enter();
     const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -192,11 +197,14 @@ dot_kernel(int n, const double *x, int incx, const double *y, int incy,
         return;
     }
     if (threadIdx.x == 0) part[blockIdx.x] = b;
-    if (!last_block(counter)) return;
+    if (!last_block(red)) return;
     double s = 0.0;
     for (int i = threadIdx.x; i < (int)gridDim.x; i += L1_THREADS) s += __ldcg(part + i);
     b = block_sum(s);
-    if (threadIdx.x == 0) *res = b;
+    if (threadIdx.x == 0) {
+        *res = b;
+        reduction_ended(red);
+    }
 }
 
 // ---------------------------------------------------------------- dnrm2 ---
@@ -343,7 +351,7 @@ __device__ __forceinline__ double blue_finish(double asml, double amed, double a
 }
 
 static __global__ void __launch_bounds__(L1_THREADS)
-nrm2_kernel(int n, const double *x, int incx, double *__restrict__ part, unsigned *counter,
+nrm2_kernel(int n, const double *x, int incx, double *__restrict__ part, gbx_red red,
             double *__restrict__ res)
 {
     gbx_launch::pdl_enter();
@@ -393,7 +401,7 @@ nrm2_kernel(int n, const double *x, int incx, double *__restrict__ part, unsigne
             part[3 * blockIdx.x + 1] = amed;
             part[3 * blockIdx.x + 2] = abig;
         }
-        if (!last_block(counter)) return;
+        if (!last_block(red)) return;
         asml = amed = abig = 0.0;
         for (int i = threadIdx.x; i < (int)gridDim.x; i += L1_THREADS) {
             asml += __ldcg(part + 3 * i);
@@ -403,7 +411,10 @@ nrm2_kernel(int n, const double *x, int incx, double *__restrict__ part, unsigne
         if (__syncthreads_or(asml != 0.0 || abig != 0.0)) block_sum3(asml, amed, abig);
         else amed = block_sum(amed);
     }
-    if (threadIdx.x == 0) *res = blue_finish(asml, amed, abig);
+    if (threadIdx.x == 0) {
+        *res = blue_finish(asml, amed, abig);
+        reduction_ended(red);
+    }
 }
 
 // ------------------------------------------------------- idamax / idamin ---
@@ -456,7 +467,7 @@ __device__ __forceinline__ void block_best(unsigned long long &k, long long &i)
 template <bool IS_MIN>
 static __global__ void __launch_bounds__(L1_THREADS)
 iamax_kernel(int n, const double *x, int incx, unsigned long long *__restrict__ keys,
-             long long *__restrict__ idx, unsigned *counter, int *__restrict__ res)
+             long long *__restrict__ idx, gbx_red red, int *__restrict__ res)
 {
     gbx_launch::pdl_enter();
     const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -511,7 +522,7 @@ iamax_kernel(int n, const double *x, int incx, unsigned long long *__restrict__ 
     block_best(bk, bi);
     if (gridDim.x > 1) {
         if (threadIdx.x == 0) { keys[blockIdx.x] = bk; idx[blockIdx.x] = bi; }
-        if (!last_block(counter)) return;
+        if (!last_block(red)) return;
         bk = 0ull;
         bi = 0x7fffffffffffffffll;
         for (int i = threadIdx.x; i < (int)gridDim.x; i += L1_THREADS) {
@@ -522,7 +533,10 @@ iamax_kernel(int n, const double *x, int incx, unsigned long long *__restrict__ 
         block_best(bk, bi);
     }
     // x_1 NaN: netlib returns 1
-    if (threadIdx.x == 0) *res = abs_bits(x[0]) > 0x7FF0000000000000ull ? 1 : (int)(bi + 1);
+    if (threadIdx.x == 0) {
+        *res = abs_bits(x[0]) > 0x7FF0000000000000ull ? 1 : (int)(bi + 1);
+        reduction_ended(red);
+    }
 }
 
 }  // namespace gbx_l1
