@@ -44,7 +44,7 @@ struct gbx_scratch {
 
 // What a stream's one-launch reductions use (gbx_reduction).
 #define GBX_RED_STREAMS 16
-#define GBX_RED_CAPTURED 4096
+#define GBX_RED_CAPTURED 16384
 struct gbx_red_stream {
     unsigned long long id;       // of the stream
     unsigned seq;                // number of its last reduction (0: the entry is unused)

@@ -89,9 +89,11 @@ __device__ __forceinline__ void reduction_ended(const gbx_red &red)
     if (red.done) *(volatile unsigned *)red.done = red.seq;
 }
 
-// A plain load: the vectors may be results of the call before, which still runs
-// when the CTA is placed, so loads through the non-coherent path are not for them.
-__device__ __forceinline__ double2 ldg2(const double2 *p) { return *p; }
+// A load from L2: the vectors may be results of the call before, which still runs
+// when the CTA is placed, so loads through the non-coherent path are not for them,
+// and an ordinary one also allocates a line in L1 that nobody reads again (DDOT of
+// 2^26 elements: 162 us so, 153 now, as with the non-coherent load).
+__device__ __forceinline__ double2 load2(const double2 *p) { return __ldcg(p); }
 
 static __global__ void zero_result(double *res) { *res = 0.0; }
 static __global__ void zero_index(int *res) { *res = 0; }
@@ -115,14 +117,14 @@ axpy_unit(int n, double a, const double *x, double *__restrict__ y)
         double2 *y2 = (double2 *)(y + peel);
         long long i = tid;
         for (; i + stride < n2; i += 2 * stride) {
-            double2 xa = ldg2(x2 + i), xb = ldg2(x2 + i + stride);
+            double2 xa = load2(x2 + i), xb = load2(x2 + i + stride);
             double2 ya = y2[i], yb = y2[i + stride];
             ya.x = fma(a, xa.x, ya.x); ya.y = fma(a, xa.y, ya.y);
             yb.x = fma(a, xb.x, yb.x); yb.y = fma(a, xb.y, yb.y);
             y2[i] = ya; y2[i + stride] = yb;
         }
         for (; i < n2; i += stride) {
-            double2 xa = ldg2(x2 + i), ya = y2[i];
+            double2 xa = load2(x2 + i), ya = y2[i];
             ya.x = fma(a, xa.x, ya.x); ya.y = fma(a, xa.y, ya.y);
             y2[i] = ya;
         }
@@ -154,7 +156,7 @@ scal_kernel(int n, double a, double *__restrict__ x, int incx)
 }
 
 // ----------------------------------------------------------------- ddot ---
-static __global__ void __launch_bounds__(L1_THREADS)
+static __global__ void __launch_bounds__(L1_THREADS, L1_BLOCKS_PER_SM)
 dot_kernel(int n, const double *x, int incx, const double *y, int incy,
            double *__restrict__ part, gbx_red red, double *__restrict__ res)
 {
@@ -169,22 +171,23 @@ dot_kernel(int n, const double *x, int incx, const double *y, int incy,
         const long long n2 = (long long)(n - peel) >> 1;
         const double2 *x2 = (const double2 *)(x + peel), *y2 = (const double2 *)(y + peel);
         long long i = tid;
-        // eight 128-bit loads in flight per thread
-        for (; i + 3 * stride < n2; i += 4 * stride) {
-            double2 xv[4], yv[4];
+        // four 128-bit loads in flight per thread; eight cost the registers of the
+        // SM's third and fourth CTA (10^6 elements 9.7 us, with four 8.1)
+        for (; i + stride < n2; i += 2 * stride) {
+            double2 xv[2], yv[2];
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-                xv[u] = ldg2(x2 + i + u * stride);
-                yv[u] = ldg2(y2 + i + u * stride);
+            for (int u = 0; u < 2; u++) {
+                xv[u] = load2(x2 + i + u * stride);
+                yv[u] = load2(y2 + i + u * stride);
             }
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
+            for (int u = 0; u < 2; u++) {
                 s0 = fma(xv[u].x, yv[u].x, s0);
                 s1 = fma(xv[u].y, yv[u].y, s1);
             }
         }
         for (; i < n2; i += stride) {
-            double2 xa = ldg2(x2 + i), ya = ldg2(y2 + i);
+            double2 xa = load2(x2 + i), ya = load2(y2 + i);
             s0 = fma(xa.x, ya.x, s0); s1 = fma(xa.y, ya.y, s1);
         }
         if (((n - peel) & 1) && tid == 0) s1 = fma(x[n - 1], y[n - 1], s1);
@@ -368,7 +371,7 @@ nrm2_kernel(int n, const double *x, int incx, double *__restrict__ part, gbx_red
         SqFix fx;
         fx.init();
         for (; i + stride < n2; i += 2 * stride) {
-            double2 a = ldg2(x2 + i), b = ldg2(x2 + i + stride);
+            double2 a = load2(x2 + i), b = load2(x2 + i + stride);
             if (all_medium4(a.x, a.y, b.x, b.y)) {
                 // three squares on the FP64 pipe, the fourth on the integer pipe
                 amed = fma(a.x, a.x, amed);
@@ -384,7 +387,7 @@ nrm2_kernel(int n, const double *x, int incx, double *__restrict__ part, gbx_red
         amed += ((m1 + m2) + m3) + fx.value();
         abig += (b1 + b2) + b3;
         for (; i < n2; i += stride) {
-            double2 a = ldg2(x2 + i);
+            double2 a = load2(x2 + i);
             blue_acc(a.x, asml, amed, abig); blue_acc(a.y, asml, amed, abig);
         }
         if ((n & 1) && tid == 0) blue_acc(x[n - 1], asml, amed, abig);
@@ -483,7 +486,7 @@ iamax_kernel(int n, const double *x, int incx, unsigned long long *__restrict__ 
         for (; i + 3 * stride < n2; i += 4 * stride) {
             double2 v[4];
 #pragma unroll
-            for (int u = 0; u < 4; u++) v[u] = ldg2(x2 + i + u * stride);
+            for (int u = 0; u < 4; u++) v[u] = load2(x2 + i + u * stride);
             // pairwise tree over the 8 elements (short dependency chains),
             // then one merge into the running best; ties resolve to the
             // smaller index at every level
@@ -504,7 +507,7 @@ iamax_kernel(int n, const double *x, int incx, unsigned long long *__restrict__ 
             if (better(k[0], e[0], bk, bi)) { bk = k[0]; bi = e[0]; }
         }
         for (; i < n2; i += stride) {
-            double2 v = ldg2(x2 + i);
+            double2 v = load2(x2 + i);
             unsigned long long k0 = amax_key<IS_MIN>(v.x), k1 = amax_key<IS_MIN>(v.y);
             if (better(k0, 2 * i, bk, bi)) { bk = k0; bi = 2 * i; }
             if (better(k1, 2 * i + 1, bk, bi)) { bk = k1; bi = 2 * i + 1; }

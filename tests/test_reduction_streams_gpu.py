@@ -108,22 +108,22 @@ def test_replays_beside_other_calls(own):
 
 
 def test_more_captured_calls_than_counters(own):
-    """The context has 4096 counters for captured reductions."""
+    """The context has 16384 counters for captured reductions."""
     import torch
     v = Vectors()
     n = SIZES[1]
     ref = v.alone(own)[1]
     st = torch.cuda.Stream()
-    f = torch.zeros(4200, dtype=torch.float64, device="cuda")
+    f = torch.zeros(16500, dtype=torch.float64, device="cuda")
     torch.cuda.synchronize()
     own.set_stream(st.cuda_stream)
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph, stream=st):
-        for r in range(4200):
+        for r in range(16500):
             own.ddot(n, v.x, 1, v.y, 1, f[r:])
     for _ in range(2):
         f.fill_(float("nan"))
         torch.cuda.synchronize()
         graph.replay()
         torch.cuda.synchronize()
-        assert torch.equal(f, ref[0][:1].expand(4200))
+        assert torch.equal(f, ref[0][:1].expand(16500))
