@@ -222,7 +222,7 @@ struct TrsvArgs {
     double *xw;         // solution in solve order, nblk * 64 values, all bits set until known
     double *zw;         // b - (the blocks subtracted one by one), likewise
     double *inv;        // inverted diagonal blocks, element (i, k) at [64 k + i]
-    int *ready;         // per block: all bits set until its inverse is there
+    int *ready;         // per block: all bits set until its inverse is there, then 1 if M may be used, else 0
     int *status, *status_host;
 };
 
@@ -342,17 +342,19 @@ __device__ __forceinline__ void tv_publish(double *p, double r)
 }
 
 // Waits for the inverse of block s and starts the copy of the slice's rows of
-// it to dst[k * 17 + i]; by the whole CTA.
-__device__ __forceinline__ void tv_fetch_inv(const TrsvArgs &a, double *dst, int s, int sl)
+// it to dst[k * 17 + i], *fold: M may be used for it; by the whole CTA.
+__device__ __forceinline__ void tv_fetch_inv(const TrsvArgs &a, double *dst, int s, int sl, int *fold)
 {
     const int tid = threadIdx.x;
     if (tid == 0) {
         const unsigned long long t0 = tv_now();
-        while (*(volatile int *)(a.ready + s) != 0)
+        int r;
+        while ((r = *(volatile int *)(a.ready + s)) < 0)
             if (tv_now() - t0 > TV_TIMEOUT_NS) {
                 tv_timeout(a);
                 break;
             }
+        *fold = r > 0;
         __threadfence();
     }
     __syncthreads();
@@ -362,6 +364,40 @@ __device__ __forceinline__ void tv_fetch_inv(const TrsvArgs &a, double *dst, int
         const int k = (tid >> 4) + 16 * u;
         tv_copy8(dst + k * TV_RLD + (tid & 15), src + k * TV_NB, 1);
     }
+}
+
+// |x| as a float, to 21 bits; at least 2^-126 unless zero, infinite beyond the FP32
+// range and for NaN.  On the integer pipe: a conversion is an FP64 instruction.
+__device__ __forceinline__ float tv_absf(double x)
+{
+    const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
+    if (h < 0x38100000u) return h ? 0x1p-126f : 0.0f;
+    return __uint_as_float(h < 0x47f00000u ? (h - 0x38000000u) << 3 : 0x7f800000u);
+}
+
+// Whether M = X T(s, s-1) may be formed for a block D with inverse X: the condition
+// number of D, the largest row sum of |X| |D|, is at most 16.  X times the
+// right-hand side is then as good as substitution; but x_s = X (b - sum) - M x
+// multiplies b - sum and T x by X before they cancel, and its backward error grows
+// with the condition number (measured against the form without M, 400 triangles: up
+// to 16 both stay below 2 u; at 16-64 20 times as much, at 1e7 400 times).  By
+// the whole CTA; r: 64 floats, the answer in the first warp.
+__device__ __forceinline__ bool tv_may_fold(const double *D, const double *X, float *r)
+{
+    const int i = threadIdx.x >> 2, q = threadIdx.x & 3;
+    float v = 0.0f;
+#pragma unroll 4
+    for (int k = q; k <= i; k += 4) v += tv_absf(D[k * TV_LD + i]);
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    if (q == 0) r[i] = v;
+    __syncthreads();
+    v = 0.0f;
+#pragma unroll 4
+    for (int k = q; k <= i; k += 4) v = fmaf(tv_absf(X[k * TV_LD + i]), r[k], v);
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    return __syncthreads_and(v <= 16.0f);   // (a NaN is not)
 }
 
 // Sum over the CTA of the 16 values that its threads (row lane & 15, columns
@@ -393,9 +429,10 @@ __device__ __forceinline__ double tv_sum(double *red, double v, int lane, int wa
 //     its own ring (they do not depend on x), without barriers.
 //   * The four slices exchange z = b - sum through zw; x_s = inv z goes to the
 //     later blocks through xw and to x.
-//   * From block TV_FOLD on M = inv T(s, s-1) is formed beforehand, so that
-//     x_s = inv (b - sum over K < s-1) - M x_(s-1): the exchange and the
-//     inverse lie before x_(s-1), which needs one product.
+//   * From block TV_FOLD on, for well-conditioned diagonal blocks (tv_may_fold), M =
+//     inv T(s, s-1) is formed beforehand, so that x_s = inv (b - sum over K < s-1) -
+//     M x_(s-1): the exchange and the inverse lie before x_(s-1), which needs one
+//     product.
 // What bounds it: the chain over the blocks, each link one hand-over through
 // L2 and the product with x_(s-1), 1.2 us; for the last blocks the FP64 pipe,
 // which takes 0.33 us for each 16 x 64 part and 11 us for M.  (With a block per
@@ -408,6 +445,7 @@ __global__ void __launch_bounds__(TV_THREADS)
 trsv_solve(TrsvArgs a)
 {
     extern __shared__ __align__(16) double tv_sm[];
+    __shared__ int s_fold[2];
     double *T1 = tv_sm;                              // T(s, s-1)
     double *work = T1 + TV_TILE;                     // to invert a block
     double *Ia = work;                               // the slice's rows of the inverse, [k * 17 + i]: two
@@ -437,19 +475,20 @@ trsv_solve(TrsvArgs a)
             asm volatile("cp.async.wait_all;" ::: "memory");
             __syncthreads();
             gbx_tri::invert64(D, X, X + TV_TILE);
+            const int may = ib >= TV_FOLD && tv_may_fold(D, X, (float *)(X + TV_TILE));   // (uniform)
             double *o = a.inv + (size_t)ib * TV_NB * TV_NB;
             for (int e = tid; e < TV_NB * TV_NB; e += TV_THREADS) o[e] = X[(e >> 6) * TV_LD + (e & 63)];
             __threadfence();
             __syncthreads();
-            if (tid == 0) *(volatile int *)(a.ready + ib) = 0;
+            if (tid == 0) *(volatile int *)(a.ready + ib) = may;
         }
         const int s = t / TV_SL, sl = t % TV_SL;
         const int row = s * TV_NB + tv_row(sl, r16);
-        const bool fold = s >= TV_FOLD;
         double *I = Ia + (round & 1) * TV_NB * TV_RLD;
-        if (fold && round == 0) tv_fetch(a, T1, s, s - 1);
-        if (round % TV_SL == 0) tv_fetch_inv(a, I, s, sl);
+        if (s >= TV_FOLD && round == 0) tv_fetch(a, T1, s, s - 1);
+        if (round % TV_SL == 0) tv_fetch_inv(a, I, s, sl, s_fold + (round & 1));
         asm volatile("cp.async.commit_group;" ::: "memory");
+        const bool fold = s >= TV_FOLD && s_fold[round & 1];   // the same in all slices of the block
         const int nk = fold ? s - 1 : s;                 // blocks subtracted one by one
         TvPart part(a, s, sl, 8 * warp, lane);
 #pragma unroll 1
@@ -487,7 +526,7 @@ trsv_solve(TrsvArgs a)
         const int sn = (t + gridDim.x) / TV_SL;          // the next slice's
         if (sn < a.nblk && sn >= TV_FOLD) tv_fetch(a, T1, sn, sn - 1);
         if (sn < a.nblk && (round + 1) % TV_SL != 0)
-            tv_fetch_inv(a, Ia + ((round + 1) & 1) * TV_NB * TV_RLD, sn, sl);
+            tv_fetch_inv(a, Ia + ((round + 1) & 1) * TV_NB * TV_RLD, sn, sl, s_fold + ((round + 1) & 1));
         asm volatile("cp.async.commit_group;" ::: "memory");
         // x of four blocks at a time: lane 8 u + c has column 8 warp + c of block 4 g + u
         const double *xp = a.xw + (lane >> 3) * TV_NB + 8 * warp + (lane & 7);
