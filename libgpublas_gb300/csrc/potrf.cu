@@ -31,7 +31,7 @@ constexpr int PR = 8;           // panel rows per CTA
 constexpr int PT_THREADS = 320;
 
 // 1 / d to within an ulp or two for a positive d: an approximate reciprocal y
-// and one step of Halley's third-order iteration, y (1 + e + e^2) with
+// and one step of Chebyshev's third-order iteration, y (1 + e + e^2) with
 // e = 1 - d y (e < 2^-18 leaves e^3 < 2^-54), three dependent FP64 operations
 // where a division takes a dozen (65 cycles each on this part).  Not for a d
 // whose reciprocal is near the ends of the range: its column is divided by d.
@@ -70,22 +70,26 @@ __device__ __noinline__ double potrf_ratio(double a, double d) { return a / d; }
 // four warps that passed column and reciprocal on barriers where everybody waits
 // for everybody (19 us a step, now 12; with a barrier of 256 threads and a
 // reciprocal square root per column it was 30).
-// A wait that did not end at once, out of line and bounded.
-__device__ __noinline__ void potrf_wait_long(uint64_t *bar, int *status)
+// A wait that did not end at once, out of line and bounded.  The arrival is that of
+// a warp of the same CTA, which comes whatever an earlier call has left in the
+// status word: only the deadline ends the wait, and sets *failed.
+__device__ __noinline__ void potrf_wait_long(uint64_t *bar, int *status, int *failed)
 {
-    gbx_tc::mbar_wait(bar, 0u, status, gbx_tc::TC_TIMEOUT_FULL);
+    if (!gbx_tc::mbar_wait_timed(bar, 0u, status, gbx_tc::TC_TIMEOUT_FULL)) *(volatile int *)failed = 1;
 }
 
 __global__ void __launch_bounds__(PT_THREADS)
-potrf_step(int n, int j0, double *__restrict__ A, long long lda, int *__restrict__ info, unsigned *done, int *status)
+potrf_step(int n, int j0, double *__restrict__ A, long long lda, int *__restrict__ info, unsigned *done, int *status,
+           int *status_host)
 {
     __shared__ double colA[PB][PB];   // column k, unscaled, once final
     __shared__ double colM[PB][PB];   // -(column k) / d_k
     __shared__ double colP[PB][PR];
     __shared__ double rec[PB];        // reciprocal (then reciprocal square root) of pivot k
     __shared__ __align__(8) uint64_t barM[PB];
-    __shared__ int s_last;
+    __shared__ int s_last, s_failed;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) s_failed = 0;
     if (tid < PB) gbx_tc::mbar_init(barM + tid, 1);
     __syncthreads();
     pdl_enter();
@@ -94,7 +98,7 @@ potrf_step(int n, int j0, double *__restrict__ A, long long lda, int *__restrict
     double *D = A + (long long)j0 * lda + j0;
     constexpr unsigned ALL = 0xffffffffu;
     auto wait = [&](uint64_t *bar) {
-        if (!gbx_tc::mbar_try_wait(bar, 0u)) potrf_wait_long(bar, status);
+        if (!gbx_tc::mbar_try_wait(bar, 0u)) potrf_wait_long(bar, status, &s_failed);
     };
     if (warp < 8) {
         const int row = 16 + (lane & 15), jb = 16 + warp + 8 * (lane >> 4);   // of ab
@@ -197,6 +201,13 @@ potrf_step(int n, int j0, double *__restrict__ A, long long lda, int *__restrict
         for (int q = 0; q < 4; q++) colP[pg + 8 * q][pr] = p[q];
     }
     __syncthreads();
+    if (s_failed) {   // uniform: nothing is stored, and the host is told
+        if (tid == 0) {
+            *(volatile int *)status_host = *(volatile int *)status;
+            __threadfence_system();
+        }
+        return;
+    }
     // 1-based column of the first non-positive pivot (zero, negative or NaN, by
     // the bit pattern), or 0; every warp gets the same answer
     const double d = colA[lane][lane];
@@ -264,7 +275,7 @@ extern "C" gbx_status gbx_dpotrf_small(gbx_ctx *ctx, char uplo, int n, double *A
         const int b = n - j0 < PB ? n - j0 : PB;
         const int rows = n - j0 - b;
         const int grid = rows > 0 ? (rows + PR - 1) / PR : 1;
-        launch_pdl(potrf_step, grid, PT_THREADS, 0, s, n, j0, A, lda, info, done, words);
+        launch_pdl(potrf_step, grid, PT_THREADS, 0, s, n, j0, A, lda, info, done, words, mirror);
         gbx_count_launch(ctx, 1);
         if ((st = gbx_check_launch(ctx, "dpotrf_small")) != GBX_OK) return st;
         if (rows > 0) {
