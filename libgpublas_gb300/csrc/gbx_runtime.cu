@@ -372,6 +372,14 @@ extern "C" gbx_status gbx_ws(gbx_ctx *c, int slot, size_t bytes, void **ptr)
                             cudaGetErrorString(e));
         }
         c->ws_bytes[slot] = want;
+        // a context with workspace has its status words too: a call that needs both
+        // can then be captured
+        if (!c->status_dev) {
+            int *words, *mirror;
+            const int armed = c->status_armed;
+            gbx_ctx_status(c, &words, &mirror);
+            c->status_armed = armed;
+        }
     }
     *ptr = c->ws[slot];
     return GBX_OK;

@@ -685,11 +685,12 @@ extern "C" gbx_status gbx_dtrsv(gbx_ctx *ctx, char uplo, char trans, char diag, 
     double *xw;
     TrsvArgs p{};
     gbx_status st;
-    // x and z in solve order and the blocks' ready words (eight bytes each)
+    // the inverses, then x and z in solve order and the blocks' ready words (eight
+    // bytes each): a slot that DTRSM of this order has used is large enough
+    const size_t ibytes = sizeof(double) * (size_t)nblk * TV_NB * TV_NB;
     const size_t wbytes = sizeof(double) * (size_t)nblk * (2 * TV_NB + 1);
-    if ((st = gbx_ws(ctx, GBX_WS_TMP1, sizeof(double) * (size_t)nblk * TV_NB * TV_NB, (void **)&p.inv)) != GBX_OK)
-        return st;
-    if ((st = gbx_ws(ctx, GBX_WS_TMP2, wbytes, (void **)&xw)) != GBX_OK) return st;
+    if ((st = gbx_ws(ctx, GBX_WS_TMP1, ibytes + wbytes, (void **)&p.inv)) != GBX_OK) return st;
+    xw = p.inv + ibytes / sizeof(double);
     if ((st = gbx_ctx_status(ctx, &p.status, &p.status_host)) != GBX_OK) return st;
     p.n = n;
     p.nblk = nblk;
