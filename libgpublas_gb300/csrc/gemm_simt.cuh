@@ -164,7 +164,7 @@ struct PanelLoader {
     static constexpr int PER = MN * BK / GEMM_THREADS;
     T r[PER];
 
-    __device__ __forceinline__ void load(const T *__restrict__ X, long long ld, bool contig_mn,
+    __device__ __forceinline__ void load(const T *X, long long ld, bool contig_mn,
                                          int mn0, int mn_lim, int k0, int k_lim, int conj, int tri,
                                          bool is_a, int sym)
     {
