@@ -59,14 +59,14 @@ template gbx_status scale_matrix<dcplx>(gbx_ctx *, int, int, dcplx, dcplx *, lon
 // The same kernel behind a device-side condition.
 template <typename T, int TM, int TN, int BK>
 __global__ void __launch_bounds__(GEMM_THREADS)
-gemm_simt_if(GemmArgs<T> p, const unsigned *flag, unsigned tag)
+gemm_simt_if(GemmArgs<T> p, const unsigned *marks, unsigned tag)
 {
-    if (*flag != tag) return;
+    if (!split_uncovered(marks, tag)) return;
     gemm_simt_tile<T, TM, TN, BK>(p, blockIdx.x);
 }
 
 template <typename T, int TM>
-gbx_status launch_gemm_tile(gbx_ctx *ctx, GemmArgs<T> p, const char *what, const unsigned *flag = nullptr,
+gbx_status launch_gemm_tile(gbx_ctx *ctx, GemmArgs<T> p, const char *what, const unsigned *marks = nullptr,
                             unsigned tag = 0)
 {
     constexpr int TN = TM, BK = TM == 1 ? 16 : 8;
@@ -81,8 +81,8 @@ gbx_status launch_gemm_tile(gbx_ctx *ctx, GemmArgs<T> p, const char *what, const
     }
     if (blocks > 0x7fffffffLL) return gbx_fail(ctx, GBX_ERR_UNSUPPORTED, "%s: grid too large", what);
     if constexpr (std::is_same<T, float>::value) {
-        if (flag) {
-            gemm_simt_if<T, TM, TN, BK><<<(unsigned)blocks, GEMM_THREADS, 0, S(ctx)>>>(p, flag, tag);
+        if (marks) {
+            gemm_simt_if<T, TM, TN, BK><<<(unsigned)blocks, GEMM_THREADS, 0, S(ctx)>>>(p, marks, tag);
             gbx_count_launch(ctx, 1);
             return gbx_check_launch(ctx, what);
         }
@@ -111,7 +111,7 @@ gbx_status launch_gemm_tile(gbx_ctx *ctx, GemmArgs<T> p, const char *what, const
 // operand reuse), 64x64 and 32x32 for complex double (its 8x8 register tile
 // would not fit), then smaller for the skinny and small products.
 template <typename T>
-static gbx_status choose_and_launch(gbx_ctx *ctx, GemmArgs<T> p, const char *what, const unsigned *flag, unsigned tag)
+static gbx_status choose_and_launch(gbx_ctx *ctx, GemmArgs<T> p, const char *what, const unsigned *marks, unsigned tag)
 {
     if (p.m <= 0 || p.n <= 0) return GBX_OK;
     const long long want = 2LL * gbx_ctx_sms(ctx);
@@ -132,15 +132,15 @@ static gbx_status choose_and_launch(gbx_ctx *ctx, GemmArgs<T> p, const char *wha
         return launch_gemm_tile<T, 1>(ctx, p, what);
     } else if constexpr (sizeof(T) <= 8) {
         if constexpr (std::is_same<T, float>::value) {
-            if (!flag && launch_gemm_short(ctx, p)) {
+            if (!marks && launch_gemm_short(ctx, p)) {
                 gbx_count_launch(ctx, 1);
                 return gbx_check_launch(ctx, what);
             }
         }
-        if (tiles(128) >= want) return launch_gemm_tile<T, 8>(ctx, p, what, flag, tag);
-        if (tiles(64) >= want) return launch_gemm_tile<T, 4>(ctx, p, what, flag, tag);
-        if (tiles(32) >= want) return launch_gemm_tile<T, 2>(ctx, p, what, flag, tag);
-        return launch_gemm_tile<T, 1>(ctx, p, what, flag, tag);
+        if (tiles(128) >= want) return launch_gemm_tile<T, 8>(ctx, p, what, marks, tag);
+        if (tiles(64) >= want) return launch_gemm_tile<T, 4>(ctx, p, what, marks, tag);
+        if (tiles(32) >= want) return launch_gemm_tile<T, 2>(ctx, p, what, marks, tag);
+        return launch_gemm_tile<T, 1>(ctx, p, what, marks, tag);
     } else {
         if (tiles(64) >= want) return launch_gemm_tile<T, 4>(ctx, p, what);
         return launch_gemm_tile<T, 2>(ctx, p, what);
@@ -151,9 +151,9 @@ gbx_status launch_gemm(gbx_ctx *ctx, GemmArgs<T> p, const char *what)
 {
     return choose_and_launch<T>(ctx, p, what, nullptr, 0);
 }
-gbx_status launch_gemm_if(gbx_ctx *ctx, GemmArgs<float> p, const char *what, const unsigned *flag, unsigned tag)
+gbx_status launch_gemm_if(gbx_ctx *ctx, GemmArgs<float> p, const char *what, const unsigned *marks, unsigned tag)
 {
-    return choose_and_launch<float>(ctx, p, what, flag, tag);
+    return choose_and_launch<float>(ctx, p, what, marks, tag);
 }
 template gbx_status launch_gemm<float>(gbx_ctx *, GemmArgs<float>, const char *);
 template gbx_status launch_gemm<double>(gbx_ctx *, GemmArgs<double>, const char *);

@@ -19,12 +19,17 @@
 // operands of one sign 3.9e-8 / 8.7e-8 / 1.7e-7 / 2.1e-7 (4.6e-8 / 2.2e-7 /
 // 8.5e-7 / 1.7e-6).
 //
-// Operands the split does not cover (Inf, NaN, or a nonzero magnitude outside
-// [2^-60, 2^60], whose low terms could leave the FP32 range in a product) are
-// found by the splitting kernel, which sets a flag; the tensor kernel then
-// returns at once and the SIMT kernel queued behind it, which otherwise
-// returns at once, computes the product.  No host synchronisation is needed.
-//
+// Operands the split does not cover are found by the splitting kernel, which marks
+// them; the tensor kernel then returns at once and the SIMT kernel queued behind
+// it, which otherwise returns at once, computes the product.  No host
+// synchronisation is needed.  Covered are zeros and magnitudes in [2^-90, 2^60]:
+// above, sums of products could overflow before a later term brings them back (and
+// Inf and NaN have no split); below, products could be subnormal, where six of them
+// are rounded for the SIMT core's one.  For the same reason the other operand
+// must not go below 2^-34 where one goes below 2^-60 (no product below 2^-124:
+// relative error 6e-8 there, the SIMT core's 1.1e-6).  The lower ends matter for
+// operands with a few tiny entries, exp(-x) among them: the SIMT core takes seven
+// times as long.
 // Kernel layout: persistent, one CTA per SM and 128 x 128 tile of C, 576
 // threads: warp 0 issues the TMA loads, warp 1 the MMAs, warps 2-17 drain (one
 // row and 32 columns per thread).  The planes of B lie side by side as 384 rows
@@ -94,7 +99,7 @@ __device__ __forceinline__ float hi_f(uint32_t v) { return __uint_as_float(v & 0
 // contiguous index, written as 16-byte pieces along k.  Bound by memory: 4
 // bytes read and 6 written per element.
 __global__ void __launch_bounds__(256)
-split_bf16x3(SplitOp a, SplitOp b, int K, long long pitch, int blocks_a, unsigned *flag,
+split_bf16x3(SplitOp a, SplitOp b, int K, long long pitch, int blocks_a, unsigned *marks,
              unsigned tag)
 {
     __shared__ float s[64][65];
@@ -103,7 +108,7 @@ split_bf16x3(SplitOp a, SplitOp b, int K, long long pitch, int blocks_a, unsigne
     const int blk = is_a ? blockIdx.x : blockIdx.x - blocks_a;
     const int r0 = (blk % o.tiles_r) * 64, k0 = (blk / o.tiles_r) * 64;
     const int t = threadIdx.x;
-    bool bad = false;
+    unsigned least = 0xffffffffu, most = 0u;   // of the magnitudes' bit patterns; the least less one, without zeros
     float v[16];
 #pragma unroll
     for (int u = 0; u < 16; u++) {
@@ -114,15 +119,17 @@ split_bf16x3(SplitOp a, SplitOp b, int K, long long pitch, int blocks_a, unsigne
 #pragma unroll
     for (int u = 0; u < 16; u++) {
         const uint32_t m = __float_as_uint(v[u]) & 0x7fffffffu;
-        // 2^-60 <= |x| <= 2^60, or zero
-        bad |= m != 0u && m - ((127u - 60u) << 23) > (120u << 23);
+        least = min(least, m - 1u);
+        most = max(most, m);
         const int x = t & 63, y = (t >> 6) + 4 * u;
         if (o.row_k) s[y][x] = v[u];
         else s[x][y] = v[u];
     }
-    if (__syncthreads_or(bad)) {
-        if (t == 0) *flag = tag;
-    }
+    __syncthreads();
+    auto below = [&](int e) { return least < ((unsigned)(127 + e) << 23) - 1u; };   // an element below 2^e
+    if (below(-34)) marks[is_a ? SPLIT_A_SMALL : SPLIT_B_SMALL] = tag;
+    if (below(-60)) marks[is_a ? SPLIT_A_TINY : SPLIT_B_TINY] = tag;
+    if (below(-90) || most > (127u + 60u) << 23) marks[SPLIT_UNCOVERED] = tag;
     const size_t plane = (size_t)o.rows * pitch;
 #pragma unroll
     for (int q = 0; q < 2; q++) {
@@ -152,7 +159,7 @@ struct StParams {
     float alpha, beta;
     float *C;
     long long ldc;
-    const unsigned *flag;
+    const unsigned *marks;
     unsigned tag;
     int *status, *status_host;
 };
@@ -219,7 +226,7 @@ __device__ __forceinline__ void st_store(const StParams &p, const float (&acc)[3
 __global__ void __launch_bounds__(ST_THREADS, 1)
 sgemm_bf16x3(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, StParams p)
 {
-    if (*p.flag == p.tag) return;   // the SIMT kernel behind this one computes the product
+    if (gbx_gemm::split_uncovered(p.marks, p.tag)) return;   // the SIMT kernel behind this one computes the product
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t *smB = smem + ST_ASLOTS * ST_PLANE;
@@ -444,7 +451,7 @@ size_t st_plane_bytes(int m, int n, int k, size_t *a_bytes)
     return a + 6 * (size_t)n * pitch;
 }
 
-// What the flag is set to: different in every call of the process, so that
+// What marks are set to: different in every call of the process, so that
 // scratch need not be cleared.  (Scratch that happens to hold it costs the SIMT
 // kernel's time, no more.)
 unsigned next_tag()
@@ -462,14 +469,14 @@ gbx_status run_planes(gbx_ctx *ctx, const GemmArgs<float> &g, const char *what, 
     CUtensorMap tmA, tmB;
     if (!plane_map(&tmA, pa, g.m, g.k, pitch, 1) || !plane_map(&tmB, pb, g.n, g.k, pitch, 3))
         return gbx_fail(ctx, GBX_ERR_CUDA, "%s: cuTensorMapEncodeTiled failed", what);
-    unsigned *flag = (unsigned *)ws;
+    unsigned *marks = (unsigned *)ws;
     const unsigned tag = next_tag();
 
     SplitOp a{}, b{};
     a.X = g.A; a.ld = g.lda; a.row_k = g.ta; a.rows = g.m; a.P = pa; a.tiles_r = (g.m + 63) / 64;
     b.X = g.B; b.ld = g.ldb; b.row_k = !g.tb; b.rows = g.n; b.P = pb; b.tiles_r = (g.n + 63) / 64;
     const int kt = (g.k + 63) / 64;
-    split_bf16x3<<<(unsigned)(kt * (a.tiles_r + b.tiles_r)), 256, 0, S(ctx)>>>(a, b, g.k, pitch, kt * a.tiles_r, flag,
+    split_bf16x3<<<(unsigned)(kt * (a.tiles_r + b.tiles_r)), 256, 0, S(ctx)>>>(a, b, g.k, pitch, kt * a.tiles_r, marks,
                                                                                tag);
     StParams p{};
     p.M = g.m; p.N = g.n;
@@ -479,7 +486,7 @@ gbx_status run_planes(gbx_ctx *ctx, const GemmArgs<float> &g, const char *what, 
     p.chunk = p.nkb > 4 ? 2 : 1;
     p.alpha = g.alpha; p.beta = g.beta;
     p.C = g.C; p.ldc = g.ldc;
-    p.flag = flag; p.tag = tag;
+    p.marks = marks; p.tag = tag;
     p.status = words + 4;
     p.status_host = mirror;
     // a per-device function attribute; setting it is a cheap host call
@@ -492,7 +499,7 @@ gbx_status run_planes(gbx_ctx *ctx, const GemmArgs<float> &g, const char *what, 
     gbx_count_launch(ctx, 2);
     gbx_status st = gbx_check_launch(ctx, what);
     if (st != GBX_OK) return st;
-    return launch_gemm_if(ctx, g, what, flag, tag);
+    return launch_gemm_if(ctx, g, what, marks, tag);
 }
 
 }  // namespace
@@ -558,7 +565,7 @@ gbx_status sgemm_tensor(gbx_ctx *ctx, const GemmArgs<float> &g, const char *what
     }
     int *words, *mirror;
     if (gbx_ctx_status(ctx, &words, &mirror) != GBX_OK) return GBX_OK;
-    // 256 bytes of flag, then the planes; where they cannot be had the SIMT core
+    // 256 bytes of marks, then the planes; where they cannot be had the SIMT core
     // takes the call
     void *ws;
     int block;
