@@ -366,40 +366,6 @@ __device__ __forceinline__ void tv_fetch_inv(const TrsvArgs &a, double *dst, int
     }
 }
 
-// |x| as a float, to 21 bits; at least 2^-126 unless zero, infinite beyond the FP32
-// range and for NaN.  On the integer pipe: a conversion is an FP64 instruction.
-__device__ __forceinline__ float tv_absf(double x)
-{
-    const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
-    if (h < 0x38100000u) return h ? 0x1p-126f : 0.0f;
-    return __uint_as_float(h < 0x47f00000u ? (h - 0x38000000u) << 3 : 0x7f800000u);
-}
-
-// Whether M = X T(s, s-1) may be formed for a block D with inverse X: the condition
-// number of D, the largest row sum of |X| |D|, is at most 16.  X times the
-// right-hand side is then as good as substitution; but x_s = X (b - sum) - M x
-// multiplies b - sum and T x by X before they cancel, and its backward error grows
-// with the condition number (measured against the form without M, 400 triangles: up
-// to 16 both stay below 2 u; at 16-64 20 times as much, at 1e7 400 times).  By
-// the whole CTA; r: 64 floats, the answer in the first warp.
-__device__ __forceinline__ bool tv_may_fold(const double *D, const double *X, float *r)
-{
-    const int i = threadIdx.x >> 2, q = threadIdx.x & 3;
-    float v = 0.0f;
-#pragma unroll 4
-    for (int k = q; k <= i; k += 4) v += tv_absf(D[k * TV_LD + i]);
-    v += __shfl_xor_sync(0xffffffffu, v, 1);
-    v += __shfl_xor_sync(0xffffffffu, v, 2);
-    if (q == 0) r[i] = v;
-    __syncthreads();
-    v = 0.0f;
-#pragma unroll 4
-    for (int k = q; k <= i; k += 4) v = fmaf(tv_absf(X[k * TV_LD + i]), r[k], v);
-    v += __shfl_xor_sync(0xffffffffu, v, 1);
-    v += __shfl_xor_sync(0xffffffffu, v, 2);
-    return __syncthreads_and(v <= 16.0f);   // (a NaN is not)
-}
-
 // Sum over the CTA of the 16 values that its threads (row lane & 15, columns
 // 4 (2 warp + lane / 16) ..) have for each row: in warps 0-3, lanes 4 r' + ..:
 // row 4 warp + (lane & 3).
@@ -429,10 +395,13 @@ __device__ __forceinline__ double tv_sum(double *red, double v, int lane, int wa
 //     its own ring (they do not depend on x), without barriers.
 //   * The four slices exchange z = b - sum through zw; x_s = inv z goes to the
 //     later blocks through xw and to x.
-//   * From block TV_FOLD on, for well-conditioned diagonal blocks (tv_may_fold), M =
-//     inv T(s, s-1) is formed beforehand, so that x_s = inv (b - sum over K < s-1) -
-//     M x_(s-1): the exchange and the inverse lie before x_(s-1), which needs one
-//     product.
+//   * From block TV_FOLD on, for well-conditioned diagonal blocks (whose inverse was
+//     joined), M = inv T(s, s-1) is formed beforehand, so that x_s = inv (b - sum over
+//     K < s-1) - M x_(s-1): the exchange and the inverse lie before x_(s-1), which
+//     needs one product.  It multiplies b - sum and T x by the inverse before they
+//     cancel, so its backward error grows with the condition number (against the form
+//     without M, 400 triangles: up to 16 both stay below 2 u; at 16 to 64 20 times as
+//     much, at 1e7 400 times).
 // What bounds it: the chain over the blocks, each link one hand-over through
 // L2 and the product with x_(s-1), 1.2 us; for the last blocks the FP64 pipe,
 // which takes 0.33 us for each 16 x 64 part and 11 us for M.  (With a block per
@@ -474,8 +443,7 @@ trsv_solve(TrsvArgs a)
             }
             asm volatile("cp.async.wait_all;" ::: "memory");
             __syncthreads();
-            gbx_tri::invert64(D, X, X + TV_TILE);
-            const int may = ib >= TV_FOLD && tv_may_fold(D, X, (float *)(X + TV_TILE));   // (uniform)
+            const int may = gbx_tri::invert64<true>(D, X, X + TV_TILE);
             double *o = a.inv + (size_t)ib * TV_NB * TV_NB;
             for (int e = tid; e < TV_NB * TV_NB; e += TV_THREADS) o[e] = X[(e >> 6) * TV_LD + (e & 63)];
             __threadfence();

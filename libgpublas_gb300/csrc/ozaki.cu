@@ -2606,9 +2606,13 @@ namespace {
 //   * oz_trinv_kernel: forward substitution by blocks of 32 rows, two columns
 //     of the inverse per CTA (j and n - 1 - j: together they have about n rows
 //     to solve whatever j is), one thread per row.  Block I of both columns is
-//     the inverse diagonal block times the running right-hand side; then every
-//     row below subtracts its 32 products, from columns of L' that were loaded
-//     during the block before.
+//     the inverse diagonal block times the running right-hand side, or, where
+//     that block is ill-conditioned (its inverse was not joined), solved row by
+//     row by one warp; then every row below subtracts its 32 products, from
+//     columns of L' that were loaded during the block before.  (Multiplying by the
+//     inverse of an ill-conditioned block loses its condition number once more:
+//     the Cholesky factor of a Gaussian kernel with a nugget of 1e-8 left DTRSM
+//     380 times the backward error of substitution.)
 // The bound is the FP64 pipe (2 lanes per clock per SM, n^2 / 2 FMAs per CTA: 16
 // us at n = 256) and eight block steps.  n = 256: 10 + 22 us; one warp
 // per column stepping through its 256 rows one by one took 235 us.
@@ -2628,9 +2632,9 @@ struct OzTriView {
 
 // D: per block 32 x 32, column-major; the two 16 x 16 halves by a warp each, then
 // joined (10 us; substitution on 32 rows by four warps, a hand-over per
-// row, took 15).
+// row, took 15), if it is well-conditioned: joined[block].
 __global__ void __launch_bounds__(128)
-oz_trinv_diag(OzTriView L, int unit, double *D)
+oz_trinv_diag(OzTriView L, int unit, double *D, int *joined)
 {
     gbx_launch::pdl_enter();
     constexpr int LD = OZ_TI_BLK + 1;
@@ -2648,17 +2652,21 @@ oz_trinv_diag(OzTriView L, int unit, double *D)
     for (int q = 0; q < 8; q++) sL[(4 * q + warp) * LD + lane] = v[q];
     __syncthreads();
     if (warp < 2) gbx_tri::invert16<LD>(sL, sX, 16 * warp);
+    else gbx_tri::row_sums<OZ_TI_BLK, LD>(sL, sX, t - 64);
     __syncthreads();
     gbx_tri::join32_w<LD>(sL, sX, sW, 0, t);
     __syncthreads();
     gbx_tri::join32_x<LD>(sX, sW, 0, t);
     __syncthreads();
+    const bool ok = gbx_tri::well_conditioned<OZ_TI_BLK, LD>(sL, sX);
+    if (t == 0) joined[blockIdx.x] = ok;
+    if (!ok) return;   // the block is not used
     double *d = D + (size_t)blockIdx.x * OZ_TI_BLK * OZ_TI_BLK;
     for (int e = t; e < OZ_TI_BLK * OZ_TI_BLK; e += 128) d[e] = sX[(e >> 5) * LD + (e & 31)];
 }
 
 __global__ void __launch_bounds__(OZ_TI_NMAX)
-oz_trinv_kernel(OzTriView L, int trans, const double *D, double *X, long long ldx)
+oz_trinv_kernel(OzTriView L, int unit, int trans, const double *D, const int *joined, double *X, long long ldx)
 {
     gbx_launch::pdl_enter();
     __shared__ double st[2][OZ_TI_BLK], sx[2][OZ_TI_BLK];
@@ -2674,7 +2682,7 @@ oz_trinv_kernel(OzTriView L, int trans, const double *D, double *X, long long ld
         if (I >= nb) return;
 #pragma unroll
         for (int k = 0; k < OZ_TI_BLK; k++)
-            l[k] = (warp > I && r < n) ? L(r, I * OZ_TI_BLK + k) : 0.0;
+            l[k] = (r < n && (warp > I || (warp == I && k <= lane))) ? L(r, I * OZ_TI_BLK + k) : 0.0;
 #pragma unroll
         for (int k = 0; k < 8; k++)
             d[k] = D[(size_t)I * OZ_TI_BLK * OZ_TI_BLK + (8 * pq + k) * OZ_TI_BLK + pi];
@@ -2682,16 +2690,40 @@ oz_trinv_kernel(OzTriView L, int trans, const double *D, double *X, long long ld
     load(first);
     for (int I = first; I < nb; I++) {
         const bool two = c1 < (I + 1) * OZ_TI_BLK;   // the second column has begun (uniform)
-        if (warp == I) { st[0][lane] = t0; st[1][lane] = t1; }
-        __syncthreads();
-        double x = 0.0;
-        if (pc == 0 || two) {
+        if (!joined[I]) {   // uniform
+            if (warp == I) {   // row by row
+                double dl = 1.0;
 #pragma unroll
-            for (int k = 0; k < 8; k++) x = fma(d[k], st[pc][8 * pq + k], x);
-            x += __shfl_xor_sync(0xffffffffu, x, 1);
-            x += __shfl_xor_sync(0xffffffffu, x, 2);
+                for (int k = 0; k < OZ_TI_BLK; k++)
+                    if (k == lane) dl = l[k];
+                const double rd = unit || r >= n ? 1.0 : 1.0 / dl;
+#pragma unroll
+                for (int k = 0; k < OZ_TI_BLK; k++) {
+                    // (uniform; a column has no part in the pivots before its first row)
+                    const bool in0 = I * OZ_TI_BLK + k >= c0, in1 = I * OZ_TI_BLK + k >= c1;
+                    const double y0 = in0 ? __shfl_sync(0xffffffffu, t0 * rd, k) : 0.0;
+                    const double y1 = in1 ? __shfl_sync(0xffffffffu, t1 * rd, k) : 0.0;
+                    if (lane == k) { x0 = y0; x1 = y1; }
+                    if (lane > k) {
+                        t0 = fma(-l[k], y0, t0);
+                        t1 = fma(-l[k], y1, t1);
+                    }
+                }
+                sx[0][lane] = x0;
+                sx[1][lane] = x1;
+            }
+        } else {
+            if (warp == I) { st[0][lane] = t0; st[1][lane] = t1; }
+            __syncthreads();
+            double x = 0.0;
+            if (pc == 0 || two) {
+#pragma unroll
+                for (int k = 0; k < 8; k++) x = fma(d[k], st[pc][8 * pq + k], x);
+                x += __shfl_xor_sync(0xffffffffu, x, 1);
+                x += __shfl_xor_sync(0xffffffffu, x, 2);
+            }
+            if (pq == 0) sx[pc][pi] = x;
         }
-        if (pq == 0) sx[pc][pi] = x;
         __syncthreads();
         if (warp == I) { x0 = sx[0][lane]; x1 = sx[1][lane]; }
         if (warp > I) {
@@ -2743,9 +2775,9 @@ extern "C" gbx_status gbx_dtrsm_ozaki(gbx_ctx *ctx, char side, char uplo, char t
     if (alpha == 0.0 || na > 1024) return gbx_dtrsm(ctx, side, uplo, ta, diag, m, n, alpha, A, lda, B, ldb);
     gbx_status st;
     void *px;
-    // the inverse, then (n <= 256) its inverted diagonal blocks
+    // the inverse, then (n <= 256) its inverted diagonal blocks and which of them are there
     const int nblk = (na + OZ_TI_BLK - 1) / OZ_TI_BLK;
-    const size_t dsz = na <= OZ_TI_NMAX ? (size_t)nblk * OZ_TI_BLK * OZ_TI_BLK : 0;
+    const size_t dsz = na <= OZ_TI_NMAX ? (size_t)nblk * (OZ_TI_BLK * OZ_TI_BLK + 1) : 0;
     if ((st = gbx_ws(ctx, GBX_WS_TRSM_X, sizeof(double) * ((size_t)na * na + dsz), &px)) != GBX_OK) return st;
     double *X = (double *)px;
     cudaStream_t s = S_(ctx);
@@ -2753,8 +2785,11 @@ extern "C" gbx_status gbx_dtrsm_ozaki(gbx_ctx *ctx, char side, char uplo, char t
         // X = op(A)^-1 by blocked substitution
         const OzTriView L{A, lda, na, gbx_lsame(uplo, 'L') ? 1 : 0};
         double *D = X + (size_t)na * na;
-        gbx_launch::launch_pdl(oz_trinv_diag, nblk, 128, 0, s, L, gbx_lsame(diag, 'U') ? 1 : 0, D);
-        gbx_launch::launch_pdl(oz_trinv_kernel, (na + 1) / 2, OZ_TI_NMAX, 0, s, L, gbx_lsame(ta, 'N') ? 0 : 1, D, X, na);
+        int *joined = (int *)(D + (size_t)nblk * OZ_TI_BLK * OZ_TI_BLK);
+        const int unit = gbx_lsame(diag, 'U') ? 1 : 0;
+        gbx_launch::launch_pdl(oz_trinv_diag, nblk, 128, 0, s, L, unit, D, joined);
+        gbx_launch::launch_pdl(oz_trinv_kernel, (na + 1) / 2, OZ_TI_NMAX, 0, s, L, unit, gbx_lsame(ta, 'N') ? 0 : 1, D, joined,
+                               X, na);
         gbx_count_launch(ctx, 2);
         if ((st = gbx_check_launch(ctx, "dtrsm_ozaki inverse")) != GBX_OK) return st;
     } else {

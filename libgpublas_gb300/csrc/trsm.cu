@@ -108,7 +108,7 @@ trinv64_blocks(int na, const double *__restrict__ A, long long lda, int tr, int 
         D[k * gbx_tri::LD + i] = d;
     }
     __syncthreads();
-    gbx_tri::invert64(D, X, W);
+    gbx_tri::invert64<false>(D, X, W);
     double *out = Inv + (long long)blockIdx.x * NB * NB;
     for (int t = threadIdx.x; t < NB * NB; t += blockDim.x) {
         const int i = t & 63, k = t >> 6;
