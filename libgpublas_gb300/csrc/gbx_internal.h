@@ -39,6 +39,10 @@ gbx_status gbx_fail(gbx_ctx *ctx, gbx_status st, const char *fmt, ...);
 #define GBX_WS_GEMV     14  /* gemv partial sums                            */
 #define GBX_WS_RED      15  /* reduction partials                           */
 gbx_status gbx_ws(gbx_ctx *ctx, int slot, size_t bytes, void **ptr);
+/* Whether gbx_ws would return without allocating. */
+int gbx_ws_ready(const gbx_ctx *ctx, int slot, size_t bytes);
+/* Whether the context's stream is being captured, or cannot be asked. */
+int gbx_capturing(const gbx_ctx *ctx);
 /* Scratch that one call uses between get and put, which comes after its last
  * launch; calls of the context on other streams have other blocks.  Not for a
  * stream that is being captured. */

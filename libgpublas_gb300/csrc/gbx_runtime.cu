@@ -385,6 +385,21 @@ extern "C" gbx_status gbx_ws(gbx_ctx *c, int slot, size_t bytes, void **ptr)
     return GBX_OK;
 }
 
+extern "C" int gbx_ws_ready(const gbx_ctx *c, int slot, size_t bytes)
+{
+    return slot >= 0 && slot < GBX_WS_SLOTS && c->ws_bytes[slot] >= bytes;
+}
+
+extern "C" int gbx_capturing(const gbx_ctx *c)
+{
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess) {
+        cudaGetLastError();
+        return 1;
+    }
+    return cap != cudaStreamCaptureStatusNone;
+}
+
 // A call's own scratch.  Calls on one stream share a block (they run in turn); a
 // call on another stream takes a block that nobody uses any more, or a new one, so
 // that the two stay independent; only with all blocks in use, or GBX_SCRATCH_MAX

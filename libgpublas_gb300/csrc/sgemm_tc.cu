@@ -529,12 +529,7 @@ gbx_status sgemm_tensor(gbx_ctx *ctx, const GemmArgs<float> &g, const char *what
     if (!gbx_sgemm_tensor_choice(g.m, g.n, g.k, gbx_ctx_sms(ctx))) return GBX_OK;
     // A capture gets the SIMT core: its replays outlive this call, may run on any
     // stream, and must not use scratch that other calls use too.
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(S(ctx), &cap) != cudaSuccess) {
-        cudaGetLastError();
-        return GBX_OK;
-    }
-    if (cap != cudaStreamCaptureStatusNone) return GBX_OK;
+    if (gbx_capturing(ctx)) return GBX_OK;
     size_t a_bytes;
     const size_t planes = st_plane_bytes(g.m, g.n, g.k, &a_bytes);
     if (planes > ST_WS_MAX) {
