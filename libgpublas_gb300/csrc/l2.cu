@@ -87,8 +87,8 @@ gemv_n_partial(int m, int n, int chunk, const double *A, long long lda,
 }
 
 // ROWS rows per CTA, 256 / ROWS threads per row, each summing its share of the
-// partials in order with eight loads in flight, placed while the partials are
-// computed.  64 rows per CTA: DGEMV N of 8192 x 8192 (38 partials) takes 124.5 us
+// partials in order with eight loads in flight, placed as the CTAs of the partials
+// end (or while they run, where that launch overlaps too).  64 rows per CTA: DGEMV N of 8192 x 8192 (38 partials) takes 124.5 us
 // in a stream of calls, with one thread per row in a launch that waits 129.6.
 // 16 where one CTA per SM does (few rows have many partials): 300 rows, 250
 // partials 13.5 us with 64, 9 with 16.

@@ -407,7 +407,8 @@ __device__ __forceinline__ double tv_sum(double *red, double v, int lane, int wa
 // which takes 0.33 us for each 16 x 64 part and 11 us for M.  (With a block per
 // CTA, 1.3 us of the pipe for each 64 x 64 part, a link took 2.3 us; two CTAs
 // per SM fill the pipe but share it with the link: n = 8192 6 % slower, 16000
-// 10 % faster.)  n = 8192: N or T 300 us with a block per CTA, now 214.  M for
+// 10 % faster.)  n = 8192: N or T 300 us with a block per CTA, now 208
+// to 218 (by where the exchanged words lie); without M, for ill-conditioned blocks, 334.  M for
 // every block from the 8th on: from the 12th n = 2000 is 3 us slower, from the
 // 6th all sizes the same.
 __global__ void __launch_bounds__(TV_THREADS)

@@ -1545,8 +1545,9 @@ constexpr int OZS_BN = 32, OZS_AMAX = 6, OZS_BSTG = 2, OZS_DRAIN_WARPS = 16;
 constexpr int OZS_A2 = 2 * OZ_A_BYTES;                      // an A stage: two slices
 constexpr int OZS_B_BYTES = OZS_BN * OZ_BK;                 // 4 KB: one slice's 32 rows (BN = 32)
 constexpr int OZS_THREADS = 64 + 32 * OZS_DRAIN_WARPS;
-// Dynamic shared memory: the two B stages (S x 4 KB each) and as many 16 KB
-// A stages as fit (8 for S <= 10, 6 for S = 14), barriers at the end.
+// Dynamic shared memory: the two B stages (P prepared planes of 4 KB each, BN = 16:
+// 2 KB) and as many 32 KB A stages as fit (P = 12: three, BN = 16: five), barriers
+// at the end.
 constexpr size_t OZS_SMEM = 220 * 1024;
 constexpr size_t OZS_DATA = OZS_SMEM - 1024 - 512;   // alignment slack, barriers
 static_assert(OZS_DATA >= 2 * OZ_SMAX * OZS_B_BYTES + 2 * (size_t)OZS_A2, "small-K stages");
@@ -2218,8 +2219,8 @@ bool oz_small_k(int K)
 // its 256 x 256 tiles.  Whole calls, pair / one-CTA kernel, uniform operands:
 // 2048^3 0.45 / 0.70 ms, 4096^3 2.64 / 3.07, 5120^3 4.84 / 5.41, 6144^3 8.4 / 9.0,
 // 7168^3 (10.3 waves) 13.8 / 14.2; at 8192 (calls of 20 ms and more under the
-// power cap) it draws more power, the SM clock falls further, and it loses by
-// 1.5 %.  GBX_OZAKI_PAIR=1 selects it for every product with more than one
+// power cap) it draws more power, the SM clock falls further, and the two are
+// within 2 % of each other.  GBX_OZAKI_PAIR=1 selects it for every product with more than one
 // 128-row tile (small K included), GBX_OZAKI_PAIR=0 never.
 bool oz_use_pair(int M, int N, int K, int sms)
 {
@@ -2614,7 +2615,7 @@ namespace {
 //     the Cholesky factor of a Gaussian kernel with a nugget of 1e-8 left DTRSM
 //     380 times the backward error of substitution.)
 // The bound is the FP64 pipe (2 lanes per clock per SM, n^2 / 2 FMAs per CTA: 16
-// us at n = 256) and eight block steps.  n = 256: 10 + 22 us; one warp
+// us at n = 256) and eight block steps.  n = 256: 10 + 25 us; one warp
 // per column stepping through its 256 rows one by one took 235 us.
 constexpr int OZ_TI_NMAX = 256, OZ_TI_BLK = 32;
 

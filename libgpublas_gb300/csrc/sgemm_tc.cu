@@ -43,9 +43,10 @@
 // accumulators, so its hand-over to the drain warps overlaps the next MMAs.
 // CTA pairs (256 x 256 tiles) were slower, 648 us at 4096^3: the hand-overs
 // between the two SMs take longer than the planes that fit can cover.
-// Bound by the tensor pipe: 4096^3 takes 532 us, 52 of them the splitting (which
-// runs at HBM rate), so the products run at 1.74 PFLOP/s of bf16 against a
-// measured cuBLAS burst of 1.92.  SIMT core: 4.6 ms.
+// Bound by the tensor pipe (74 % of the cycles active): 4096^3 takes 0.54 ms in a
+// stream of calls, 0.59 through sgemm_, which waits for each; 54 us of them are the
+// splitting (5.2 TB/s, bound by instruction issue) and 480 the products, 1.72 PFLOP/s
+// of bf16 against a measured cuBLAS burst of 1.92.  SIMT core: 4.6 ms.
 #include "gbx_internal.h"
 #include "gemm_host.h"
 #include "tc_ptx.cuh"
@@ -96,8 +97,8 @@ __device__ __forceinline__ float lo_f(uint32_t v) { return __uint_as_float(v << 
 __device__ __forceinline__ float hi_f(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
 
 // Both operands, 64 x 64 tiles through shared memory: read along the
-// contiguous index, written as 16-byte pieces along k.  Bound by memory: 4
-// bytes read and 6 written per element.
+// contiguous index, written as 16-byte pieces along k: 4 bytes read and 6 written
+// per element.  Bound by instruction issue (84 % of the slots) at 5.2 TB/s.
 __global__ void __launch_bounds__(256)
 split_bf16x3(SplitOp a, SplitOp b, int K, long long pitch, int blocks_a, unsigned *marks,
              unsigned tag)
