@@ -53,6 +53,8 @@ gbx_status gbx_scratch_put(gbx_ctx *ctx, int block);
  * unless null, where its last block writes seq at its end. */
 typedef struct gbx_red { unsigned *counter, *done; unsigned seq; } gbx_red;
 gbx_status gbx_reduction(gbx_ctx *ctx, size_t part_bytes, void **part, gbx_red *red);
+/* Its workspace, allocated by the first call. */
+gbx_status gbx_reduction_reserve(gbx_ctx *ctx, size_t part_bytes);
 /* Pinned host scratch owned by the context (for small results). */
 gbx_status gbx_pinned(gbx_ctx *ctx, size_t bytes, void **ptr);
 void gbx_count_launch(gbx_ctx *ctx, int n);

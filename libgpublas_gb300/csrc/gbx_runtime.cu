@@ -480,6 +480,38 @@ extern "C" gbx_status gbx_scratch_put(gbx_ctx *c, int block)
     return e == cudaSuccess ? GBX_OK : gbx_fail(c, GBX_ERR_CUDA, "scratch: %s", cudaGetErrorString(e));
 }
 
+namespace {
+struct RedLayout {
+    size_t part, counters, count;   // bytes of an entry's partials, offset and number of the counters
+    explicit RedLayout(size_t part_bytes)
+        : part((part_bytes + 255) & ~(size_t)255), counters(part * (GBX_RED_STREAMS + 1)),
+          count(GBX_RED_STREAMS + GBX_RED_CAPTURED) {}
+    size_t bytes() const { return counters + sizeof(unsigned) * count; }
+};
+}
+
+extern "C" gbx_status gbx_reduction_reserve(gbx_ctx *c, size_t part_bytes)
+{
+    if (c->red_done) return GBX_OK;
+    const RedLayout lay(part_bytes);
+    char *base;
+    gbx_status st = gbx_ws(c, GBX_WS_RED, lay.bytes(), (void **)&base);
+    if (st != GBX_OK) return st;
+    void *h = nullptr;
+    cudaError_t e = cudaMemsetAsync(base + lay.counters, 0, sizeof(unsigned) * lay.count, c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    if (e == cudaSuccess) e = cudaHostAlloc(&h, sizeof(unsigned) * GBX_RED_STREAMS, cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&c->red_done_dev, h, 0);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        if (h) cudaFreeHost(h);
+        return gbx_fail(c, GBX_ERR_ALLOC, "reduction: %s", cudaGetErrorString(e));
+    }
+    memset(h, 0, sizeof(unsigned) * GBX_RED_STREAMS);
+    c->red_done = (volatile unsigned *)h;
+    return GBX_OK;
+}
+
 // State of a one-launch reduction: the blocks' partials, the count of finished
 // blocks (zero between launches) and where its last block writes seq.  The
 // reductions of one stream run in turn and share an entry; another stream has
@@ -492,9 +524,7 @@ extern "C" gbx_status gbx_scratch_put(gbx_ctx *c, int block)
 // one array for all: their replays must not overlap.)
 extern "C" gbx_status gbx_reduction(gbx_ctx *c, size_t part_bytes, void **part, gbx_red *red)
 {
-    part_bytes = (part_bytes + 255) & ~(size_t)255;   // the same in every call
-    const size_t counters = part_bytes * (GBX_RED_STREAMS + 1);
-    const size_t count = GBX_RED_STREAMS + GBX_RED_CAPTURED;
+    const RedLayout lay(part_bytes);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     unsigned long long id = 0;
     cudaError_t e = cudaStreamIsCapturing(c->stream, &cap);
@@ -503,29 +533,15 @@ extern "C" gbx_status gbx_reduction(gbx_ctx *c, size_t part_bytes, void **part, 
         cudaGetLastError();
         return gbx_fail(c, GBX_ERR_CUDA, "reduction: %s", cudaGetErrorString(e));
     }
-    char *base;
-    gbx_status st = gbx_ws(c, GBX_WS_RED, counters + sizeof(unsigned) * count, (void **)&base);
+    const gbx_status st = gbx_reduction_reserve(c, part_bytes);
     if (st != GBX_OK) return st;
-    if (!c->red_done) {
-        void *h = nullptr;
-        e = cudaMemsetAsync(base + counters, 0, sizeof(unsigned) * count, c->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-        if (e == cudaSuccess) e = cudaHostAlloc(&h, sizeof(unsigned) * GBX_RED_STREAMS, cudaHostAllocMapped);
-        if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&c->red_done_dev, h, 0);
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            if (h) cudaFreeHost(h);
-            return gbx_fail(c, GBX_ERR_ALLOC, "reduction: %s", cudaGetErrorString(e));
-        }
-        memset(h, 0, sizeof(unsigned) * GBX_RED_STREAMS);
-        c->red_done = (volatile unsigned *)h;
-    }
+    char *base = (char *)c->ws[GBX_WS_RED];
     red->done = nullptr;
     red->seq = 0;
     if (cap != cudaStreamCaptureStatusNone) {
-        *part = base + part_bytes * GBX_RED_STREAMS;
+        *part = base + lay.part * GBX_RED_STREAMS;
         const bool fresh = c->red_captured < GBX_RED_CAPTURED - 1;
-        red->counter = (unsigned *)(base + counters) + GBX_RED_STREAMS + c->red_captured;
+        red->counter = (unsigned *)(base + lay.counters) + GBX_RED_STREAMS + c->red_captured;
         if (fresh) c->red_captured++;
         else if (cudaMemsetAsync(red->counter, 0, sizeof(unsigned), c->stream) != cudaSuccess)   // the last one, cleared
             return gbx_check_launch(c, "reduction counter");
@@ -550,8 +566,8 @@ extern "C" gbx_status gbx_reduction(gbx_ctx *c, size_t part_bytes, void **part, 
     r.id = id;
     r.used = ++c->red_uses;
     if (++r.seq == 0) r.seq = 1;
-    *part = base + part_bytes * pick;
-    red->counter = (unsigned *)(base + counters) + pick;
+    *part = base + lay.part * pick;
+    red->counter = (unsigned *)(base + lay.counters) + pick;
     red->done = c->red_done_dev + pick;
     red->seq = r.seq;
     return GBX_OK;

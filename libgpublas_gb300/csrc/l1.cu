@@ -42,14 +42,16 @@ inline int reduction_grid(gbx_ctx *ctx, long long n)
 }
 
 // Partials (at most three values per block) and counter of a reduction.  One block
-// needs neither.
+// needs neither; its call allocates them all the same, so that any reduction can be
+// captured on a context that has run one.
 template <typename P>
 gbx_status reduction_ws(gbx_ctx *ctx, int g, P **part, gbx_red *red)
 {
+    const size_t bytes = 3 * sizeof(double) * (size_t)gbx_ctx_sms(ctx) * L1_BLOCKS_PER_SM;
     *part = nullptr;
     *red = gbx_red{};
-    if (g == 1) return GBX_OK;
-    return gbx_reduction(ctx, 3 * sizeof(double) * (size_t)gbx_ctx_sms(ctx) * L1_BLOCKS_PER_SM, (void **)part, red);
+    if (g > 1) return gbx_reduction(ctx, bytes, (void **)part, red);
+    return gbx_reduction_reserve(ctx, bytes);
 }
 
 // element offset of the first element a kernel should touch: netlib walks a

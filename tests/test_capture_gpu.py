@@ -63,6 +63,23 @@ def test_dtrsv_after_dtrsm(own, n):
     assert torch.equal(x, y)
 
 
+def test_reduction_after_a_shorter_one(own):
+    """A context that has run a reduction of one block can capture one of any size."""
+    import torch
+    x = uni(10, 1 << 20)
+    r = torch.zeros(2, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    own.dnrm2(100, x, 1, r)
+    own.sync()
+    graph = capture(own, lambda: own.ddot(1 << 20, x, 1, x, 1, r[1:]))
+    graph.replay()
+    torch.cuda.synchronize()
+    want = torch.zeros(1, dtype=torch.float64, device="cuda")
+    own.ddot(1 << 20, x, 1, x, 1, want)
+    own.sync()
+    assert torch.equal(r[1:], want)
+
+
 def test_a_sequence_of_calls(own):
     import torch
     n, m = 300, 200
